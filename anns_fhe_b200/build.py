@@ -27,8 +27,9 @@ OBJDIR = os.path.join(os.path.dirname(HERE), "_build", "afhe")
 ROOT = os.path.dirname(HERE)
 INCLUDE = os.path.join(ROOT, "include")
 
-SOURCES = ["api.cu", "driver.cu", "encode.cu", "ivfpq.cu", "kernels.cu", "ksfused.cu", "noalloc.cu", "tables.cpp"]
-HEADERS = ["internal.h", "lanes.h", "modarith.cuh", "ntt.cuh", "tables.h"]
+SOURCES = ["api.cu", "driver.cu", "encode.cu", "ivfpq.cu", "kernels.cu", "ksfused.cu", "ksfused_multi.cu",
+           "ksfused_raw.cu", "ksfused_single.cu", "kswitch.cu", "kswitch_down.cu", "noalloc.cu", "rescale.cu", "tables.cpp"]
+HEADERS = ["internal.h", "ksfused.cuh", "lanes.h", "modarith.cuh", "ntt.cuh", "tables.h"]
 
 ARCH_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a"]
 

@@ -79,8 +79,9 @@ int zf_from(afhe_ctx* ctx, const u64* vals, uint32_t n, ZField* out) {
 
 namespace {
 
-PrimeConst host_prime_const(u64 q, u64 ninv, u64 itw1) {
-    PrimeConst c;
+// transforms: with the constants in transform form (only a transform needs them)
+PrimeConst host_prime_const(u64 q, u64 ninv, u64 itw1, bool transforms) {
+    PrimeConst c{};
     c.q = q;
     ModConst m = make_modconst(q);
     c.r64 = m.r64;
@@ -90,6 +91,7 @@ PrimeConst host_prime_const(u64 q, u64 ninv, u64 itw1) {
     c.ninv_sh = host_shoup(c.ninv, q);
     c.w1ninv = (u64)((unsigned __int128)(itw1 % q) * c.ninv % q);
     c.w1ninv_sh = host_shoup(c.w1ninv, q);
+    if (transforms) set_transform_constants(c);
     return c;
 }
 
@@ -193,27 +195,37 @@ int build_native_tables(afhe_ctx* ctx) {
     for (uint32_t i = 0; i < L; ++i) primes[i] = ctx->prm.q[i];
     for (uint32_t k = 0; k < K; ++k) primes[L + k] = ctx->prm.p[k];
 
-    std::vector<u64> tw(n), itw(n);
-    std::vector<ulonglong2> tw2((size_t)np * n), itw2((size_t)np * n);
+    // raw twiddles (natural order) to the device, which lays them out as
+    // transform constants in the rounds' order
+    std::vector<u64> tw((size_t)np * n), itw((size_t)np * n);
     std::vector<PrimeConst> pc(np);
     for (uint32_t i = 0; i < np; ++i) {
         u64 q = primes[i];
-        u64 psi = root_of(ctx, i);
-        gen_twiddles(ctx->log_n, q, psi, tw.data(), itw.data());
-        for (uint32_t j = 0; j < n; ++j) {
-            tw2[(size_t)i * n + j] = make_ulonglong2(tw[j], host_shoup(tw[j], q));
-            itw2[(size_t)i * n + j] = make_ulonglong2(itw[j], host_shoup(itw[j], q));
-        }
-        pc[i] = host_prime_const(q, inv_mod(n % q, q), itw[1]);
+        u64* const iw = &itw[(size_t)i * n];
+        gen_twiddles(ctx->log_n, q, root_of(ctx, i), &tw[(size_t)i * n], iw);
+        pc[i] = host_prime_const(q, inv_mod(n % q, q), iw[1], true);
     }
     DevPrimeSet& s = ctx->nat;
     s.count = np;
     CK(dalloc(&s.pc, np));
     CK(dalloc(&s.tw2, (size_t)np * n));
     CK(dalloc(&s.itw2, (size_t)np * n));
+    CK(dalloc(&s.tw2b, (size_t)np * n));
+    CK(dalloc(&s.itw2b, (size_t)np * n));
     CK(cudaMemcpy(s.pc, pc.data(), np * sizeof(PrimeConst), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(s.tw2, tw2.data(), tw2.size() * sizeof(ulonglong2), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(s.itw2, itw2.data(), itw2.size() * sizeof(ulonglong2), cudaMemcpyHostToDevice));
+    {
+        u64* raw = nullptr;
+        const size_t w = (size_t)np * n;
+        CK(dalloc(&raw, 2 * w + np));
+        cudaError_t e = cudaMemcpy(raw, tw.data(), w * 8, cudaMemcpyHostToDevice);
+        if (e == cudaSuccess) e = cudaMemcpy(raw + w, itw.data(), w * 8, cudaMemcpyHostToDevice);
+        if (e == cudaSuccess) e = cudaMemcpy(raw + 2 * w, primes.data(), np * 8, cudaMemcpyHostToDevice);
+        if (e == cudaSuccess) e = launch_twiddles(raw, raw + 2 * w, s.tw2, s.tw2b, np, ctx->log_n, ctx->st);
+        if (e == cudaSuccess) e = launch_twiddles(raw + w, raw + 2 * w, s.itw2, s.itw2b, np, ctx->log_n, ctx->st);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->st);
+        cudaFree(raw);
+        if (e != cudaSuccess) return cuda_fail(ctx, e, "twiddle tables");
+    }
 
     // per-level CRT tables, each followed by its Shoup companions
     std::vector<u64> buf;
@@ -228,7 +240,28 @@ int build_native_tables(afhe_ctx* ctx) {
     };
     struct LvlRefs {
         Ref qi[AFHE_MAX_PARTS], qm[AFHE_MAX_PARTS], pinv, phinv, phq, qlql, qlinv;
+        size_t qm_sp[AFHE_MAX_PARTS], phq_sp, fin_q, fin_p, pmq, pinv_tc;   // 16-byte aligned
         uint32_t parts;
+    };
+    auto align2 = [&]() { if (buf.size() & 1) buf.push_back(0); return buf.size(); };
+    auto push_split = [&](const std::vector<u64>& vals, const std::vector<u64>& mods) {
+        const size_t at = align2();
+        buf.resize(at + 4 * vals.size());
+        for (size_t i = 0; i < vals.size(); ++i) split_constant(vals[i], mods[i], &buf[at + 4 * i]);
+        return at;
+    };
+    // f times the last inverse stage's constants, and w itself, as prime i transforms
+    auto push_fin = [&](u64 f, uint32_t i) {
+        const u64 m = primes[i];
+        u64 o[8];
+        transform_constant((u64)((unsigned __int128)pc[i].ninv * f % m), m, o);
+        transform_constant((u64)((unsigned __int128)pc[i].w1ninv * f % m), m, o + 4);
+        buf.insert(buf.end(), o, o + 8);
+    };
+    auto push_tc = [&](u64 w, u64 m) {
+        u64 o[4];
+        transform_constant(w % m, m, o);
+        buf.insert(buf.end(), o, o + 4);
     };
     std::vector<LvlRefs> refs(L + 1);
     const u64* q = primes.data();
@@ -252,6 +285,7 @@ int build_native_tables(afhe_ctx* ctx) {
             }
             R.qi[j] = push(qi, mi);
             R.qm[j] = push(qm, mm);
+            R.qm_sp[j] = push_split(qm, mm);
         }
         std::vector<u64> pinv(lvl), phinv(K), phq((size_t)K * lvl), mq(lvl), mp(K), mphq((size_t)K * lvl);
         moddown_tables(q, lvl, p, K, pinv.data(), phinv.data(), phq.data());
@@ -263,6 +297,22 @@ int build_native_tables(afhe_ctx* ctx) {
         R.pinv = push(pinv, mq);
         R.phinv = push(phinv, mp);
         R.phq = push(phq, mphq);
+        R.phq_sp = push_split(phq, mphq);
+        R.fin_q = align2();
+        for (uint32_t i = 0; i < lvl; ++i) {
+            const uint32_t j = i / ctx->alpha;
+            push_fin(buf[R.qi[j].v + (i - j * ctx->alpha)], i);
+        }
+        R.fin_p = align2();
+        for (uint32_t k = 0; k < K; ++k) push_fin(phinv[k], L + k);
+        R.pmq = align2();
+        for (uint32_t i = 0; i < lvl; ++i) {
+            u64 prod = 1;
+            for (uint32_t k = 0; k < K; ++k) prod = (u64)((unsigned __int128)prod * (p[k] % q[i]) % q[i]);
+            push_tc(prod, q[i]);
+        }
+        R.pinv_tc = align2();
+        for (uint32_t i = 0; i < lvl; ++i) push_tc(pinv[i], q[i]);
         std::vector<u64> qlql(lvl > 1 ? lvl - 1 : 1, 0), qlinv(lvl > 1 ? lvl - 1 : 1, 0), mr(lvl > 1 ? lvl - 1 : 1, 3);
         if (lvl > 1) {
             rescale_tables(q, lvl, qlql.data(), qlinv.data());
@@ -288,7 +338,13 @@ int build_native_tables(afhe_ctx* ctx) {
             t.qhat_inv_sh[j] = b + R.qi[j].sh;
             t.qhat_modp[j] = b + R.qm[j].v;
             t.qhat_modp_sh[j] = b + R.qm[j].sh;
+            t.qhat_modp_sp[j] = b + R.qm_sp[j];
         }
+        t.phat_modq_sp = b + R.phq_sp;
+        t.fin_q = b + R.fin_q;
+        t.fin_p = b + R.fin_p;
+        t.p_mod_q = b + R.pmq;
+        t.p_inv_tc = b + R.pinv_tc;
         t.p_inv_mod_q = b + R.pinv.v;
         t.p_inv_mod_q_sh = b + R.pinv.sh;
         t.phat_inv_modp = b + R.phinv.v;
@@ -456,7 +512,9 @@ int afhe_ctx_destroy(afhe_ctx* ctx) {
     auto fr = [](void* p) { if (p) cudaFree(p); };
     fr(ctx->poly); fr(ctx->key); fr(ctx->lvbuf); fr(ctx->lv_dev); fr(ctx->jobs_qp);
     for (auto& j : ctx->lvjobs) fr(j.modup);
-    for (DevPrimeSet* s : {&ctx->nat, &ctx->ld}) { fr(s->pc); fr(s->tw); fr(s->itw); fr(s->tw2); fr(s->itw2); }
+    for (DevPrimeSet* s : {&ctx->nat, &ctx->ld}) {
+        fr(s->pc); fr(s->tw); fr(s->itw); fr(s->tw2); fr(s->itw2); fr(s->tw2b); fr(s->itw2b);
+    }
     fr(ctx->ld_crt); fr(ctx->ld_crt_sh); fr(ctx->ld_mod);
     for (auto& kv : ctx->rot) fr(kv.second.map);
     for (auto& kv : ctx->auto_maps) fr(kv.second);
@@ -576,11 +634,6 @@ int afhe_ctx_set_option(afhe_ctx* ctx, uint32_t option, int64_t value) {
         return AFHE_OK;
     case AFHE_OPT_KS_SLICE:
         if (value != 12 && value != 13) return fail(ctx, AFHE_E_ARG, "the slice must be 2^12 or 2^13 values");
-        if (value == 12 && (ctx->log_n == 14 || ctx->log_n == 15)) {
-            if (cudaSetDevice(ctx->device) != cudaSuccess) return fail(ctx, AFHE_E_CUDA, "cudaSetDevice");
-            if (key_switch_fused_capacity(ctx->log_n, 8, 12) <= 0)
-                return fail(ctx, AFHE_E_ARG, "clusters of 2^12-value slices cannot run on this GPU");
-        }
         ctx->ks_slice = (uint32_t)value;
         return AFHE_OK;
     case AFHE_OPT_KS_CAPACITY:
@@ -600,7 +653,7 @@ int afhe_ctx_get_option(afhe_ctx* ctx, uint32_t option, int64_t* value) {
     case AFHE_OPT_KS_SLICE: *value = ctx->ks_slice; return AFHE_OK;
     case AFHE_OPT_KS_CAPACITY:
         if (cudaSetDevice(ctx->device) != cudaSuccess) return fail(ctx, AFHE_E_CUDA, "cudaSetDevice");
-        *value = key_switch_fused_capacity(ctx->log_n, (int)ctx->ks_ept, (int)ctx->ks_slice);
+        *value = key_switch_fused_capacity(ctx->log_n);
         return AFHE_OK;
     default: return fail(ctx, AFHE_E_ARG, "unknown option");
     }
@@ -780,13 +833,16 @@ int load_context(afhe_ctx* ctx, const afhe_accel_args* a) {
     // twiddles: (L + K) rows, Q then P
     DevPrimeSet& s = ctx->ld;
     if (s.count < L + K) {
-        for (void* pp : {(void*)s.pc, (void*)s.tw, (void*)s.itw, (void*)s.tw2, (void*)s.itw2}) if (pp) cudaFree(pp);
+        for (void* pp : {(void*)s.pc, (void*)s.tw, (void*)s.itw, (void*)s.tw2, (void*)s.itw2, (void*)s.tw2b, (void*)s.itw2b})
+            if (pp) cudaFree(pp);
         s = DevPrimeSet{};
         CK(dalloc(&s.pc, AFHE_MAX_Q + AFHE_MAX_P));
         CK(dalloc(&s.tw, (size_t)(AFHE_MAX_Q + AFHE_MAX_P) * n));
         CK(dalloc(&s.itw, (size_t)(AFHE_MAX_Q + AFHE_MAX_P) * n));
         CK(dalloc(&s.tw2, (size_t)(AFHE_MAX_Q + AFHE_MAX_P) * n));
         CK(dalloc(&s.itw2, (size_t)(AFHE_MAX_Q + AFHE_MAX_P) * n));
+        CK(dalloc(&s.tw2b, (size_t)(AFHE_MAX_Q + AFHE_MAX_P) * n));
+        CK(dalloc(&s.itw2b, (size_t)(AFHE_MAX_Q + AFHE_MAX_P) * n));
         s.count = AFHE_MAX_Q + AFHE_MAX_P;
     }
     cudaStream_t st = ctx->st;
@@ -805,8 +861,8 @@ int load_context(afhe_ctx* ctx, const afhe_accel_args* a) {
     CK(dalloc(&dn, L + K));
     CK(cudaMemcpyAsync(dq, qv.data(), qv.size() * 8, cudaMemcpyHostToDevice, st));
     CK(cudaMemcpyAsync(dn, ninv.data(), ninv.size() * 8, cudaMemcpyHostToDevice, st));
-    CK(launch_interleave(s.tw, dq, s.tw2, L + K, n, st));
-    CK(launch_interleave(s.itw, dq, s.itw2, L + K, n, st));
+    CK(launch_twiddles(s.tw, dq, s.tw2, s.tw2b, L + K, ctx->log_n, st));
+    CK(launch_twiddles(s.itw, dq, s.itw2, s.itw2b, L + K, ctx->log_n, st));
     CK(launch_prime_consts(s.pc, dq, dn, s.itw, n, L + K, st));
     CK(cudaStreamSynchronize(st));
     cudaFree(dq); cudaFree(dn);
@@ -1016,7 +1072,7 @@ extern "C" int afhe_dispatch(afhe_ctx* ctx, const afhe_accel_args* a) {
         std::vector<PrimeConst> pc(L);
         for (uint32_t i = 0; i < L; ++i) {
             if (a->rns_primes[i] < 3 || a->rns_primes[i] >= (1ull << 61)) return fail(ctx, AFHE_E_ARG, "modulus out of range");
-            pc[i] = host_prime_const(a->rns_primes[i], 1, 1);
+            pc[i] = host_prime_const(a->rns_primes[i], 1, 1, false);
         }
         static_assert(sizeof(PrimeConst) % sizeof(u64) == 0, "PrimeConst is staged as words");
         u64* dpc_words = nullptr;

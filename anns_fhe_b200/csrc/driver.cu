@@ -109,9 +109,8 @@ int ks_batch(afhe_ctx* ctx, const ZField& in, const ZField& out0, const ZField& 
     zb.mid = lane_field(ctx, &Lane::ks);
     if (lvz && !(ctx->ks_fused && fused_ok)) return fail(ctx, AFHE_E_STATE, "mixed levels need the one-kernel key switch");
     if (ctx->ks_fused && fused_ok && (lvz || nz >= ctx->fused_min)) {
-        CK(launch_key_switch_fused(ctx->log_n, t, limbs, ctx->K, ctx->key, evk, evk + (u64)ctx->dnum * S * n,
-                                   (uint32_t)S, ctx->L, ctx->poly, ctx->scr, nz, zb, ctx->st, fuse, prep,
-                                   lvz ? ctx->lv_dev : nullptr, lvz, (int)ctx->ks_ept, (int)ctx->ks_slice));
+        CK(launch_key_switch_fused(ctx->log_n, ctx->lv_dev, ctx->alpha, limbs, ctx->K, ctx->key, evk, evk + (u64)ctx->dnum * S * n,
+                                   (uint32_t)S, ctx->L, ctx->poly, ctx->scr, nz, zb, ctx->st, fuse, prep, lvz));
         return AFHE_OK;
     }
     CK(launch_key_switch(ctx->log_n, t, ctx->jobs_qp, lj.modup, lj.n_modup, ctx->L, limbs, ctx->K, ctx->key, evk,
@@ -293,13 +292,14 @@ int rotate_batch(afhe_ctx* ctx, const afhe_ct_ref* in, const afhe_ct_ref* dst, u
 
 u64 key_region_words(const afhe_ctx* ctx) { return 2ull * ctx->dnum * (ctx->L + ctx->K) * ctx->n; }
 
-// The one-kernel key switch reads a registered key through a prepared copy:
-// (k mod q, Shoup companion) per key word, derived on the device.
+// The one-kernel key switch reads a registered key through a prepared copy,
+// derived on the device (key_prep_kernel).
 int prep_key(afhe_ctx* ctx, u64 evk, ulonglong2** prep) {
     if (!ctx->ks_fused) return AFHE_OK;
     const u64 words = key_region_words(ctx);
     if (!*prep) CK(cudaMalloc((void**)prep, words * sizeof(ulonglong2)));
-    CK(launch_key_prep(ctx->key + evk, *prep, ctx->nat.pc, ctx->n, ctx->L + ctx->K, words, ctx->st));
+    CK(launch_key_prep(ctx->key + evk, *prep, ctx->nat.pc, ctx->log_n, ctx->L, ctx->L + ctx->K, ctx->dnum, ctx->alpha,
+                       words, ctx->st));
     return AFHE_OK;
 }
 
@@ -704,9 +704,8 @@ int afhe_eval_rotate_steps_batch(afhe_ctx* ctx, const afhe_ct_ref* in, const afh
                 ZF(f.prepz, preps);
                 prep = ctx->rot.at(steps[s]).prep;
             }
-            CK(launch_key_switch_fused(ctx->log_n, t, limbs, ctx->K, ctx->key, 0, (u64)ctx->dnum * S * n, (uint32_t)S,
-                                       ctx->L, ctx->poly, ctx->scr, m, zb, ctx->st, &f, prep, nullptr, nullptr,
-                                       (int)ctx->ks_ept, (int)ctx->ks_slice));
+            CK(launch_key_switch_fused(ctx->log_n, ctx->lv_dev, ctx->alpha, limbs, ctx->K, ctx->key, 0, (u64)ctx->dnum * S * n, (uint32_t)S,
+                                       ctx->L, ctx->poly, ctx->scr, m, zb, ctx->st, &f, prep));
             return AFHE_OK;
         }
         CK(launch_key_switch(ctx->log_n, t, ctx->jobs_qp, lj.modup, lj.n_modup, ctx->L, limbs, ctx->K, ctx->key, 0,

@@ -35,19 +35,31 @@ struct OpTabs {
     const u64* qlql_sh;
     const u64* qlinv;
     const u64* qlinv_sh;
+    // base-conversion constants in split form (4 words each, split_constant)
+    const u64* qhat_modp_sp[AFHE_MAX_PARTS];
+    const u64* phat_modq_sp;
+    // one-kernel key switch (native tables): the last inverse stage's two
+    // constants times qHatInv (per Q limb) and times PHatInv (per special
+    // limb), 8 words each; P and P^-1 mod q_i as transform constants, 4 each
+    const u64* fin_q;
+    const u64* fin_p;
+    const u64* p_mod_q;
+    const u64* p_inv_tc;
 };
 
 // Owned device storage for one twiddle table set. tw / itw hold raw tables
-// (only for tables loaded by OP_LOAD_CONTEXT); tw2 / itw2 the (w, companion)
-// pairs the kernels read.
+// (only for tables loaded by OP_LOAD_CONTEXT); tw2 / itw2 (tw2b / itw2b) the
+// transform constants the kernels read.
 struct DevPrimeSet {
     PrimeConst* pc = nullptr;
     u64* tw = nullptr;
     u64* itw = nullptr;
     ulonglong2* tw2 = nullptr;
     ulonglong2* itw2 = nullptr;
+    ulonglong2* tw2b = nullptr;
+    ulonglong2* itw2b = nullptr;
     uint32_t count = 0;
-    PrimeTables view() const { return PrimeTables{pc, tw2, itw2}; }
+    PrimeTables view() const { return PrimeTables{pc, tw2, itw2, tw2b, itw2b}; }
 };
 
 // Ring of small per-launch descriptor arrays (ZField::arr): pinned host
@@ -66,7 +78,7 @@ struct RotKey {
     uint32_t galois;
     u64 evk_offset;
     uint32_t* map;              // device, N entries
-    ulonglong2* prep = nullptr;  // (k mod q, Shoup companion) per key word, for the one-kernel key switch
+    ulonglong2* prep = nullptr;  // prepared copy for the one-kernel key switch (key_prep_kernel)
 };
 
 // Key-switch job templates for one level (device arrays).
@@ -118,8 +130,8 @@ struct afhe_ctx {
     bool ks_fused = true;   // one-kernel key switch where supported (AFHE_KS_FUSED=0 turns it off)
     uint32_t chunk = 0;     // ciphertexts per launch of a batched call (0: all lanes)
     uint32_t fused_min = 1; // launches of fewer ciphertexts take the multi-kernel key switch
-    uint32_t ks_ept = 8;    // values per thread of the one-kernel key switch (8 or 16)
-    uint32_t ks_slice = 13; // log2 of the slice a CTA of a cluster holds (12: N = 2^14, 2^15 only)
+    uint32_t ks_ept = 8;    // AFHE_OPT_KS_EPT and AFHE_OPT_KS_SLICE: kept for callers that set them
+    uint32_t ks_slice = 13;
     // afhe_fence: fence f is event fences[f % size], recorded on st
     std::vector<cudaEvent_t> fences;
     uint64_t fence_next = 0;
@@ -253,37 +265,36 @@ cudaError_t launch_key_switch(int log_n, const OpTabs& t, const LimbJob* jobs_qp
                               u64* arena, u64* scratch, uint32_t nz, const ZBases& zb, cudaStream_t st,
                               const KsFuse* fuse = nullptr);
 
-// The same key switch as one kernel per polynomial: for N <= 2^13 one CTA,
-// above that a cluster of N / 2^13 CTAs (distributed shared memory) keeps
-// the limb being transformed and both accumulators in shared memory
+// The same key switch as one kernel per polynomial: for N <= 2^12 one CTA,
+// above that a cluster of CTAs (distributed shared memory) keeps the limb
+// being transformed and both sums in shared memory
 // and needs ks_fused_scratch_words(...) words of scratch at zb.mid (the INTT
-// of the input's limbs and of the special accumulators). Entries of one
+// of the input's limbs and of the special sums). Entries of one
 // launch run concurrently, so an entry's outputs must not overlap another
 // entry's inputs (in place within an entry is fine).
-// `prep`, when given, holds the key (evk_a digits then evk_b digits, the key
-// region's word order) as (k mod q, Shoup companion) pairs; the inner product
-// then multiplies with Shoup's method instead of a full 128-bit reduction.
+// `prep`, when given, holds the key in the form the kernel's products take
+// (launch_key_prep); an unprepared key goes through full 128-bit reductions.
 bool key_switch_fused_supported(int log_n);
 // ciphertexts the one-kernel key switch holds at once on the current device
-// (resident CTAs at N <= 2^13, resident clusters above; 0: cannot run)
-int key_switch_fused_capacity(int log_n, int ept = 8, int slice = 13);
+// (resident CTAs at N <= 2^12, resident clusters above; 0: cannot run)
+int key_switch_fused_capacity(int log_n);
 size_t ks_fused_scratch_words(uint32_t n, uint32_t sizeQl, uint32_t K);
-cudaError_t launch_key_switch_fused(int log_n, const OpTabs& t, uint32_t sizeQl, uint32_t K, const u64* key, u64 evk_a,
+cudaError_t launch_key_switch_fused(int log_n, const OpTabs* lvtabs, uint32_t alpha, uint32_t sizeQl, uint32_t K, const u64* key, u64 evk_a,
                                     u64 evk_b, uint32_t key_stride, uint32_t key_pbase, u64* arena, u64* scratch,
                                     uint32_t nz, const ZBases& zb, cudaStream_t st, const KsFuse* fuse = nullptr,
-                                    const ulonglong2* prep = nullptr, const OpTabs* lvtabs = nullptr,
-                                    const ZField* lvz = nullptr, int ept = 8, int slice = 13);
-// With lvtabs and lvz (mixed levels), entry z runs at level lvz->at(z) with
-// the tables lvtabs[level] (a device copy of the context's per-level tables;
-// sizeQl is then the largest level), each reading and writing that many limbs.
-// prep[w] = (k mod q, companion) for k = key[w], w < words, where word w
-// belongs to key limb slot (w / n) mod S and slot i uses prime pc[i].
-cudaError_t launch_key_prep(const u64* key, ulonglong2* prep, const PrimeConst* pc, uint32_t n, uint32_t S, u64 words,
-                            cudaStream_t st);
+                                    const ulonglong2* prep = nullptr, const ZField* lvz = nullptr);
+// lvtabs: device copy of the context's per-level tables. With lvz (mixed
+// levels), entry z runs at level lvz->at(z) with the tables lvtabs[level],
+// reading and writing that many limbs (sizeQl is then the largest level).
+// launch_key_prep: the prepared copy of `words` = 2 dnum S N key words, S = L
+// + K limb slots per digit, slot i under prime pc[i].
+cudaError_t launch_key_prep(const u64* key, ulonglong2* prep, const PrimeConst* pc, int log_n, uint32_t L, uint32_t S,
+                            uint32_t dnum, uint32_t alpha, u64 words, cudaStream_t st);
 
-// Twiddle pairs: out2[r * n + j] = (w, companion of w), w = raw[r * n + j] mod q[r].
-cudaError_t launch_interleave(const u64* raw, const u64* q, ulonglong2* out2, uint32_t rows, uint32_t n,
-                              cudaStream_t st);
+// Twiddle rows: raw[r n + j] = psi^bitrev(j) mod q[r] (or its inverse), j < n,
+// as transform constants in the rounds' order (PrimeTables).
+cudaError_t launch_twiddles(const u64* raw, const u64* q, ulonglong2* out2, ulonglong2* out2b, uint32_t rows, int log_n,
+                            cudaStream_t st);
 // Companion prep: sh[e] = shoup_companion(v[e] mod m[e], m[e]); v reduced in place.
 cudaError_t launch_companions(u64* v, u64* sh, const u64* m, size_t count, cudaStream_t st);
 // Loaded prime constants: fills pc[i] from q/ninv arrays (device) and itw.

@@ -476,336 +476,6 @@ cudaError_t launch_ntt_plain(bool inverse, int log_n, const PrimeTables& pt, con
 }
 
 // ---------------------------------------------------------------------------
-// rescale (rescale.cpp:3-72)
-//   step 1: INTT of the last limb -> coefficients in scratch
-//   step 2: NTT over limbs i < L-1 whose prologue is the centred lift of the
-//           last limb times QlQlInvModqlDivqlModq[i], and whose epilogue is
-//           a_i * qlInvModq[i] + NTT(...)
-// ---------------------------------------------------------------------------
-struct RescaleLoad {
-    const u64* scratch;
-    const u64* qlql;
-    const u64* qlql_sh;
-    const PrimeConst* pc_last;   // q_l, the prime being dropped
-    __device__ __forceinline__ u64 operator()(const LimbJob& j, const ZBases& zb, uint32_t z, uint32_t x,
-                                              const PrimeConst& pc) const {
-        const u64 q = pc.q;
-        const u64 ql = pc_last->q, ql_half = ql >> 1;
-        u64 v = scratch[zb.aux.at(z) + x];                           // last limb coefficient, [0, q_l)
-        u64 vm = csub(mul_shoup_lazy(v, 1, pc.one_sh, q), q);         // v mod q_i
-        u64 qlm = csub(mul_shoup_lazy(ql, 1, pc.one_sh, q), q);       // q_l mod q_i
-        u64 val = (v > ql_half) ? sub_mod(vm, qlm, q) : vm;           // rescale.cpp:50 tie rule
-        return mul_shoup(val, __ldg(qlql + j.aux), __ldg(qlql_sh + j.aux), q);
-    }
-};
-
-struct RescaleStore {
-    u64* arena;
-    const u64* qlinv;
-    const u64* qlinv_sh;
-    __device__ __forceinline__ void operator()(const LimbJob& j, const ZBases& zb, uint32_t z, uint32_t x, u64 v,
-                                               const PrimeConst& pc) const {
-        const u64 q = pc.q;
-        u64 a = arena[zb.src.at(z) + j.src + x];
-        u64 s = mul_shoup(a, __ldg(qlinv + j.aux), __ldg(qlinv_sh + j.aux), q);
-        arena[zb.out.at(z) + j.out + x] = add_mod(s, v, q);
-    }
-};
-
-// zb.src = input poly (arena), zb.out = output poly (arena), zb.mid = scratch
-// region of sizeQl * N words per z: words [0, N) hold the last limb's
-// coefficients, words [N, sizeQl * N) the step-2 intermediates.
-cudaError_t launch_rescale(int log_n, const OpTabs& t, const LimbJob* jobs_q, uint32_t sizeQl, u64* arena,
-                           u64* scratch, uint32_t nz, const ZBases& zb_in, cudaStream_t st) {
-    if (sizeQl < 2 || nz == 0) return cudaSuccess;
-    const u64 n = 1ull << log_n;
-    const uint32_t last = sizeQl - 1;
-    // step 1: INTT(last limb). jobs_q[last] has src = dst = out = last * N,
-    // so shifting mid / out back by last * N lands it at scratch + mid(z).
-    ZBases z1 = zb_in;
-    z1.mid = zf_plus(zb_in.mid, (u64)0 - (u64)last * n);
-    z1.out = z1.mid;
-    cudaError_t e = launch_ntt<true>(log_n, t.pt, jobs_q + last, 1, nz, scratch, z1, LoadPlain{arena},
-                                     StorePlain{scratch}, st);
-    if (e != cudaSuccess) return e;
-    // step 2
-    ZBases z2 = zb_in;
-    z2.aux = zb_in.mid;                      // coefficients of the last limb
-    z2.mid = zf_plus(zb_in.mid, n);          // intermediates
-    RescaleLoad pro{scratch, t.qlql, t.qlql_sh, t.pt.pc + last};
-    RescaleStore epi{arena, t.qlinv, t.qlinv_sh};
-    return launch_ntt<false>(log_n, t.pt, jobs_q, last, nz, scratch, z2, pro, epi, st);
-}
-
-// ---------------------------------------------------------------------------
-// key switch (key_switch.cpp:167-439)
-// ---------------------------------------------------------------------------
-// Scratch layout per polynomial (S = slots_q + K limb slots, Q limb i at slot
-// i, special limb k at slot slots_q + k):
-//   coef   : slots_q * N   INTT of the input's Q limbs, times qHatInv (ModUp's first factor)
-//   modup  : parts * S * N digit j's complementary limbs, evaluation form
-//   ext0   : S * N         sum_j digit_j * evk_b   (then ModDown input)
-//   ext1   : S * N         sum_j digit_j * evk_a
-//   mid    : 2 * slots_q * N  two-pass intermediates of the ModDown NTTs
-//   t0     : slots_q * N   c0 gathered through the automorphism (rotation)
-size_t ks_scratch_words(uint32_t n, uint32_t slots_q, uint32_t K, uint32_t parts) {
-    const size_t S = slots_q + K;
-    return (size_t)n * (slots_q + parts * S + 2 * S + 3 * (size_t)slots_q);
-}
-
-// Input load through the automorphism: the key switch of auto(c1) reads
-// c1[map[x]] (the reference applies automorphism() first, fhe_host_driver.cpp:342-350).
-struct LoadGather {
-    const u64* base;
-    const uint32_t* map;
-    ZField mapz;        // per-entry map addresses (per_z)
-    int per_z;
-    __device__ __forceinline__ u64 operator()(const LimbJob& j, const ZBases& zb, uint32_t z, uint32_t x,
-                                              const PrimeConst&) const {
-        const uint32_t* m = per_z ? (const uint32_t*)mapz.at(z) : map;
-        return base[zb.src.at(z) + j.src + __ldg(m + x)];
-    }
-};
-
-// Epilogue of the input's INTT: stores y_i = [x_i * qHatInv_i]_{q_i}, the
-// first factor of ModUp's base conversion (key_switch.cpp:7-60), once per
-// input limb instead of once per complementary output limb. job.aux = Q limb i.
-struct StoreQhatInv {
-    u64* scratch;
-    OpTabs t;
-    __device__ __forceinline__ void operator()(const LimbJob& j, const ZBases& zb, uint32_t z, uint32_t x, u64 v,
-                                               const PrimeConst& pc) const {
-        const uint32_t part = j.aux / t.alpha, idx = j.aux - part * t.alpha;
-        scratch[zb.out.at(z) + j.out + x] =
-            mul_shoup(v, __ldg(t.qhat_inv[part] + idx), __ldg(t.qhat_inv_sh[part] + idx), pc.q);
-    }
-};
-
-// Epilogue of the special limbs' INTT before ModDown: stores
-// [x_k * PHatInv_k]_{p_k}, the first factor of the P -> Q base conversion
-// (key_switch.cpp:62-163), once per special limb. job.aux = special limb k.
-struct StorePhatInv {
-    u64* scratch;
-    OpTabs t;
-    __device__ __forceinline__ void operator()(const LimbJob& j, const ZBases& zb, uint32_t z, uint32_t x, u64 v,
-                                               const PrimeConst& pc) const {
-        scratch[zb.out.at(z) + j.out + x] =
-            mul_shoup(v, __ldg(t.phat_inv_modp + j.aux), __ldg(t.phat_inv_modp_sh + j.aux), pc.q);
-    }
-};
-
-// ModUp base conversion as the NTT prologue: job.aux = digit << 16 | k, where
-// k is the output's position among the digit's complementary primes. Reads
-// y_i = [x_i * qHatInv_i]_{q_i} (StoreQhatInv) and sums y_i * [qHat_i]_p.
-struct ModUpLoad {
-    const u64* scratch;   // coef region at zb.aux[z]
-    OpTabs t;
-    uint32_t K;
-    uint32_t n;
-    __device__ __forceinline__ u64 operator()(const LimbJob& j, const ZBases& zb, uint32_t z, uint32_t x,
-                                              const PrimeConst& pc) const {
-        const uint32_t part = j.aux >> 16, k = j.aux & 0xFFFFu;
-        const uint32_t start = part * t.alpha;
-        const uint32_t size = (part == t.parts - 1) ? t.sizeQl - start : t.alpha;
-        const uint32_t row = t.sizeQl - size + K;   // complementary primes of this digit
-        const u64 p = pc.q, p2 = p << 1;
-        const u64* qm = t.qhat_modp[part];
-        const u64* qmsh = t.qhat_modp_sh[part];
-        u64 s = 0;
-        for (uint32_t i = 0; i < size; ++i) {
-            const uint32_t limb = start + i;
-            const u64 y = scratch[zb.aux.at(z) + (u64)limb * n + x];            // [x * qHatInv]_{q_i}
-            u64 w = mul_shoup_lazy(y, __ldg(qm + i * row + k), __ldg(qmsh + i * row + k), p);
-            s += w;
-            s = s >= p2 ? s - p2 : s;
-        }
-        return csub(s, p);
-    }
-};
-
-struct StoreSlot {   // plain store into scratch
-    u64* scratch;
-    __device__ __forceinline__ void operator()(const LimbJob& j, const ZBases& zb, uint32_t z, uint32_t x, u64 v,
-                                               const PrimeConst&) const {
-        scratch[zb.out.at(z) + j.out + x] = v;
-    }
-};
-
-// Inner product with the evaluation key. One thread per (slot, coefficient).
-// slot s < sizeQl is Q limb s, slot slots_q + k is special limb k.
-__global__ void __launch_bounds__(256) ks_mac_kernel(OpTabs t, uint32_t n, uint32_t slots_q, uint32_t sizeQl,
-                                                     uint32_t K, const u64* __restrict__ key, u64 evk_a, u64 evk_b,
-                                                     uint32_t key_stride, uint32_t key_pbase,
-                                                     const u64* __restrict__ arena, u64* __restrict__ scratch,
-                                                     u64 modup_off, u64 ext0_off, u64 ext1_off, u64 t0_off,
-                                                     const ZBases zb, const KsFuse f) {
-    const uint32_t sidx = blockIdx.y;   // 0..sizeQl+K-1
-    const uint32_t z = blockIdx.z;
-    const bool isq = sidx < sizeQl;
-    const uint32_t slot = isq ? sidx : slots_q + (sidx - sizeQl);
-    const uint32_t prime = isq ? sidx : t.p_base + (sidx - sizeQl);
-    const uint32_t klimb_in_digit = isq ? sidx : key_pbase + (sidx - sizeQl);
-    const PrimeConst pc = t.pt.pc[prime];
-    const ModConst mc = modconst_of(pc);
-    const u64 S = (u64)slots_q + K;
-    const u64 base_scr = zb.mid.at(z);
-    const u64* in = arena + zb.src.at(z) + (u64)sidx * n;   // only valid for Q limbs
-    const u64 c0_off = f.has_c0 ? f.c0.at(z) : 0;
-    const uint32_t* map = f.per_z ? (const uint32_t*)f.mapz.at(z) : f.map;
-    const u64 koff = f.per_z ? f.keyz.at(z) : 0;           // this entry's key (per_z)
-    for (uint32_t x = blockIdx.x * blockDim.x + threadIdx.x; x < n; x += gridDim.x * blockDim.x) {
-        const uint32_t xs = map ? __ldg(map + x) : x;         // position read through the automorphism
-        if (isq && f.has_c0)
-            scratch[base_scr + t0_off + (u64)sidx * n + x] = arena[c0_off + (u64)sidx * n + xs];
-        Acc128 ab, aa;
-        acc_init(ab);
-        acc_init(aa);
-        for (uint32_t part = 0; part < t.parts; ++part) {
-            const uint32_t start = part * t.alpha;
-            const uint32_t size = (part == t.parts - 1) ? sizeQl - start : t.alpha;
-            u64 d;
-            if (isq && sidx >= start && sidx < start + size) d = in[xs];
-            else d = scratch[base_scr + modup_off + ((u64)part * S + slot) * n + x];
-            const u64 kl = koff + ((u64)part * key_stride + klimb_in_digit) * n + x;
-            acc_mad(ab, d, __ldg(key + evk_b + kl));
-            acc_mad(aa, d, __ldg(key + evk_a + kl));
-        }
-        scratch[base_scr + ext0_off + (u64)slot * n + x] = acc_reduce(ab, mc);
-        scratch[base_scr + ext1_off + (u64)slot * n + x] = acc_reduce(aa, mc);
-    }
-}
-
-// ModDown base conversion P -> Q as the NTT prologue (job = Q limb i). Reads
-// [x_k * PHatInv_k]_{p_k} (StorePhatInv) and sums it times [PHat_k]_{q_i}.
-struct ModDownLoad {
-    const u64* scratch;  // ext region at zb.aux[z]
-    OpTabs t;
-    uint32_t slots_q, K, n;
-    __device__ __forceinline__ u64 operator()(const LimbJob& j, const ZBases& zb, uint32_t z, uint32_t x,
-                                              const PrimeConst& pc) const {
-        const u64 q = pc.q, q2 = q << 1;
-        const uint32_t i = j.aux;
-        u64 s = 0;
-        for (uint32_t k = 0; k < K; ++k) {
-            const u64 y = scratch[zb.aux.at(z) + (u64)(slots_q + k) * n + x];
-            u64 w = mul_shoup_lazy(y, __ldg(t.phat_modq + k * t.sizeQl + i), __ldg(t.phat_modq_sh + k * t.sizeQl + i), q);
-            s += w;
-            s = s >= q2 ? s - q2 : s;
-        }
-        return csub(s, q);
-    }
-};
-
-// ModDown combine as the NTT epilogue: out = (x_Q - y) * P^-1 mod q_i.
-// z' = 2z + h: h = 0 writes ks0 (+ gathered c0, + acc0), h = 1 writes ks1 (+ acc1).
-struct ModDownStore {
-    const u64* scratch;  // ext region at zb.src(z)
-    u64* arena;          // outputs
-    OpTabs t;
-    uint32_t n;
-    int has_c0, has_acc;
-    ZField t0;           // scratch offset of the gathered c0, per ciphertext
-    ZField out0, out1;   // ks0 / ks1 destinations, per ciphertext
-    ZField acc0, acc1;
-    __device__ __forceinline__ void operator()(const LimbJob& j, const ZBases& zb, uint32_t z, uint32_t x, u64 v,
-                                               const PrimeConst& pc) const {
-        const u64 q = pc.q;
-        const uint32_t i = j.aux;
-        const uint32_t h = z & 1u, zc = z >> 1;
-        const u64 li = (u64)i * n + x;
-        u64 xq = scratch[zb.src.at(z) + li];
-        u64 d = sub_mod(xq, v, q);
-        u64 r = mul_shoup(d, __ldg(t.p_inv_mod_q + i), __ldg(t.p_inv_mod_q_sh + i), q);
-        if (h == 0 && has_c0) r = add_mod(r, scratch[t0.at(zc) + li], q);
-        if (has_acc) r = add_mod(r, arena[(h ? acc1.at(zc) : acc0.at(zc)) + li], q);
-        arena[(h ? out1.at(zc) : out0.at(zc)) + li] = r;
-    }
-};
-
-cudaError_t launch_key_switch(int log_n, const OpTabs& t, const LimbJob* jobs_qp, const LimbJob* jobs_modup,
-                              uint32_t n_modup, uint32_t slots_q, uint32_t sizeQl, uint32_t K, const u64* key,
-                              u64 evk_a, u64 evk_b, uint32_t key_stride, uint32_t key_pbase, u64* arena,
-                              u64* scratch, uint32_t nz, const ZBases& zb, cudaStream_t st, const KsFuse* fuse) {
-    if (nz == 0) return cudaSuccess;
-    if (2ull * nz > 65535ull) return cudaErrorInvalidValue;
-    KsFuse f{};
-    if (fuse) f = *fuse;
-    const u64 n = 1ull << log_n;
-    const u64 S = (u64)slots_q + K;
-    const u64 off_coef = 0;
-    const u64 off_modup = off_coef + (u64)slots_q * n;
-    const u64 off_ext0 = off_modup + (u64)t.parts * S * n;
-    const u64 off_ext1 = off_ext0 + S * n;
-    const u64 off_mid = off_ext1 + S * n;
-    const u64 off_t0 = off_mid + 2ull * slots_q * n;
-    cudaError_t e;
-
-    // 1. INTT of the input's Q limbs -> coef (slot i at coef + i*N)
-    {
-        ZBases a = zb;
-        a.mid = zf_plus(zb.mid, off_coef);
-        a.out = a.mid;
-        if (f.map || f.per_z)
-            e = launch_ntt<true>(log_n, t.pt, jobs_qp, sizeQl, nz, scratch, a,
-                                 LoadGather{arena, f.map, f.mapz, f.per_z}, StoreQhatInv{scratch, t}, st);
-        else
-            e = launch_ntt<true>(log_n, t.pt, jobs_qp, sizeQl, nz, scratch, a, LoadPlain{arena},
-                                 StoreQhatInv{scratch, t}, st);
-        if (e != cudaSuccess) return e;
-    }
-    // 2. ModUp: base conversion + NTT for every (digit, complementary limb)
-    {
-        ZBases a = zb;
-        a.aux = zf_plus(zb.mid, off_coef);
-        a.mid = zf_plus(zb.mid, off_modup);
-        a.out = a.mid;
-        ModUpLoad pro{scratch, t, K, (uint32_t)n};
-        e = launch_ntt<false>(log_n, t.pt, jobs_modup, n_modup, nz, scratch, a, pro, StoreSlot{scratch}, st);
-        if (e != cudaSuccess) return e;
-    }
-    // 3. inner product with the key
-    {
-        dim3 grid((uint32_t)((n + 255) / 256), sizeQl + K, nz);
-        ks_mac_kernel<<<grid, 256, 0, st>>>(t, (uint32_t)n, slots_q, sizeQl, K, key, evk_a, evk_b, key_stride,
-                                            key_pbase, arena, scratch, off_modup, off_ext0, off_ext1, off_t0, zb, f);
-        count_launches(1);
-        e = cudaGetLastError();
-        if (e != cudaSuccess) return e;
-    }
-    // 4. ModDown of both accumulators: z' = 2z (ext0 -> ks0), 2z + 1 (ext1 -> ks1)
-    {
-        ZBases a{};
-        a.src = zf_pair(zf_plus(zb.mid, off_ext0), off_ext1 - off_ext0);
-        a.aux = a.src;
-        a.mid = a.src;
-        a.out = a.src;
-        // 4a. INTT of the special limbs, in place, times PHatInv
-        e = launch_ntt<true>(log_n, t.pt, jobs_qp + slots_q, K, 2 * nz, scratch, a, LoadPlain{scratch},
-                             StorePhatInv{scratch, t}, st);
-        if (e != cudaSuccess) return e;
-        // 4b. NTT over Q limbs with base-conversion prologue and ModDown epilogue
-        ZBases b = a;
-        b.mid = zf_pair(zf_plus(zb.mid, off_mid), (u64)slots_q * n);
-        ModDownLoad pro{scratch, t, slots_q, K, (uint32_t)n};
-        ModDownStore epi{};
-        epi.scratch = scratch;
-        epi.arena = arena;
-        epi.t = t;
-        epi.n = (uint32_t)n;
-        epi.has_c0 = f.has_c0;
-        epi.has_acc = f.has_acc;
-        epi.t0 = zf_plus(zb.mid, off_t0);
-        epi.out0 = zb.out;
-        epi.out1 = zb.aux;
-        epi.acc0 = f.acc0;
-        epi.acc1 = f.acc1;
-        e = launch_ntt<false>(log_n, t.pt, jobs_qp, sizeQl, 2 * nz, scratch, b, pro, epi, st);
-        if (e != cudaSuccess) return e;
-    }
-    return cudaSuccess;
-}
-
-// ---------------------------------------------------------------------------
 // table preparation
 // ---------------------------------------------------------------------------
 __global__ void companions_kernel(u64* v, u64* sh, const u64* m, size_t count) {
@@ -827,22 +497,32 @@ cudaError_t launch_companions(u64* v, u64* sh, const u64* m, size_t count, cudaS
     return cudaGetLastError();
 }
 
-__global__ void interleave_kernel(const u64* raw, const u64* q, ulonglong2* out2, uint32_t rows, uint32_t n) {
-    const size_t total = (size_t)rows * n;
+__global__ void twiddles_kernel(const u64* __restrict__ raw, const u64* __restrict__ q, ulonglong2* __restrict__ out2,
+                                ulonglong2* __restrict__ out2b, uint32_t rows, int log_n) {
+    const size_t total = (size_t)rows << log_n;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-        const u64 m = q[i / n];
-        const u64 w = raw[i] % m;
-        out2[i] = make_ulonglong2(w, shoup_companion(w, m));
+        const size_t row = i >> log_n;
+        const uint32_t j = (uint32_t)(i & ((1u << log_n) - 1));
+        const u64 m = q[row];
+        u64 o[4];
+        transform_constant(raw[i] % m, m, o);
+        uint32_t at = 0;                       // j = 0 belongs to no stage
+        if (j) {
+            const int lg = 31 - __clz((int)j);
+            at = tw_place(log_n, log_n - 1 - lg, j - (1u << lg));
+        }
+        out2[(row << log_n) + at] = make_ulonglong2(o[0], o[1]);
+        out2b[(row << log_n) + at] = make_ulonglong2(o[2], o[3]);
     }
 }
 
-cudaError_t launch_interleave(const u64* raw, const u64* q, ulonglong2* out2, uint32_t rows, uint32_t n,
-                              cudaStream_t st) {
+cudaError_t launch_twiddles(const u64* raw, const u64* q, ulonglong2* out2, ulonglong2* out2b, uint32_t rows, int log_n,
+                            cudaStream_t st) {
     if (rows == 0) return cudaSuccess;
-    size_t total = (size_t)rows * n;
+    const size_t total = (size_t)rows << log_n;
     unsigned blocks = (unsigned)((total + 255) / 256);
     if (blocks > 8192) blocks = 8192;
-    interleave_kernel<<<blocks, 256, 0, st>>>(raw, q, out2, rows, n);
+    twiddles_kernel<<<blocks, 256, 0, st>>>(raw, q, out2, out2b, rows, log_n);
     count_launches(1);
     return cudaGetLastError();
 }
@@ -861,6 +541,7 @@ __global__ void prime_consts_kernel(PrimeConst* pc, const u64* q, const u64* nin
     c.ninv_sh = shoup_companion(c.ninv, c.q);
     c.w1ninv = mul_mod(itw[(u64)i * n + 1] % c.q, c.ninv, m);
     c.w1ninv_sh = shoup_companion(c.w1ninv, c.q);
+    set_transform_constants(c);
     pc[i] = c;
 }
 

@@ -1,0 +1,70 @@
+// rescale.cu -- rescale (hardware_fpga_model/hls/src/rescale.cpp:3-72): two
+// transforms, with the lift of the dropped limb as the second one's prologue
+// and the combine as its epilogue.
+#include "internal.h"
+
+namespace afhe {
+
+// ---------------------------------------------------------------------------
+// rescale (rescale.cpp:3-72)
+//   step 1: INTT of the last limb -> coefficients in scratch
+//   step 2: NTT over limbs i < L-1 whose prologue is the centred lift of the
+//           last limb times QlQlInvModqlDivqlModq[i], and whose epilogue is
+//           a_i * qlInvModq[i] + NTT(...)
+// ---------------------------------------------------------------------------
+struct RescaleLoad {
+    const u64* scratch;
+    const u64* qlql;
+    const u64* qlql_sh;
+    const PrimeConst* pc_last;   // q_l, the prime being dropped
+    __device__ __forceinline__ u64 operator()(const LimbJob& j, const ZBases& zb, uint32_t z, u64 x,
+                                              const PrimeConst& pc) const {
+        const u64 q = pc.q;
+        const u64 ql = pc_last->q, ql_half = ql >> 1;
+        u64 v = scratch[zb.aux.at(z) + x];                           // last limb coefficient, [0, q_l)
+        u64 vm = csub(mul_shoup_lazy(v, 1, pc.one_sh, q), q);         // v mod q_i
+        u64 qlm = csub(mul_shoup_lazy(ql, 1, pc.one_sh, q), q);       // q_l mod q_i
+        u64 val = (v > ql_half) ? sub_mod(vm, qlm, q) : vm;           // rescale.cpp:50 tie rule
+        return mul_shoup(val, __ldg(qlql + j.aux), __ldg(qlql_sh + j.aux), q);
+    }
+};
+
+struct RescaleStore {
+    u64* arena;
+    const u64* qlinv;
+    const u64* qlinv_sh;
+    __device__ __forceinline__ void operator()(const LimbJob& j, const ZBases& zb, uint32_t z, u64 x, u64 v,
+                                               const PrimeConst& pc) const {
+        const u64 q = pc.q;
+        u64 a = arena[zb.src.at(z) + j.src + x];
+        u64 s = mul_shoup(a, __ldg(qlinv + j.aux), __ldg(qlinv_sh + j.aux), q);
+        arena[zb.out.at(z) + j.out + x] = add_mod(s, v, q);
+    }
+};
+
+// zb.src = input poly (arena), zb.out = output poly (arena), zb.mid = scratch
+// region of sizeQl * N words per z: words [0, N) hold the last limb's
+// coefficients, words [N, sizeQl * N) the step-2 intermediates.
+cudaError_t launch_rescale(int log_n, const OpTabs& t, const LimbJob* jobs_q, uint32_t sizeQl, u64* arena,
+                           u64* scratch, uint32_t nz, const ZBases& zb_in, cudaStream_t st) {
+    if (sizeQl < 2 || nz == 0) return cudaSuccess;
+    const u64 n = 1ull << log_n;
+    const uint32_t last = sizeQl - 1;
+    // step 1: INTT(last limb). jobs_q[last] has src = dst = out = last * N,
+    // so shifting mid / out back by last * N lands it at scratch + mid(z).
+    ZBases z1 = zb_in;
+    z1.mid = zf_plus(zb_in.mid, (u64)0 - (u64)last * n);
+    z1.out = z1.mid;
+    cudaError_t e = launch_ntt<true>(log_n, t.pt, jobs_q + last, 1, nz, scratch, z1, LoadPlain{arena},
+                                     StorePlain{scratch}, st);
+    if (e != cudaSuccess) return e;
+    // step 2
+    ZBases z2 = zb_in;
+    z2.aux = zb_in.mid;                      // coefficients of the last limb
+    z2.mid = zf_plus(zb_in.mid, n);          // intermediates
+    RescaleLoad pro{scratch, t.qlql, t.qlql_sh, t.pt.pc + last};
+    RescaleStore epi{arena, t.qlinv, t.qlinv_sh};
+    return launch_ntt<false>(log_n, t.pt, jobs_q, last, nz, scratch, z2, pro, epi, st);
+}
+
+}  // namespace afhe
