@@ -16,7 +16,9 @@
 
 #include <algorithm>
 #include <cstdlib>
+#include <cstring>
 #include <map>
+#include <tuple>
 #include <vector>
 
 #include "internal.h"
@@ -229,6 +231,29 @@ bool fused_rotation_safe(const Offs& i0, const Offs& i1, const Offs& o0, const O
             auto it = std::lower_bound(outs.begin(), outs.end(), std::make_pair(lo, 0u));
             for (; it != outs.end() && it->first < a + w; ++it)
                 if (it->second != z || it->first != a) return false;
+        }
+    return true;
+}
+
+// Whether a rescale may read its inputs where they are: every output polynomial
+// is disjoint from every input polynomial (inputs span w words, outputs less),
+// or starts where its own input does.
+bool rescale_in_place_safe(const Offs& i0, const Offs& i1, const Offs& o0, const Offs& o1, u64 w) {
+    const size_t nz = i0.size();
+    std::vector<std::pair<u64, size_t>> outs;       // (start, polynomial)
+    outs.reserve(2 * nz);
+    for (size_t z = 0; z < nz; ++z) {
+        outs.emplace_back(o0[z], 2 * z);
+        outs.emplace_back(o1[z], 2 * z + 1);
+    }
+    std::sort(outs.begin(), outs.end());
+    for (size_t z = 0; z < nz; ++z)
+        for (size_t h = 0; h < 2; ++h) {
+            const u64 a = h ? i1[z] : i0[z];
+            const u64 lo = a >= w ? a - w + 1 : 0;
+            for (auto it = std::lower_bound(outs.begin(), outs.end(), std::make_pair(lo, (size_t)0));
+                 it != outs.end() && it->first < a + w; ++it)
+                if (it->first != a || it->second != 2 * z + h) return false;
         }
     return true;
 }
@@ -539,9 +564,18 @@ int afhe_rescale_batch(afhe_ctx* ctx, const afhe_ct_ref* a, const afhe_ct_ref* d
     if ((rc = check_limbs(ctx, limbs, 2)) || (rc = check_cts(ctx, a, count, limbs)) ||
         (rc = check_cts(ctx, d, count, limbs - 1)))
         return rc;
-    // OP 8 on both polynomials (fhe_accel_top.cpp:286-292); the inputs go to
-    // lane temps first, so outputs may alias any input
+    // OP 8 on both polynomials (fhe_accel_top.cpp:286-292). A polynomial is read
+    // and written word by word in place, so an output may lie on its own input;
+    // where one overlaps an input otherwise, the inputs go to lane temps first.
     return for_chunks(ctx, count, [&](uint32_t s, uint32_t m) {
+        {
+            Offs i0(m), i1(m), o0(m), o1(m);
+            for (uint32_t z = 0; z < m; ++z) {
+                i0[z] = a[s + z].c0_offset; i1[z] = a[s + z].c1_offset;
+                o0[z] = d[s + z].c0_offset; o1[z] = d[s + z].c1_offset;
+            }
+            if (rescale_in_place_safe(i0, i1, o0, o1, (u64)limbs * ctx->n)) return rescale_batch(ctx, i0, i1, o0, o1, limbs);
+        }
         Offs A(2 * m), T(2 * m), t0(m), t1(m), o0(m), o1(m);
         for (uint32_t z = 0; z < m; ++z) {
             t0[z] = lane_temp(ctx, z, 0);
@@ -989,40 +1023,106 @@ int afhe_eval_diag_inner_batch(afhe_ctx* ctx, const afhe_ct_ref* out, uint32_t c
                 staged = ctx->auto_map_local[unit_galois[k]];
             }
         }
+    // Runs of outputs with the same sources and the same units, but for one
+    // distance between their plaintexts (a result's giant steps), share their
+    // descriptors.
+    auto follows = [&](uint32_t j) -> bool {       // output j continues the run of output j - 1
+        const uint32_t a = first_unit[j - 1], b = first_unit[j], nu = first_unit[j + 1] - b;
+        if (b - a != nu || memcmp(src + (u64)(j - 1) * nb, src + (u64)j * nb, nb * sizeof(afhe_ct_ref))) return false;
+        for (uint32_t k = 0; k < nu; ++k)
+            if (unit_galois[a + k] != unit_galois[b + k] || unit_pt[b + k] - unit_pt[a + k] != unit_pt[b] - unit_pt[a])
+                return false;
+        return true;
+    };
     const size_t seg = ctx->ring.seg_words - 96;
+    const u64 tiles = (u64)limbs * ((ctx->n + 255) / 256);
     std::vector<DiagJob> J;
+    std::vector<uint32_t> step;             // output's place in its run
     std::vector<u64> S;
     std::vector<DiagUnit> U;
+    std::multimap<u64, std::pair<uint32_t, uint32_t>> lists;    // hash of a run's units -> their [u0, u1) in U
     auto flush = [&]() -> int {
         if (J.empty()) return AFHE_OK;
-        u64 *dj = nullptr, *ds = nullptr, *du = nullptr;
+        // Outputs at the same place of their runs side by side: a run's
+        // sources stay in L2 from one place to the next. Among them those
+        // with the same plaintexts (queries that scan the same list) form
+        // groups, whose plaintexts are read and added up once; a group ends
+        // where larger ones would leave too few blocks (4 an SM).
+        std::vector<uint32_t> by(J.size());
+        for (uint32_t i = 0; i < by.size(); ++i) by[i] = i;
+        std::stable_sort(by.begin(), by.end(), [&](uint32_t x, uint32_t y) {
+            return std::tie(step[x], J[x].u0, J[x].add) < std::tie(step[y], J[y].u0, J[y].add);
+        });
+        const u64 most = std::max<u64>(1, J.size() * tiles / (4 * 148));
+        std::vector<DiagJob> ordered;
+        std::vector<DiagGroup> G;
+        for (uint32_t i : by) {
+            const DiagJob& p = J[i];
+            if (G.empty() || G.back().count >= most || ordered.back().u0 != p.u0 || ordered.back().u1 != p.u1 ||
+                ordered.back().add != p.add)
+                G.push_back(DiagGroup{(uint32_t)ordered.size(), 0});
+            ++G.back().count;
+            ordered.push_back(p);
+        }
+        u64 *dg = nullptr, *dj = nullptr, *ds = nullptr, *du = nullptr;
         int r;
         if (U.empty()) U.push_back(DiagUnit{0, nullptr});
-        if ((r = ring_put(ctx, J.data(), J.size() * sizeof(DiagJob) / sizeof(u64), &dj))) return r;
+        if ((r = ring_put(ctx, G.data(), G.size() * sizeof(DiagGroup) / sizeof(u64), &dg))) return r;
+        if ((r = ring_put(ctx, ordered.data(), J.size() * sizeof(DiagJob) / sizeof(u64), &dj))) return r;
         if ((r = ring_put(ctx, S.data(), S.size(), &ds))) return r;
         if ((r = ring_put(ctx, U.data(), U.size() * sizeof(DiagUnit) / sizeof(u64), &du))) return r;
-        CK(launch_diag_inner(ctx->nat.pc, ctx->poly, ctx->n, limbs, (uint32_t)J.size(), nb, (const DiagJob*)dj, ds,
-                             (const DiagUnit*)du, pt_stride, reduce_every, accumulate ? 1 : 0, staged,
+        CK(launch_diag_inner(ctx->nat.pc, ctx->poly, ctx->n, limbs, (uint32_t)G.size(), nb, (const DiagGroup*)dg,
+                             (const DiagJob*)dj, ds, (const DiagUnit*)du, pt_stride, accumulate ? 1 : 0, staged,
                              qmax < (1ull << 50), ctx->st));
         J.clear();
+        step.clear();
         S.clear();
         U.clear();
+        lists.clear();
         return AFHE_OK;
     };
+    constexpr size_t jw = sizeof(DiagJob) / sizeof(u64);
     for (uint32_t j = 0; j < count; ++j) {
         const size_t nu = first_unit[j + 1] - first_unit[j];
-        if (3 + 2 * nb + 2 * nu + 2 > seg / 3) return fail(ctx, AFHE_E_ARG, "too many units in one output for the descriptor ring");
-        if ((J.size() + 1) * 3 > seg / 3 || S.size() + 2 * nb > seg / 3 || (U.size() + nu + 1) * 2 > seg / 3)
+        if (jw + 2 * nb + 2 * nu + 2 > seg) return fail(ctx, AFHE_E_ARG, "too many units in one output for the descriptor ring");
+        if ((J.size() + 1) * jw > seg || S.size() + 2 * nb > seg || (U.size() + nu + 1) * 2 > seg)
             if ((rc = flush())) return rc;
-        J.push_back(DiagJob{out[j].c0_offset, out[j].c1_offset, (uint32_t)U.size(), (uint32_t)(U.size() + nu)});
-        for (uint32_t b = 0; b < nb; ++b) {
-            S.push_back(src[(u64)j * nb + b].c0_offset);
-            S.push_back(src[(u64)j * nb + b].c1_offset);
+        if (!J.empty() && follows(j)) {
+            DiagJob n = J.back();
+            n.out0 = out[j].c0_offset;
+            n.out1 = out[j].c1_offset;
+            if (nu) n.add += unit_pt[first_unit[j]] - unit_pt[first_unit[j - 1]];
+            J.push_back(n);
+            step.push_back(step.back() + 1);
+            continue;
         }
+        u64 hash = nu;
         for (uint32_t k = first_unit[j]; k < first_unit[j + 1]; ++k) {
             const uint32_t* map = nullptr;
             if (unit_galois[k] != 1 && (rc = cached_map(ctx, unit_galois[k], &map))) return rc;
             U.push_back(DiagUnit{unit_pt[k], map});
+            hash = (hash ^ unit_pt[k] ^ ((u64)unit_galois[k] << 40)) * 0x9e3779b97f4a7c15ull;
+        }
+        // a run's units that an earlier run has too are kept once
+        uint32_t u1 = (uint32_t)U.size(), u0 = u1 - (uint32_t)nu;
+        bool found = false;
+        for (auto it = lists.lower_bound(hash); it != lists.end() && it->first == hash && !found; ++it) {
+            const uint32_t a = it->second.first;
+            found = it->second.second - a == nu && std::equal(U.begin() + u0, U.end(), U.begin() + a, [](const DiagUnit& x, const DiagUnit& y) {
+                return x.pt == y.pt && x.map == y.map;
+            });
+            if (found) {
+                U.resize(u0);
+                u0 = a;
+                u1 = a + (uint32_t)nu;
+            }
+        }
+        if (!found) lists.insert({hash, {u0, u1}});
+        J.push_back(DiagJob{out[j].c0_offset, out[j].c1_offset, 0, u0, u1, (uint32_t)(S.size() / 2), 0});
+        step.push_back(0);
+        for (uint32_t b = 0; b < nb; ++b) {
+            S.push_back(src[(u64)j * nb + b].c0_offset);
+            S.push_back(src[(u64)j * nb + b].c1_offset);
         }
     }
     return flush();

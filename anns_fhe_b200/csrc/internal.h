@@ -205,22 +205,32 @@ struct MacTerm {
 };
 // The diagonal method's inner products (afhe_eval_diag_inner_batch): job z
 // writes out = sum over its units k of sum over b < nb of
-// pt_k[b stride + map_k[i]] * src_{z, b}, srcs[z nb + b] = (c0, c1) offsets.
+// pt_k[add + b stride + map_k[i]] * src_b, src_b = (c0, c1) offsets at
+// srcs[2 (s + b)]. Jobs of one result share their units and sources and differ
+// in `add` (the giant step). Neighbouring jobs run side by side on the same
+// coefficients.
 // staged: every map keeps 256-word tiles within themselves, every plaintext
 // offset and the stride are even and N is a multiple of 256 (the
-// shared-memory form); halves (staged only): every prime is below 2^50
-// (25-bit split products).
+// shared-memory form); halves: every prime is below 2^50 (25-bit split
+// products).
 struct DiagJob {
     u64 out0, out1;
+    u64 add;
     uint32_t u0, u1;
+    uint32_t s, pad;
 };
 struct DiagUnit {
     u64 pt;
     const uint32_t* map;   // null: identity
 };
-cudaError_t launch_diag_inner(const PrimeConst* pc, u64* arena, uint32_t n, uint32_t limbs, uint32_t jobs,
-                              uint32_t nb, const DiagJob* job, const u64* srcs, const DiagUnit* unit, u64 stride,
-                              uint32_t reduce_every, int accumulate, bool staged, bool halves, cudaStream_t st);
+// outputs [first, first + count) share u0, u1 and add
+struct DiagGroup {
+    uint32_t first, count;
+};
+cudaError_t launch_diag_inner(const PrimeConst* pc, u64* arena, uint32_t n, uint32_t limbs, uint32_t groups,
+                              uint32_t nb, const DiagGroup* group, const DiagJob* job, const u64* srcs,
+                              const DiagUnit* unit, u64 stride, int accumulate, bool staged, bool halves,
+                              cudaStream_t st);
 cudaError_t launch_mac_plain(const PrimeConst* pc, u64* arena, uint32_t n, uint32_t limbs, uint32_t jobs,
                              const MacJob* job, const MacGroup* group, const MacTerm* term, uint32_t reduce_every,
                              int accumulate, cudaStream_t st);

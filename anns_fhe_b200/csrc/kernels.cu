@@ -201,75 +201,6 @@ __global__ void __launch_bounds__(256) mac_plain_kernel(const PrimeConst* __rest
     arena[J.out1 + off] = r1;
 }
 
-// One coefficient per thread: the nb baby-step ciphertexts' coefficients stay
-// in registers while the job's units stream through; a unit's automorphism
-// index is loaded once for its nb plaintexts, which lie `stride` words apart.
-template <int NB>
-__global__ void __launch_bounds__(256) diag_inner_kernel(const PrimeConst* __restrict__ pc, u64* __restrict__ arena,
-                                                         uint32_t n, const DiagJob* __restrict__ jobs,
-                                                         const u64* __restrict__ srcs,
-                                                         const DiagUnit* __restrict__ units, u64 stride,
-                                                         uint32_t reduce_every, int accumulate) {
-    const uint32_t l = blockIdx.y;
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const DiagJob J = jobs[blockIdx.z];
-    const ModConst m = modconst_of(pc[l]);
-    const u64 off = (u64)l * n;
-    const u64* s = srcs + (u64)blockIdx.z * 2 * NB;
-    u64 x0[NB], x1[NB];
-#pragma unroll
-    for (int b = 0; b < NB; ++b) {
-        x0[b] = arena[s[2 * b] + off + i];
-        x1[b] = arena[s[2 * b + 1] + off + i];
-    }
-    Acc128 a0, a1;
-    acc_init(a0);
-    acc_init(a1);
-    uint32_t cnt = 0;
-    // the next unit's descriptor and automorphism index are loaded while the
-    // current unit's plaintexts are read and multiplied
-    DiagUnit Un{};
-    uint32_t jn = i;
-    if (J.u0 < J.u1) {
-        Un = units[J.u0];
-        jn = Un.map ? __ldg(Un.map + i) : i;
-    }
-    for (uint32_t k = J.u0; k < J.u1; ++k) {
-        const u64* p = arena + Un.pt + off + jn;
-        if (k + 1 < J.u1) {
-            Un = units[k + 1];
-            jn = Un.map ? __ldg(Un.map + i) : i;
-        }
-        if (cnt + NB > reduce_every) {
-            acc_fold(a0, m);
-            acc_fold(a1, m);
-            cnt = 1;
-        }
-#pragma unroll
-        for (int b = 0; b < NB; ++b) {
-            const u64 v = p[(u64)b * stride];
-            acc_mad(a0, v, x0[b]);
-            acc_mad(a1, v, x1[b]);
-        }
-        cnt += NB;
-    }
-    u64 r0 = acc_reduce(a0, m), r1 = acc_reduce(a1, m);
-    if (accumulate) {
-        r0 = add_mod(r0, arena[J.out0 + off + i], m.q);
-        r1 = add_mod(r1, arena[J.out1 + off + i], m.q);
-    }
-    arena[J.out0 + off + i] = r0;
-    arena[J.out1 + off + i] = r1;
-}
-
-// The same sums with the plaintexts staged through shared memory: every
-// placement map of the launch keeps each 256-coefficient tile within itself
-// (a slot rotation by a multiple of D permutes the evaluation form inside
-// blocks of N / 2D words), so a CTA copies the tile of all nb plaintexts of
-// its next unit with cp.async while it multiplies the current one
-// (double-buffered), and gathers from shared memory. One coefficient per
-// thread, 256 threads: tile t = coefficients [256 t, 256 t + 256).
 __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
     const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem) : "memory");
@@ -278,20 +209,22 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int K>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(K) : "memory"); }
 
-constexpr uint32_t kDiagTile = 256;
+constexpr uint32_t kDiagTile = 256, kDiagUnits = 128;
 
 // Residues below 2^50: operands split into 25-bit halves, x = x1 2^25 + x0;
 // the partial sums x0 y0, x0 y1 + x1 y0, x1 y1 of the products accumulate
 // in 64-bit registers by single 32 x 32 + 64 multiply-adds (products of
-// halves < 2^50: 4,096 products fit between folds); recombined in 128 bits.
-constexpr uint32_t kHalfBits = 25, kHalfMask = (1u << kHalfBits) - 1, kHalfFold = 4096;
+// halves below 2^57: room for 32 of the middle ones, used for at most 16 of
+// them twice); recombined in 128 bits.
+constexpr uint32_t kHalfBits = 25, kHalfMask = (1u << kHalfBits) - 1;
 __device__ __forceinline__ void mad_wide(u64& acc, uint32_t a, uint32_t b) {
     asm("mad.wide.u32 %0, %1, %2, %0;" : "+l"(acc) : "r"(a), "r"(b));
 }
 struct Halves {
     u64 s00, s01, s11;
 };
-__device__ __forceinline__ void halves_mad(Halves& h, uint32_t v0, uint32_t v1, uint32_t x0, uint32_t x1) {
+__device__ __forceinline__ void halves_mad(Halves& h, uint32_t v0, uint32_t v1, u64 x) {
+    const uint32_t x0 = (uint32_t)x & kHalfMask, x1 = (uint32_t)(x >> kHalfBits);
     mad_wide(h.s00, v0, x0);
     mad_wide(h.s01, v0, x1);
     mad_wide(h.s01, v1, x0);
@@ -307,151 +240,233 @@ __device__ __forceinline__ u64 halves_reduce(const Halves& h, const ModConst& m)
     return reduce128(hi, lo, m);
 }
 
+// The diagonal method's inner products, out = sum over units u, baby steps b of
+// plaintext(u, b) x(b). Every unit of an output meets the same baby steps, so
+// a thread first adds up its coefficient of the units' plaintexts (a sum for
+// each of the nb baby steps) and then multiplies: nb products an output instead
+// of nb times its units. The sums hold for every output of
+// a group (results of other baby steps with the same units: queries that scan
+// the same list), so a group's plaintexts are read once too; what is left is
+// the reading of each output's 2 nb coefficients, from L2 where the outputs of
+// neighbouring CTAs share their baby steps.
+// HALVES: primes below 2^50; sums of up to kDiagUnits residues are below 2^57, a
+// 25-bit half and a 32-bit one, and multiply as they are. Else the sums have
+// 96 bits and are reduced once. One coefficient per thread, tile t =
+// coefficients [256 t, 256 t + 256); groups vary fastest across the grid, so
+// consecutive CTAs are other groups of the same tile.
 template <int NB, bool HALVES>
-__global__ void __launch_bounds__(kDiagTile) diag_inner_staged_kernel(
-    const PrimeConst* __restrict__ pc, u64* __restrict__ arena, uint32_t n, const DiagJob* __restrict__ jobs,
-    const u64* __restrict__ srcs, const DiagUnit* __restrict__ units, u64 stride, uint32_t reduce_every,
-    int accumulate) {
-    extern __shared__ u64 stage[];          // 2 buffers x NB plaintexts x kDiagTile words
-    // jobs vary fastest across the grid: consecutive CTAs are other outputs
-    // of the same tile, so outputs that share their baby steps (one query's
-    // giant steps) read them from L2
-    const uint32_t z = blockIdx.x, l = blockIdx.z, tid = threadIdx.x;
-    const uint32_t base = blockIdx.y * kDiagTile, i = base + tid;
-    const DiagJob J = jobs[z];
-    const ModConst m = modconst_of(pc[l]);
-    const u64 off = (u64)l * n;
-    const u64* s = srcs + (u64)z * 2 * NB;
-    u64 x0[HALVES ? 1 : NB], x1[HALVES ? 1 : NB];
-    uint32_t h00[HALVES ? NB : 1], h01[HALVES ? NB : 1], h10[HALVES ? NB : 1], h11[HALVES ? NB : 1];
+struct DiagSums {
+    u64 p[NB];
+    uint32_t hi[HALVES ? 1 : NB];
+    __device__ __forceinline__ DiagSums() {
 #pragma unroll
-    for (int b = 0; b < NB; ++b) {
-        const u64 y0 = arena[s[2 * b] + off + i], y1 = arena[s[2 * b + 1] + off + i];
-        if (HALVES) {
-            h00[b] = (uint32_t)y0 & kHalfMask;
-            h01[b] = (uint32_t)(y0 >> kHalfBits);
-            h10[b] = (uint32_t)y1 & kHalfMask;
-            h11[b] = (uint32_t)(y1 >> kHalfBits);
-        } else {
-            x0[b] = y0;
-            x1[b] = y1;
+        for (int b = 0; b < NB; ++b) p[b] = 0;
+#pragma unroll
+        for (int b = 0; b < (HALVES ? 1 : NB); ++b) hi[b] = 0;
+    }
+    // unit k's plaintexts, `stride` words apart
+    __device__ __forceinline__ void add(uint32_t k, const u64* t, u64 stride, const ModConst& m) {
+#pragma unroll
+        for (int b = 0; b < NB; ++b) {
+            const u64 v = t[b * stride];
+            p[b] += v;
+            if (!HALVES) hi[b] += p[b] < v ? 1u : 0u;
+        }
+        if (HALVES && k % (kDiagUnits - 1) == kDiagUnits - 2) {
+#pragma unroll 1
+            for (int b = 0; b < NB; ++b) {      // rotates through the array: one copy of the reduction
+                const u64 r = reduce128(0, p[0], m);
+#pragma unroll
+                for (int c = 0; c + 1 < NB; ++c) p[c] = p[c + 1];
+                p[NB - 1] = r;
+            }
         }
     }
-    // unit k's tile of its NB plaintexts into buffer `buf`: NB x 128 chunks of 16 bytes
-    auto issue = [&](uint32_t k, uint32_t buf) {
-        const u64* g = arena + units[k].pt + off + base;
-        u64* d = stage + (size_t)buf * NB * kDiagTile;
-        for (uint32_t c = tid; c < NB * (kDiagTile / 2); c += kDiagTile) {
-            const uint32_t b = c / (kDiagTile / 2), w = (c % (kDiagTile / 2)) * 2;
-            cp_async16(d + b * kDiagTile + w, g + (u64)b * stride + w);
+    // after the last unit: residues, or their halves side by side
+    __device__ __forceinline__ void close(const ModConst& m) {
+#pragma unroll
+        for (int b = 0; b < NB; ++b)
+            p[b] = HALVES ? (p[b] >> kHalfBits << 32 | ((uint32_t)p[b] & kHalfMask)) : reduce128(hi[HALVES ? 0 : b], p[b], m);
+    }
+    template <typename X>
+    __device__ __forceinline__ u64 times(X&& x, const ModConst& m) const {
+        if (HALVES) {
+            Halves c{0, 0, 0};
+#pragma unroll
+            for (int b = 0; b < NB; ++b) halves_mad(c, (uint32_t)p[b], (uint32_t)(p[b] >> 32), x(b));
+            return halves_reduce(c, m);
+        }
+        Acc128 a;
+        acc_init(a);
+#pragma unroll
+        for (int b = 0; b < NB; ++b) acc_mad(a, p[b], x(b));
+        return acc_reduce(a, m);
+    }
+};
+
+// Plaintexts and baby steps straight from global memory: any placement map,
+// any alignment.
+template <int NB, bool HALVES>
+__global__ void __launch_bounds__(kDiagTile) diag_inner_kernel(
+    const PrimeConst* __restrict__ pc, u64* __restrict__ arena, uint32_t n, const DiagGroup* __restrict__ groups,
+    const DiagJob* __restrict__ jobs, const u64* __restrict__ srcs, const DiagUnit* __restrict__ units, u64 stride,
+    int accumulate) {
+    const uint32_t l = blockIdx.z, i = blockIdx.y * kDiagTile + threadIdx.x;
+    if (i >= n) return;
+    const DiagGroup G = groups[blockIdx.x];
+    const ModConst m = modconst_of(pc[l]);
+    arena += (u64)l * n;
+    DiagSums<NB, HALVES> sums;
+    const DiagJob J = jobs[G.first];
+    for (uint32_t k = J.u0; k < J.u1; ++k) {
+        const DiagUnit U = units[k];
+        sums.add(k - J.u0, arena + U.pt + J.add + (U.map ? __ldg(U.map + i) : i), stride, m);
+    }
+    sums.close(m);
+    for (uint32_t z = G.first; z < G.first + G.count; ++z) {
+        const u64* s = srcs + 2ull * jobs[z].s;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            u64* out = arena + (h ? jobs[z].out1 : jobs[z].out0) + i;
+            const u64 r = sums.times([&](int b) { return arena[s[2 * b + h] + i]; }, m);
+            *out = accumulate ? add_mod(r, *out, m.q) : r;
+        }
+    }
+}
+
+// Every placement map of the launch keeps each 256-coefficient tile within
+// itself (a slot rotation by a multiple of D permutes the evaluation form
+// inside blocks of N / 2D words): tiles of nb rows, a unit's plaintexts or one
+// half of an output's baby steps, come by cp.async into one of two buffers
+// while the other is worked on. 64 KB a CTA at nb = 16, three on an SM.
+// 480 outputs of 9 units at nb = 16, N = 2^15, two limbs: 43 GB through L2, of
+// which 9.5 GB from HBM, in 3.3 ms (7.0 ms with a product for each plaintext
+// word); L2 at 56% and the issue slots at 54% of their peaks. Measured and
+// slower: four buffers of eight rows (3.7 ms: the instructions of a deeper
+// ring), the products with a baby step for each unit in double precision
+// (9.0 ms).
+template <int NB, bool HALVES>
+__global__ void __launch_bounds__(kDiagTile, HALVES ? 3 : 2) diag_inner_staged_kernel(
+    const PrimeConst* __restrict__ pc, u64* __restrict__ arena, uint32_t n, const DiagGroup* __restrict__ groups,
+    const DiagJob* __restrict__ jobs, const u64* __restrict__ srcs, const DiagUnit* __restrict__ units, u64 stride,
+    int accumulate) {
+    extern __shared__ __align__(16) u64 stage[];          // 2 buffers x NB rows x kDiagTile words
+    __shared__ u64 from[2][2 * NB];         // an output's baby steps, one output ahead
+    const uint32_t l = blockIdx.z, tid = threadIdx.x;
+    const DiagGroup G = groups[blockIdx.x];
+    const ModConst m = modconst_of(pc[l]);
+    const uint32_t base = blockIdx.y * kDiagTile, i = base + tid;
+    arena += (u64)l * n + base;
+    const DiagJob J = jobs[G.first];
+    const uint32_t nu = J.u1 - J.u0, items = nu + 2 * G.count;
+    units += J.u0;
+    if (tid < 2 * NB) from[0][tid] = srcs[2ull * J.s + tid];
+    // thread t copies words [2 (t % 128), + 2) of rows t / 128, t / 128 + 2, ...
+    const uint32_t row = tid / (kDiagTile / 2), col = tid % (kDiagTile / 2) * 2;
+    const u64 first = J.add + row * stride + col;
+    const u64 step = 2 * stride;
+    auto issue_unit = [&](uint32_t k, u64 pt) {
+        if (NB > 1 || row == 0) {
+            const u64* g = arena + (first + pt);
+            u64* d = stage + ((k & 1u) * NB + row) * kDiagTile + col;
+#pragma unroll
+            for (uint32_t r = 0; r < (NB + 1) / 2; ++r, g += step) cp_async16(d + 2 * r * kDiagTile, g);
         }
         cp_async_commit();
     };
-    Acc128 a0, a1;
-    acc_init(a0);
-    acc_init(a1);
-    Halves c0{0, 0, 0}, c1{0, 0, 0};
-    uint32_t cnt = 0;
-    if (J.u0 < J.u1) issue(J.u0, 0);
-    for (uint32_t k = J.u0; k < J.u1; ++k) {
-        const uint32_t buf = (k - J.u0) & 1u;
-        const uint32_t* map = units[k].map;
-        const uint32_t j = (map ? __ldg(map + i) : i) - base;
-        if (k + 1 < J.u1) {
-            issue(k + 1, buf ^ 1u);
-            cp_async_wait<1>();
-        } else {
-            cp_async_wait<0>();
+    auto issue_baby = [&](uint32_t k) {
+        const uint32_t e = k - nu;
+        if (NB > 1 || row == 0) {
+            const u64* f = &from[e >> 1 & 1u][2 * row + (e & 1u)];
+            u64* d = stage + ((k & 1u) * NB + row) * kDiagTile + col;
+#pragma unroll
+            for (uint32_t r = 0; r < (NB + 1) / 2; ++r) cp_async16(d + 2 * r * kDiagTile, arena + f[4 * r] + col);
         }
+        cp_async_commit();
+    };
+    // the next unit's descriptor and automorphism index are loaded while the
+    // current unit is added
+    DiagUnit U{0, nullptr}, V{0, nullptr};
+    uint32_t j = tid, jn = tid;
+    if (nu) U = units[0];
+    if (nu > 1) V = units[1];
+    if (nu) {
+        issue_unit(0, U.pt);
+        if (U.map) j = __ldg(U.map + i) - base;
+    } else {
         __syncthreads();
-        const u64* t = stage + (size_t)buf * NB * kDiagTile + j;
-        if (HALVES) {
-            if (cnt + NB > kHalfFold) {
-                c0 = Halves{halves_reduce(c0, m), 0, 0};
-                c1 = Halves{halves_reduce(c1, m), 0, 0};
-                cnt = 1;
-            }
-#pragma unroll
-            for (int b = 0; b < NB; ++b) {
-                const u64 v = t[b * kDiagTile];
-                const uint32_t v0 = (uint32_t)v & kHalfMask, v1 = (uint32_t)(v >> kHalfBits);
-                halves_mad(c0, v0, v1, h00[b], h01[b]);
-                halves_mad(c1, v0, v1, h10[b], h11[b]);
-            }
+        issue_baby(0);
+    }
+    DiagSums<NB, HALVES> sums;
+    for (uint32_t k = 0; k < nu; ++k) {
+        cp_async_wait<0>();
+        __syncthreads();                    // item k is here, the other buffer free
+        if (k + 1 < nu) {
+            issue_unit(k + 1, V.pt);
+            jn = V.map ? __ldg(V.map + i) - base : tid;
+            if (k + 2 < nu) V = units[k + 2];
         } else {
-            if (cnt + NB > reduce_every) {
-                acc_fold(a0, m);
-                acc_fold(a1, m);
-                cnt = 1;
-            }
-#pragma unroll
-            for (int b = 0; b < NB; ++b) {
-                const u64 v = t[b * kDiagTile];
-                acc_mad(a0, v, x0[b]);
-                acc_mad(a1, v, x1[b]);
-            }
+            issue_baby(nu);
         }
-        cnt += NB;
-        __syncthreads();                    // the buffer is refilled two units later
+        sums.add(k, stage + (k & 1u) * NB * kDiagTile + j, kDiagTile, m);
+        j = jn;
     }
-    u64 r0 = HALVES ? halves_reduce(c0, m) : acc_reduce(a0, m);
-    u64 r1 = HALVES ? halves_reduce(c1, m) : acc_reduce(a1, m);
-    if (accumulate) {
-        r0 = add_mod(r0, arena[J.out0 + off + i], m.q);
-        r1 = add_mod(r1, arena[J.out1 + off + i], m.q);
+    sums.close(m);
+    for (uint32_t k = nu; k < items; ++k) {
+        const uint32_t e = k - nu, z = G.first + (e >> 1);
+        cp_async_wait<0>();
+        __syncthreads();
+        if (k + 1 < items) issue_baby(k + 1);
+        if (!(e & 1u) && z + 1 < G.first + G.count && tid < 2 * NB) from[~(e >> 1) & 1u][tid] = srcs[2ull * jobs[z + 1].s + tid];
+        u64* out = arena + ((e & 1u) ? jobs[z].out1 : jobs[z].out0) + tid;
+        const u64* t = stage + (k & 1u) * NB * kDiagTile + tid;
+        const u64 r = sums.times([&](int b) { return t[b * kDiagTile]; }, m);
+        *out = accumulate ? add_mod(r, *out, m.q) : r;
     }
-    arena[J.out0 + off + i] = r0;
-    arena[J.out1 + off + i] = r1;
 }
 
-cudaError_t launch_diag_inner(const PrimeConst* pc, u64* arena, uint32_t n, uint32_t limbs, uint32_t jobs,
-                              uint32_t nb, const DiagJob* job, const u64* srcs, const DiagUnit* unit, u64 stride,
-                              uint32_t reduce_every, int accumulate, bool staged, bool halves, cudaStream_t st) {
-    if (limbs == 0 || jobs == 0) return cudaSuccess;
+template <int NB, bool HALVES>
+cudaError_t launch_diag(const PrimeConst* pc, u64* arena, uint32_t n, uint32_t limbs, uint32_t groups,
+                        const DiagGroup* group, const DiagJob* job, const u64* srcs, const DiagUnit* unit, u64 stride,
+                        int accumulate, bool staged, cudaStream_t st) {
+    const dim3 grid(groups, (n + kDiagTile - 1) / kDiagTile, limbs);
     if (staged) {
-        if (n % kDiagTile) return cudaErrorInvalidValue;
-        if (n / kDiagTile > 65535 || limbs > 65535) return cudaErrorInvalidValue;
-        dim3 grid(jobs, n / kDiagTile, limbs);
-        const size_t smem = 2ull * nb * kDiagTile * sizeof(u64);
-#define DIAG_STAGED_H(NBV, H)                                                                                  \
-    {                                                                                                          \
-        cudaError_t e = cudaFuncSetAttribute(diag_inner_staged_kernel<NBV, H>,                                 \
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);          \
-        if (e != cudaSuccess) return e;                                                                        \
-        diag_inner_staged_kernel<NBV, H><<<grid, kDiagTile, smem, st>>>(pc, arena, n, job, srcs, unit, stride, \
-                                                                        reduce_every, accumulate);             \
-    }
-#define DIAG_STAGED(NBV)                \
-    case NBV:                           \
-        if (halves)                     \
-            DIAG_STAGED_H(NBV, true)    \
-        else                            \
-            DIAG_STAGED_H(NBV, false)   \
-        break;
-        switch (nb) {
-            DIAG_STAGED(1)
-            DIAG_STAGED(2)
-            DIAG_STAGED(4)
-            DIAG_STAGED(8)
-            DIAG_STAGED(16)
-        default: return cudaErrorInvalidValue;
-        }
-#undef DIAG_STAGED
-#undef DIAG_STAGED_H
-        count_launches(1);
-        return cudaGetLastError();
-    }
-    dim3 grid((n + 255) / 256, limbs, jobs);
-    switch (nb) {
-    case 1: diag_inner_kernel<1><<<grid, 256, 0, st>>>(pc, arena, n, job, srcs, unit, stride, reduce_every, accumulate); break;
-    case 2: diag_inner_kernel<2><<<grid, 256, 0, st>>>(pc, arena, n, job, srcs, unit, stride, reduce_every, accumulate); break;
-    case 4: diag_inner_kernel<4><<<grid, 256, 0, st>>>(pc, arena, n, job, srcs, unit, stride, reduce_every, accumulate); break;
-    case 8: diag_inner_kernel<8><<<grid, 256, 0, st>>>(pc, arena, n, job, srcs, unit, stride, reduce_every, accumulate); break;
-    case 16: diag_inner_kernel<16><<<grid, 256, 0, st>>>(pc, arena, n, job, srcs, unit, stride, reduce_every, accumulate); break;
-    default: return cudaErrorInvalidValue;
+        const size_t smem = 2ull * NB * kDiagTile * sizeof(u64);
+        auto kern = diag_inner_staged_kernel<NB, HALVES>;
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
+        kern<<<grid, kDiagTile, smem, st>>>(pc, arena, n, group, job, srcs, unit, stride, accumulate);
+    } else {
+        diag_inner_kernel<NB, HALVES><<<grid, kDiagTile, 0, st>>>(pc, arena, n, group, job, srcs, unit, stride, accumulate);
     }
     count_launches(1);
     return cudaGetLastError();
+}
+
+cudaError_t launch_diag_inner(const PrimeConst* pc, u64* arena, uint32_t n, uint32_t limbs, uint32_t groups,
+                              uint32_t nb, const DiagGroup* group, const DiagJob* job, const u64* srcs,
+                              const DiagUnit* unit, u64 stride, int accumulate, bool staged, bool halves,
+                              cudaStream_t st) {
+    if (limbs == 0 || groups == 0) return cudaSuccess;
+    if (limbs > 65535 || (staged && n % kDiagTile)) return cudaErrorInvalidValue;
+    switch (nb) {
+    case 1:
+        return halves ? launch_diag<1, true>(pc, arena, n, limbs, groups, group, job, srcs, unit, stride, accumulate, staged, st)
+                      : launch_diag<1, false>(pc, arena, n, limbs, groups, group, job, srcs, unit, stride, accumulate, staged, st);
+    case 2:
+        return halves ? launch_diag<2, true>(pc, arena, n, limbs, groups, group, job, srcs, unit, stride, accumulate, staged, st)
+                      : launch_diag<2, false>(pc, arena, n, limbs, groups, group, job, srcs, unit, stride, accumulate, staged, st);
+    case 4:
+        return halves ? launch_diag<4, true>(pc, arena, n, limbs, groups, group, job, srcs, unit, stride, accumulate, staged, st)
+                      : launch_diag<4, false>(pc, arena, n, limbs, groups, group, job, srcs, unit, stride, accumulate, staged, st);
+    case 8:
+        return halves ? launch_diag<8, true>(pc, arena, n, limbs, groups, group, job, srcs, unit, stride, accumulate, staged, st)
+                      : launch_diag<8, false>(pc, arena, n, limbs, groups, group, job, srcs, unit, stride, accumulate, staged, st);
+    case 16:
+        return halves ? launch_diag<16, true>(pc, arena, n, limbs, groups, group, job, srcs, unit, stride, accumulate, staged, st)
+                      : launch_diag<16, false>(pc, arena, n, limbs, groups, group, job, srcs, unit, stride, accumulate, staged, st);
+    default: return cudaErrorInvalidValue;
+    }
 }
 
 cudaError_t launch_mac_plain(const PrimeConst* pc, u64* arena, uint32_t n, uint32_t limbs, uint32_t jobs,
