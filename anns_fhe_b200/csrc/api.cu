@@ -227,25 +227,15 @@ int build_native_tables(afhe_ctx* ctx) {
         if (e != cudaSuccess) return cuda_fail(ctx, e, "twiddle tables");
     }
 
-    // per-level CRT tables, each followed by its Shoup companions
+    // per-level CRT tables
     std::vector<u64> buf;
-    struct Ref { size_t v, sh; };
-    auto push = [&](const std::vector<u64>& vals, const std::vector<u64>& mods) -> Ref {
-        Ref r;
-        r.v = buf.size();
-        buf.insert(buf.end(), vals.begin(), vals.end());
-        r.sh = buf.size();
-        for (size_t i = 0; i < vals.size(); ++i) buf.push_back(host_shoup(vals[i], mods[i]));
-        return r;
-    };
     struct LvlRefs {
-        Ref qi[AFHE_MAX_PARTS], qm[AFHE_MAX_PARTS], pinv, phinv, phq, qlql, qlinv;
-        size_t qm_sp[AFHE_MAX_PARTS], phq_sp, fin_q, fin_p, pmq, pinv_tc;   // 16-byte aligned
+        size_t qi[AFHE_MAX_PARTS], qm[AFHE_MAX_PARTS], pinv, phinv, phq, qlql, qlinv, fin_q, fin_p, pmq;
         uint32_t parts;
     };
-    auto align2 = [&]() { if (buf.size() & 1) buf.push_back(0); return buf.size(); };
+    // (all of them of four or eight words: 16-byte aligned)
     auto push_split = [&](const std::vector<u64>& vals, const std::vector<u64>& mods) {
-        const size_t at = align2();
+        const size_t at = buf.size();
         buf.resize(at + 4 * vals.size());
         for (size_t i = 0; i < vals.size(); ++i) split_constant(vals[i], mods[i], &buf[at + 4 * i]);
         return at;
@@ -258,10 +248,11 @@ int build_native_tables(afhe_ctx* ctx) {
         transform_constant((u64)((unsigned __int128)pc[i].w1ninv * f % m), m, o + 4);
         buf.insert(buf.end(), o, o + 8);
     };
-    auto push_tc = [&](u64 w, u64 m) {
-        u64 o[4];
-        transform_constant(w % m, m, o);
-        buf.insert(buf.end(), o, o + 4);
+    auto push_tc = [&](const std::vector<u64>& vals, const std::vector<u64>& mods) {
+        const size_t at = buf.size();
+        buf.resize(at + 4 * vals.size());
+        for (size_t i = 0; i < vals.size(); ++i) transform_constant(vals[i] % mods[i], mods[i], &buf[at + 4 * i]);
+        return at;
     };
     std::vector<LvlRefs> refs(L + 1);
     const u64* q = primes.data();
@@ -269,6 +260,7 @@ int build_native_tables(afhe_ctx* ctx) {
     for (uint32_t lvl = 1; lvl <= L; ++lvl) {
         LvlRefs& R = refs[lvl];
         R.parts = (lvl + ctx->alpha - 1) / ctx->alpha;
+        std::vector<u64> qhat_inv;
         for (uint32_t j = 0; j < R.parts; ++j) {
             uint32_t start = j * ctx->alpha;
             uint32_t size = (j == R.parts - 1) ? lvl - start : ctx->alpha;
@@ -283,9 +275,9 @@ int build_native_tables(afhe_ctx* ctx) {
                 mi[i] = q[start + i];
                 for (uint32_t c = 0; c < row; ++c) mm[(size_t)i * row + c] = outp[c];
             }
-            R.qi[j] = push(qi, mi);
-            R.qm[j] = push(qm, mm);
-            R.qm_sp[j] = push_split(qm, mm);
+            R.qi[j] = push_tc(qi, mi);
+            R.qm[j] = push_split(qm, mm);
+            qhat_inv.insert(qhat_inv.end(), qi.begin(), qi.end());
         }
         std::vector<u64> pinv(lvl), phinv(K), phq((size_t)K * lvl), mq(lvl), mp(K), mphq((size_t)K * lvl);
         moddown_tables(q, lvl, p, K, pinv.data(), phinv.data(), phq.data());
@@ -294,32 +286,24 @@ int build_native_tables(afhe_ctx* ctx) {
             mp[k] = p[k];
             for (uint32_t i = 0; i < lvl; ++i) mphq[(size_t)k * lvl + i] = q[i];
         }
-        R.pinv = push(pinv, mq);
-        R.phinv = push(phinv, mp);
-        R.phq = push(phq, mphq);
-        R.phq_sp = push_split(phq, mphq);
-        R.fin_q = align2();
-        for (uint32_t i = 0; i < lvl; ++i) {
-            const uint32_t j = i / ctx->alpha;
-            push_fin(buf[R.qi[j].v + (i - j * ctx->alpha)], i);
-        }
-        R.fin_p = align2();
+        R.pinv = push_tc(pinv, mq);
+        R.phinv = push_tc(phinv, mp);
+        R.phq = push_split(phq, mphq);
+        R.fin_q = buf.size();
+        for (uint32_t i = 0; i < lvl; ++i) push_fin(qhat_inv[i], i);
+        R.fin_p = buf.size();
         for (uint32_t k = 0; k < K; ++k) push_fin(phinv[k], L + k);
-        R.pmq = align2();
-        for (uint32_t i = 0; i < lvl; ++i) {
-            u64 prod = 1;
-            for (uint32_t k = 0; k < K; ++k) prod = (u64)((unsigned __int128)prod * (p[k] % q[i]) % q[i]);
-            push_tc(prod, q[i]);
-        }
-        R.pinv_tc = align2();
-        for (uint32_t i = 0; i < lvl; ++i) push_tc(pinv[i], q[i]);
+        std::vector<u64> pmq(lvl, 1);
+        for (uint32_t i = 0; i < lvl; ++i)
+            for (uint32_t k = 0; k < K; ++k) pmq[i] = (u64)((unsigned __int128)pmq[i] * (p[k] % q[i]) % q[i]);
+        R.pmq = push_tc(pmq, mq);
         std::vector<u64> qlql(lvl > 1 ? lvl - 1 : 1, 0), qlinv(lvl > 1 ? lvl - 1 : 1, 0), mr(lvl > 1 ? lvl - 1 : 1, 3);
         if (lvl > 1) {
             rescale_tables(q, lvl, qlql.data(), qlinv.data());
             for (uint32_t i = 0; i + 1 < lvl; ++i) mr[i] = q[i];
         }
-        R.qlql = push(qlql, mr);
-        R.qlinv = push(qlinv, mr);
+        R.qlql = push_split(qlql, mr);
+        R.qlinv = push_tc(qlinv, mr);
     }
     CK(dalloc(&ctx->lvbuf, buf.size()));
     CK(cudaMemcpy(ctx->lvbuf, buf.data(), buf.size() * 8, cudaMemcpyHostToDevice));
@@ -334,27 +318,17 @@ int build_native_tables(afhe_ctx* ctx) {
         t.parts = R.parts;
         t.alpha = ctx->alpha;
         for (uint32_t j = 0; j < R.parts; ++j) {
-            t.qhat_inv[j] = b + R.qi[j].v;
-            t.qhat_inv_sh[j] = b + R.qi[j].sh;
-            t.qhat_modp[j] = b + R.qm[j].v;
-            t.qhat_modp_sh[j] = b + R.qm[j].sh;
-            t.qhat_modp_sp[j] = b + R.qm_sp[j];
+            t.qhat_inv_tc[j] = b + R.qi[j];
+            t.qhat_modp_sp[j] = b + R.qm[j];
         }
-        t.phat_modq_sp = b + R.phq_sp;
+        t.p_inv_tc = b + R.pinv;
+        t.phat_inv_tc = b + R.phinv;
+        t.phat_modq_sp = b + R.phq;
+        t.qlql_sp = b + R.qlql;
+        t.qlinv_tc = b + R.qlinv;
         t.fin_q = b + R.fin_q;
         t.fin_p = b + R.fin_p;
         t.p_mod_q = b + R.pmq;
-        t.p_inv_tc = b + R.pinv_tc;
-        t.p_inv_mod_q = b + R.pinv.v;
-        t.p_inv_mod_q_sh = b + R.pinv.sh;
-        t.phat_inv_modp = b + R.phinv.v;
-        t.phat_inv_modp_sh = b + R.phinv.sh;
-        t.phat_modq = b + R.phq.v;
-        t.phat_modq_sh = b + R.phq.sh;
-        t.qlql = b + R.qlql.v;
-        t.qlql_sh = b + R.qlql.sh;
-        t.qlinv = b + R.qlinv.v;
-        t.qlinv_sh = b + R.qlinv.sh;
     }
     // the same tables as one device array, for launches whose entries run at
     // different levels
@@ -515,7 +489,7 @@ int afhe_ctx_destroy(afhe_ctx* ctx) {
     for (DevPrimeSet* s : {&ctx->nat, &ctx->ld}) {
         fr(s->pc); fr(s->tw); fr(s->itw); fr(s->tw2); fr(s->itw2); fr(s->tw2b); fr(s->itw2b);
     }
-    fr(ctx->ld_crt); fr(ctx->ld_crt_sh); fr(ctx->ld_mod);
+    fr(ctx->ld_crt); fr(ctx->ld_sp);
     for (auto& kv : ctx->rot) fr(kv.second.map);
     for (auto& kv : ctx->auto_maps) fr(kv.second);
     fr(ctx->dec_ws);
@@ -887,12 +861,10 @@ int load_context(afhe_ctx* ctx, const afhe_accel_args* a) {
         if (!chk(r.first, r.second)) return fail(ctx, AFHE_E_RANGE, "OP_LOAD_CONTEXT: table offset out of range");
     if (ctx->ld_crt_words < cur) {
         if (ctx->ld_crt) cudaFree(ctx->ld_crt);
-        if (ctx->ld_crt_sh) cudaFree(ctx->ld_crt_sh);
-        if (ctx->ld_mod) cudaFree(ctx->ld_mod);
-        ctx->ld_crt = ctx->ld_crt_sh = ctx->ld_mod = nullptr;
-        CK(dalloc(&ctx->ld_crt, 2 * cur));   // raw, then a working copy
-        CK(dalloc(&ctx->ld_crt_sh, cur));
-        CK(dalloc(&ctx->ld_mod, cur));
+        if (ctx->ld_sp) cudaFree(ctx->ld_sp);
+        ctx->ld_crt = ctx->ld_sp = nullptr;
+        CK(dalloc(&ctx->ld_crt, cur));
+        CK(dalloc(&ctx->ld_sp, 8 * cur));   // every entry in split form, then as transform constants
         ctx->ld_crt_words = cur;
     }
     size_t at = 0;
@@ -927,8 +899,8 @@ int check_call_primes(afhe_ctx* ctx, const afhe_accel_args* a, uint32_t nq, uint
     return AFHE_OK;
 }
 
-// Per-call working copy of the loaded CRT tables reduced by, and with
-// companions for, the moduli each entry multiplies under at level sizeQl.
+// The loaded CRT tables' constants for the moduli each entry multiplies under at
+// level sizeQl.
 int prep_loaded_tables(afhe_ctx* ctx, uint32_t sizeQl, uint32_t parts, uint32_t alpha, bool ks, OpTabs* t) {
     const int key[4] = {(int)sizeQl, (int)parts, (int)alpha, ks ? 1 : 0};
     if (std::equal(key, key + 4, ctx->ld_tabs_key)) {   // prepared by an earlier call, in stream order
@@ -945,7 +917,8 @@ int prep_loaded_tables(afhe_ctx* ctx, uint32_t sizeQl, uint32_t parts, uint32_t 
     t->sizeQl = sizeQl;
     t->parts = parts;
     t->alpha = alpha;
-    u64* work = ctx->ld_crt + W;
+    auto sp = [&](size_t at) { return ctx->ld_sp + 4 * at; };
+    auto tc = [&](size_t at) { return ctx->ld_sp + 4 * (W + at); };
     if (ks) {
         if (parts > ctx->ld_parts) return fail(ctx, AFHE_E_LEVEL, "more digits than the loaded context");
         for (uint32_t j = 0; j < parts; ++j) {
@@ -964,10 +937,8 @@ int prep_loaded_tables(afhe_ctx* ctx, uint32_t sizeQl, uint32_t parts, uint32_t 
                 mods[ctx->ld_off_qhat_inv[j] + i] = q[start + i];
                 for (uint32_t c = 0; c < row; ++c) mods[ctx->ld_off_qhat_modp[j] + (size_t)i * row + c] = outp[c];
             }
-            t->qhat_inv[j] = work + ctx->ld_off_qhat_inv[j];
-            t->qhat_inv_sh[j] = ctx->ld_crt_sh + ctx->ld_off_qhat_inv[j];
-            t->qhat_modp[j] = work + ctx->ld_off_qhat_modp[j];
-            t->qhat_modp_sh[j] = ctx->ld_crt_sh + ctx->ld_off_qhat_modp[j];
+            t->qhat_inv_tc[j] = tc(ctx->ld_off_qhat_inv[j]);
+            t->qhat_modp_sp[j] = sp(ctx->ld_off_qhat_modp[j]);
         }
         for (uint32_t i = 0; i < sizeQl; ++i) mods[ctx->ld_off_pinv + i] = q[i];
         for (uint32_t k = 0; k < K; ++k) {
@@ -980,24 +951,18 @@ int prep_loaded_tables(afhe_ctx* ctx, uint32_t sizeQl, uint32_t parts, uint32_t 
             mods[ctx->ld_off_qlinv + i] = q[i];
         }
     }
-    t->p_inv_mod_q = work + ctx->ld_off_pinv;
-    t->p_inv_mod_q_sh = ctx->ld_crt_sh + ctx->ld_off_pinv;
-    t->phat_inv_modp = work + ctx->ld_off_phatinv;
-    t->phat_inv_modp_sh = ctx->ld_crt_sh + ctx->ld_off_phatinv;
-    t->phat_modq = work + ctx->ld_off_phatmodq;
-    t->phat_modq_sh = ctx->ld_crt_sh + ctx->ld_off_phatmodq;
-    t->qlql = work + ctx->ld_off_qlql;
-    t->qlql_sh = ctx->ld_crt_sh + ctx->ld_off_qlql;
-    t->qlinv = work + ctx->ld_off_qlinv;
-    t->qlinv_sh = ctx->ld_crt_sh + ctx->ld_off_qlinv;
+    t->p_inv_tc = tc(ctx->ld_off_pinv);
+    t->phat_inv_tc = tc(ctx->ld_off_phatinv);
+    t->phat_modq_sp = sp(ctx->ld_off_phatmodq);
+    t->qlql_sp = sp(ctx->ld_off_qlql);
+    t->qlinv_tc = tc(ctx->ld_off_qlinv);
     // the moduli go through the pinned descriptor ring: no host wait, and the
-    // working copy is rewritten in stream order after every earlier use
+    // constants are rewritten in stream order after every earlier use
     cudaStream_t st = ctx->st;
     u64* dmods = nullptr;
     int rc = ring_put(ctx, mods.data(), W, &dmods);
     if (rc != AFHE_OK) return rc;
-    CK(cudaMemcpyAsync(work, ctx->ld_crt, W * 8, cudaMemcpyDeviceToDevice, st));
-    CK(launch_companions(work, ctx->ld_crt_sh, dmods, W, st));
+    CK(launch_table_constants(ctx->ld_crt, dmods, ctx->ld_sp, ctx->ld_sp + 4 * W, W, st));
     ctx->ld_tabs = *t;
     std::copy(key, key + 4, ctx->ld_tabs_key);
     return AFHE_OK;

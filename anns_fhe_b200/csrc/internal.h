@@ -13,38 +13,29 @@
 
 namespace afhe {
 
-// Table pointers an operator needs at one level (device memory). Every
-// constant that multiplies through Shoup comes with its companion (_sh).
+// Table pointers an operator needs at one level (device memory). Constants that
+// multiply residues of one prime take four words as that prime's transforms
+// multiply (_tc, transform_constant), those of base conversions four words in
+// split form (_sp, split_constant).
 struct OpTabs {
     PrimeTables pt;
     uint32_t p_base;   // table index of special prime 0
     uint32_t sizeQl;   // level these tables are for
     uint32_t parts;    // digits at this level
     uint32_t alpha;
-    const u64* qhat_inv[AFHE_MAX_PARTS];
-    const u64* qhat_inv_sh[AFHE_MAX_PARTS];
-    const u64* qhat_modp[AFHE_MAX_PARTS];
-    const u64* qhat_modp_sh[AFHE_MAX_PARTS];
-    const u64* p_inv_mod_q;
-    const u64* p_inv_mod_q_sh;
-    const u64* phat_inv_modp;
-    const u64* phat_inv_modp_sh;
-    const u64* phat_modq;       // [K][sizeQl]
-    const u64* phat_modq_sh;
-    const u64* qlql;
-    const u64* qlql_sh;
-    const u64* qlinv;
-    const u64* qlinv_sh;
-    // base-conversion constants in split form (4 words each, split_constant)
+    const u64* qhat_inv_tc[AFHE_MAX_PARTS];
     const u64* qhat_modp_sp[AFHE_MAX_PARTS];
-    const u64* phat_modq_sp;
+    const u64* p_inv_tc;
+    const u64* phat_inv_tc;
+    const u64* phat_modq_sp;    // [K][sizeQl]
+    const u64* qlql_sp;
+    const u64* qlinv_tc;
     // one-kernel key switch (native tables): the last inverse stage's two
     // constants times qHatInv (per Q limb) and times PHatInv (per special
-    // limb), 8 words each; P and P^-1 mod q_i as transform constants, 4 each
+    // limb), 8 words each; P mod q_i as transform constants
     const u64* fin_q;
     const u64* fin_p;
     const u64* p_mod_q;
-    const u64* p_inv_tc;
 };
 
 // Owned device storage for one twiddle table set. tw / itw hold raw tables
@@ -112,8 +103,7 @@ struct afhe_ctx {
     uint32_t ld_nq = 0, ld_np = 0, ld_alpha = 0, ld_parts = 0;
     std::vector<afhe::u64> ld_q, ld_p, ld_ninv_q, ld_ninv_p;
     afhe::u64* ld_crt = nullptr;       // raw CRT tables as loaded (device)
-    afhe::u64* ld_crt_sh = nullptr;    // per-call companions (device)
-    afhe::u64* ld_mod = nullptr;       // per-call moduli for companion prep (device)
+    afhe::u64* ld_sp = nullptr;        // the entries' constants for one level (device)
     size_t ld_crt_words = 0;
     std::vector<size_t> ld_off_qhat_inv, ld_off_qhat_modp;
     size_t ld_off_pinv = 0, ld_off_phatinv = 0, ld_off_phatmodq = 0, ld_off_qlql = 0, ld_off_qlinv = 0;
@@ -305,8 +295,9 @@ cudaError_t launch_key_prep(const u64* key, ulonglong2* prep, const PrimeConst* 
 // as transform constants in the rounds' order (PrimeTables).
 cudaError_t launch_twiddles(const u64* raw, const u64* q, ulonglong2* out2, ulonglong2* out2b, uint32_t rows, int log_n,
                             cudaStream_t st);
-// Companion prep: sh[e] = shoup_companion(v[e] mod m[e], m[e]); v reduced in place.
-cudaError_t launch_companions(u64* v, u64* sh, const u64* m, size_t count, cudaStream_t st);
+// Table prep: entry v[e] mod m[e] in split form at sp + 4 e and as a transform
+// constant at tc + 4 e (where m[e] is not 0).
+cudaError_t launch_table_constants(const u64* v, const u64* m, u64* sp, u64* tc, size_t count, cudaStream_t st);
 // Loaded prime constants: fills pc[i] from q/ninv arrays (device) and itw.
 cudaError_t launch_prime_consts(PrimeConst* pc, const u64* q, const u64* ninv, const u64* itw, uint32_t n,
                                 uint32_t count, cudaStream_t st);

@@ -27,30 +27,43 @@ void set_ntt_plan(int log_n, int plan) { g_ntt_plan[log_n].store(plan, std::memo
 // ---------------------------------------------------------------------------
 // elementwise
 // ---------------------------------------------------------------------------
+// Four coefficients a thread, 256 apart: the loads of all are on their way
+// before the first is used. Products of primes below 2^50 in doubles (10 FP64
+// instructions in place of about 95 multiplier cycles for the 128-bit product
+// and its reduction).
+constexpr uint32_t kEwPer = 4;
 template <int OP>
 __global__ void __launch_bounds__(256) elementwise_kernel(const PrimeConst* __restrict__ pc, uint32_t prime0,
                                                           u64* __restrict__ arena, uint32_t n, const ZBases zb) {
     const uint32_t l = blockIdx.y, z = blockIdx.z;
     const PrimeConst p = pc[prime0 + l];
-    const u64 off = (u64)l * n;
+    const uint32_t i0 = blockIdx.x * (256 * kEwPer) + threadIdx.x;
+    const u64 off = (u64)l * n + i0;
     const u64* a = arena + zb.src.at(z) + off;
     const u64* b = arena + zb.aux.at(z) + off;
     u64* o = arena + zb.out.at(z) + off;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        u64 x = a[i];
-        u64 r;
-        if (OP == EW_ADD) r = add_mod(x, b[i], p.q);
-        else if (OP == EW_SUB) r = sub_mod(x, b[i], p.q);
-        else if (OP == EW_MUL) r = mul_mod(x, b[i], modconst_of(p));
-        else r = x;
-        o[i] = r;
+    u64 x[kEwPer], y[kEwPer];
+#pragma unroll
+    for (uint32_t k = 0; k < kEwPer; ++k) {
+        const bool in = i0 + 256 * k < n;
+        x[k] = in ? a[256 * k] : 0;
+        y[k] = OP != EW_COPY && in ? b[256 * k] : 0;
+    }
+#pragma unroll
+    for (uint32_t k = 0; k < kEwPer; ++k) {
+        u64 r = x[k];
+        if (OP == EW_ADD) r = add_mod(x[k], y[k], p.q);
+        else if (OP == EW_SUB) r = sub_mod(x[k], y[k], p.q);
+        else if (OP == EW_MUL) r = p.fp ? fp_canon(fp_mul2(fp_of(x[k]), fp_of(y[k]), p.qd, p.qi), p.qd)
+                                        : mul_mod(x[k], y[k], modconst_of(p));
+        if (i0 + 256 * k < n) o[256 * k] = r;
     }
 }
 
 cudaError_t launch_elementwise(ElemOp op, const PrimeConst* pc, uint32_t prime0, u64* arena, uint32_t n,
                                uint32_t limbs, uint32_t nz, const ZBases& zb, cudaStream_t st) {
     if (limbs == 0 || nz == 0) return cudaSuccess;
-    dim3 grid((n + 255) / 256, limbs, nz);
+    dim3 grid((n + 256 * kEwPer - 1) / (256 * kEwPer), limbs, nz);
     switch (op) {
     case EW_ADD: elementwise_kernel<EW_ADD><<<grid, 256, 0, st>>>(pc, prime0, arena, n, zb); break;
     case EW_SUB: elementwise_kernel<EW_SUB><<<grid, 256, 0, st>>>(pc, prime0, arena, n, zb); break;
@@ -68,7 +81,8 @@ cudaError_t launch_elementwise(ElemOp op, const PrimeConst* pc, uint32_t prime0,
 __global__ void __launch_bounds__(256) tensor_kernel(const PrimeConst* __restrict__ pc, u64* __restrict__ arena,
                                                      uint32_t n, const TensorArgs ta) {
     const uint32_t l = blockIdx.y, z = blockIdx.z;
-    const ModConst m = modconst_of(pc[l]);
+    const PrimeConst p = pc[l];
+    const ModConst m = modconst_of(p);
     const u64 off = (u64)l * n;
     const u64* a0 = arena + ta.a0.at(z) + off;
     const u64* a1 = arena + ta.a1.at(z) + off;
@@ -79,6 +93,14 @@ __global__ void __launch_bounds__(256) tensor_kernel(const PrimeConst* __restric
     u64* d2 = arena + ta.d2.at(z) + off;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         u64 x0 = a0[i], x1 = a1[i], y0 = b0[i], y1 = b1[i];
+        if (p.fp) {
+            const double f0 = fp_of(x0), f1 = fp_of(x1), g0 = fp_of(y0), g1 = fp_of(y1);
+            const double c = __dadd_rn(fp_mul2(f0, g1, p.qd, p.qi), fp_mul2(f1, g0, p.qd, p.qi));
+            d0[i] = fp_canon(fp_mul2(f0, g0, p.qd, p.qi), p.qd);
+            d1[i] = fp_canon(fp_center(c, p.qd, p.qi), p.qd);
+            d2[i] = fp_canon(fp_mul2(f1, g1, p.qd, p.qi), p.qd);
+            continue;
+        }
         Acc128 c;
         acc_init(c);
         acc_mad(c, x0, y1);
@@ -493,21 +515,22 @@ cudaError_t launch_ntt_plain(bool inverse, int log_n, const PrimeTables& pt, con
 // ---------------------------------------------------------------------------
 // table preparation
 // ---------------------------------------------------------------------------
-__global__ void companions_kernel(u64* v, u64* sh, const u64* m, size_t count) {
+__global__ void table_constants_kernel(const u64* __restrict__ v, const u64* __restrict__ m, u64* __restrict__ sp,
+                                       u64* __restrict__ tc, size_t count) {
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < count; i += (size_t)gridDim.x * blockDim.x) {
-        u64 mod = m[i];
-        if (mod == 0) { sh[i] = 0; continue; }
-        u64 w = v[i] % mod;
-        v[i] = w;
-        sh[i] = shoup_companion(w, mod);
+        const u64 mod = m[i];
+        if (mod == 0) continue;
+        const u64 w = v[i] % mod;
+        split_constant(w, mod, sp + 4 * i);
+        transform_constant(w, mod, tc + 4 * i);
     }
 }
 
-cudaError_t launch_companions(u64* v, u64* sh, const u64* m, size_t count, cudaStream_t st) {
+cudaError_t launch_table_constants(const u64* v, const u64* m, u64* sp, u64* tc, size_t count, cudaStream_t st) {
     if (count == 0) return cudaSuccess;
     unsigned blocks = (unsigned)((count + 255) / 256);
     if (blocks > 4096) blocks = 4096;
-    companions_kernel<<<blocks, 256, 0, st>>>(v, sh, m, count);
+    table_constants_kernel<<<blocks, 256, 0, st>>>(v, m, sp, tc, count);
     count_launches(1);
     return cudaGetLastError();
 }

@@ -25,6 +25,7 @@ size_t ks_scratch_words(uint32_t n, uint32_t slots_q, uint32_t K, uint32_t parts
 // Input load through the automorphism: the key switch of auto(c1) reads
 // c1[map[x]] (the reference applies automorphism() first, fhe_host_driver.cpp:342-350).
 struct LoadGather {
+    static constexpr bool kMany = false;
     const u64* base;
     const uint32_t* map;
     ZField mapz;        // per-entry map addresses (per_z)
@@ -45,8 +46,7 @@ struct StoreQhatInv {
     __device__ __forceinline__ void operator()(const LimbJob& j, const ZBases& zb, uint32_t z, u64 x, u64 v,
                                                const PrimeConst& pc) const {
         const uint32_t part = j.aux / t.alpha, idx = j.aux - part * t.alpha;
-        scratch[zb.out.at(z) + j.out + x] =
-            mul_shoup(v, __ldg(t.qhat_inv[part] + idx), __ldg(t.qhat_inv_sh[part] + idx), pc.q);
+        scratch[zb.out.at(z) + j.out + x] = mul_tc(v, t.qhat_inv_tc[part] + 4ull * idx, pc);
     }
 };
 
@@ -54,28 +54,20 @@ struct StoreQhatInv {
 // k is the output's position among the digit's complementary primes. Reads
 // y_i = [x_i * qHatInv_i]_{q_i} (StoreQhatInv) and sums y_i * [qHat_i]_p.
 struct ModUpLoad {
+    static constexpr bool kMany = true;
     const u64* scratch;   // coef region at zb.aux[z]
     OpTabs t;
     uint32_t K;
     uint32_t n;
-    __device__ __forceinline__ u64 operator()(const LimbJob& j, const ZBases& zb, uint32_t z, u64 x,
-                                              const PrimeConst& pc) const {
+    template <int M>
+    __device__ __forceinline__ void many(u64* o, const LimbJob& j, const ZBases& zb, uint32_t z, u64 x, u64 step,
+                                         const PrimeConst& pc) const {
         const uint32_t part = j.aux >> 16, k = j.aux & 0xFFFFu;
         const uint32_t start = part * t.alpha;
         const uint32_t size = (part == t.parts - 1) ? t.sizeQl - start : t.alpha;
-        const uint32_t row = t.sizeQl - size + K;   // complementary primes of this digit
-        const u64 p = pc.q, p2 = p << 1;
-        const u64* qm = t.qhat_modp[part];
-        const u64* qmsh = t.qhat_modp_sh[part];
-        u64 s = 0;
-        for (uint32_t i = 0; i < size; ++i) {
-            const uint32_t limb = start + i;
-            const u64 y = scratch[zb.aux.at(z) + (u64)limb * n + x];            // [x * qHatInv]_{q_i}
-            u64 w = mul_shoup_lazy(y, __ldg(qm + i * row + k), __ldg(qmsh + i * row + k), p);
-            s += w;
-            s = s >= p2 ? s - p2 : s;
-        }
-        return csub(s, p);
+        const u64* const y = scratch + zb.aux.at(z) + (u64)start * n + x;     // [x * qHatInv]_{q_i}
+        bconv<M>(o, size, t.qhat_modp_sp[part] + 4ull * k, t.sizeQl - size + K, pc.q,
+                 [&](uint32_t i, uint32_t e) { return y[(u64)i * n + e * step]; });
     }
 };
 
@@ -88,7 +80,9 @@ struct StoreSlot {   // plain store into scratch
 };
 
 // Inner product with the evaluation key. One thread per (slot, coefficient).
-// slot s < sizeQl is Q limb s, slot slots_q + k is special limb k.
+// slot s < sizeQl is Q limb s, slot slots_q + k is special limb k. The operands
+// of up to four digits are on their way before the first is used; products of
+// primes below 2^50 in doubles, else summed in 128 bits and reduced once.
 __global__ void __launch_bounds__(256) ks_mac_kernel(OpTabs t, uint32_t n, uint32_t slots_q, uint32_t sizeQl,
                                                      uint32_t K, const u64* __restrict__ key, u64 evk_a, u64 evk_b,
                                                      uint32_t key_stride, uint32_t key_pbase,
@@ -116,18 +110,41 @@ __global__ void __launch_bounds__(256) ks_mac_kernel(OpTabs t, uint32_t n, uint3
         Acc128 ab, aa;
         acc_init(ab);
         acc_init(aa);
-        for (uint32_t part = 0; part < t.parts; ++part) {
-            const uint32_t start = part * t.alpha;
-            const uint32_t size = (part == t.parts - 1) ? sizeQl - start : t.alpha;
-            u64 d;
-            if (isq && sidx >= start && sidx < start + size) d = in[xs];
-            else d = scratch[base_scr + modup_off + ((u64)part * S + slot) * n + x];
-            const u64 kl = koff + ((u64)part * key_stride + klimb_in_digit) * n + x;
-            acc_mad(ab, d, __ldg(key + evk_b + kl));
-            acc_mad(aa, d, __ldg(key + evk_a + kl));
+        double fb = 0, fa = 0;
+        constexpr uint32_t D = 4;
+        for (uint32_t part0 = 0; part0 < t.parts; part0 += D) {
+            u64 d[D], kb[D], ka[D];
+#pragma unroll
+            for (uint32_t e = 0; e < D; ++e) {
+                const uint32_t part = part0 + e;
+                if (part >= t.parts) {
+                    d[e] = kb[e] = ka[e] = 0;
+                    continue;
+                }
+                const uint32_t start = part * t.alpha;
+                const uint32_t size = (part == t.parts - 1) ? sizeQl - start : t.alpha;
+                const bool own = isq && sidx >= start && sidx < start + size;
+                const u64* const from = own ? in + xs : scratch + base_scr + modup_off + ((u64)part * S + slot) * n + x;
+                const u64 kl = koff + ((u64)part * key_stride + klimb_in_digit) * n + x;
+                d[e] = *from;
+                kb[e] = __ldg(key + evk_b + kl);
+                ka[e] = __ldg(key + evk_a + kl);
+            }
+#pragma unroll
+            for (uint32_t e = 0; e < D; ++e) {
+                if (part0 + e >= t.parts) break;
+                if (pc.fp) {
+                    const double f = fp_of(d[e]);
+                    fb = fp_center(__dadd_rn(fb, fp_mul2(f, fp_of(kb[e]), pc.qd, pc.qi)), pc.qd, pc.qi);
+                    fa = fp_center(__dadd_rn(fa, fp_mul2(f, fp_of(ka[e]), pc.qd, pc.qi)), pc.qd, pc.qi);
+                } else {
+                    acc_mad(ab, d[e], kb[e]);
+                    acc_mad(aa, d[e], ka[e]);
+                }
+            }
         }
-        scratch[base_scr + ext0_off + (u64)slot * n + x] = acc_reduce(ab, mc);
-        scratch[base_scr + ext1_off + (u64)slot * n + x] = acc_reduce(aa, mc);
+        scratch[base_scr + ext0_off + (u64)slot * n + x] = pc.fp ? fp_canon(fb, pc.qd) : acc_reduce(ab, mc);
+        scratch[base_scr + ext1_off + (u64)slot * n + x] = pc.fp ? fp_canon(fa, pc.qd) : acc_reduce(aa, mc);
     }
 }
 

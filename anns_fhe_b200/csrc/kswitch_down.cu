@@ -13,29 +13,23 @@ struct StorePhatInv {
     OpTabs t;
     __device__ __forceinline__ void operator()(const LimbJob& j, const ZBases& zb, uint32_t z, u64 x, u64 v,
                                                const PrimeConst& pc) const {
-        scratch[zb.out.at(z) + j.out + x] =
-            mul_shoup(v, __ldg(t.phat_inv_modp + j.aux), __ldg(t.phat_inv_modp_sh + j.aux), pc.q);
+        scratch[zb.out.at(z) + j.out + x] = mul_tc(v, t.phat_inv_tc + 4ull * j.aux, pc);
     }
 };
 
 // ModDown base conversion P -> Q as the NTT prologue (job = Q limb i). Reads
 // [x_k * PHatInv_k]_{p_k} (StorePhatInv) and sums it times [PHat_k]_{q_i}.
 struct ModDownLoad {
+    static constexpr bool kMany = true;
     const u64* scratch;  // ext region at zb.aux[z]
     OpTabs t;
     uint32_t slots_q, K, n;
-    __device__ __forceinline__ u64 operator()(const LimbJob& j, const ZBases& zb, uint32_t z, u64 x,
-                                              const PrimeConst& pc) const {
-        const u64 q = pc.q, q2 = q << 1;
-        const uint32_t i = j.aux;
-        u64 s = 0;
-        for (uint32_t k = 0; k < K; ++k) {
-            const u64 y = scratch[zb.aux.at(z) + (u64)(slots_q + k) * n + x];
-            u64 w = mul_shoup_lazy(y, __ldg(t.phat_modq + k * t.sizeQl + i), __ldg(t.phat_modq_sh + k * t.sizeQl + i), q);
-            s += w;
-            s = s >= q2 ? s - q2 : s;
-        }
-        return csub(s, q);
+    template <int M>
+    __device__ __forceinline__ void many(u64* o, const LimbJob& j, const ZBases& zb, uint32_t z, u64 x, u64 step,
+                                         const PrimeConst& pc) const {
+        const u64* const y = scratch + zb.aux.at(z) + (u64)slots_q * n + x;
+        bconv<M>(o, K, t.phat_modq_sp + 4ull * j.aux, t.sizeQl, pc.q,
+                 [&](uint32_t k, uint32_t e) { return y[(u64)k * n + e * step]; });
     }
 };
 
@@ -58,7 +52,7 @@ struct ModDownStore {
         const u64 li = (u64)i * n + x;
         u64 xq = scratch[zb.src.at(z) + li];
         u64 d = sub_mod(xq, v, q);
-        u64 r = mul_shoup(d, __ldg(t.p_inv_mod_q + i), __ldg(t.p_inv_mod_q_sh + i), q);
+        u64 r = mul_tc(d, t.p_inv_tc + 4ull * i, pc);
         if (h == 0 && has_c0) r = add_mod(r, scratch[t0.at(zc) + li], q);
         if (has_acc) r = add_mod(r, arena[(h ? acc1.at(zc) : acc0.at(zc)) + li], q);
         arena[(h ? out1.at(zc) : out0.at(zc)) + li] = r;

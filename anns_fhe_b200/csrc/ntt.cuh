@@ -181,6 +181,7 @@ struct ZBases {
 
 // Plain prologue / epilogue.
 struct LoadPlain {
+    static constexpr bool kMany = false;      // one value a call
     const u64* base;
     __device__ __forceinline__ u64 operator()(const LimbJob& j, const ZBases& zb, uint32_t z, u64 x,
                                               const PrimeConst&) const {
@@ -277,6 +278,68 @@ __device__ __forceinline__ u64 sp_mul(u64 a, u64 w0, u64 w1, double s0, double s
     th += cl * (uint32_t)(nq >> 32);
     th += ch * (uint32_t)nq;
     return ((u64)th << 32) | (uint32_t)t;
+}
+
+// A canonical residue times a constant (transform_constant's form), canonical.
+__device__ __forceinline__ u64 mul_tc(u64 a, const u64* __restrict__ k, const PrimeConst& pc) {
+    const ulonglong2 w = __ldg((const ulonglong2*)k);
+    if (pc.fp) return fp_canon(fp_mul(fp_of(a), as_double(w.x), as_double(w.y), pc.qd), pc.qd);
+    const ulonglong2 s = __ldg((const ulonglong2*)k + 1);
+    const u64 nq = (u64)0 - pc.q;
+    return csub(sp_mul(a, w.x, w.y, as_double(s.x), as_double(s.y), nq, sp_start(nq)), pc.q);
+}
+// The product of two canonical residues below 2^50, in (-0.76q, 0.76q): the
+// quotient from the rounded product is off by less than 0.76, the rest is exact.
+__device__ __forceinline__ double fp_mul2(double a, double b, double q, double qi) {
+    const double h = __dmul_rn(a, b);
+    const double l = __fma_rn(a, b, -h);
+    const double c = __dadd_rn(__fma_rn(h, qi, kFpRound), -kFpRound);
+    return __dadd_rn(__fma_rn(-c, q, h), l);
+}
+
+// Base conversions of M values at a time: o[e] = sum over i < size of y(i, e) w_i
+// mod q, canonical, w_i = split constants at tab + 4 i row (any q < 2^61). The
+// products' low words are summed mod 2^64 and the quotient by q in doubles
+// rounded down (sp_mul's form for a sum), so one reduction serves the whole sum
+// (a Shoup product for each term costs 2.5 times the multiplier's cycles).
+template <int M, class Y>
+__device__ __forceinline__ void bconv(u64* o, uint32_t size, const u64* __restrict__ tab, uint32_t row, u64 q, Y&& y) {
+    const u64 nq = (u64)0 - q;
+    double m[M];
+    u64 t[M];
+#pragma unroll
+    for (uint32_t e = 0; e < M; ++e) {
+        t[e] = 0;
+        m[e] = 0;
+    }
+#pragma unroll 1
+    for (uint32_t i = 0; i < size; ++i) {
+        const ulonglong2 w = __ldg((const ulonglong2*)(tab + 4ull * i * row));
+        const ulonglong2 s = __ldg((const ulonglong2*)(tab + 4ull * i * row) + 1);
+        const double s0 = as_double(s.x), s1 = as_double(s.y);
+        u64 v[M];
+#pragma unroll
+        for (uint32_t e = 0; e < M; ++e) v[e] = y(i, e);
+#pragma unroll
+        for (uint32_t e = 0; e < M; ++e) {
+            const uint32_t a0 = (uint32_t)v[e], a1 = (uint32_t)(v[e] >> 32);
+            m[e] = __fma_rd(__hiloint2double(0, (int)a0), s0, __fma_rd(__hiloint2double(0, (int)a1), s1, m[e]));
+            u64 x = mad_wide_u32(a0, (uint32_t)w.x, t[e]);
+            x = mad_wide_u32(a1, (uint32_t)w.y, x);
+            uint32_t xh = (uint32_t)(x >> 32) + a0 * (uint32_t)(w.x >> 32);
+            xh += a1 * (uint32_t)(w.y >> 32);
+            t[e] = ((u64)xh << 32) | (uint32_t)x;
+        }
+    }
+#pragma unroll
+    for (uint32_t e = 0; e < M; ++e) {
+        const double c = __dadd_rd(m[e], kSpRound);
+        const uint32_t cl = (uint32_t)__double2loint(c), ch = (uint32_t)__double2hiint(c) - kSpHigh;
+        const u64 x = mad_wide_u32(cl, (uint32_t)nq, t[e]);
+        uint32_t xh = (uint32_t)(x >> 32) + cl * (uint32_t)(nq >> 32);
+        xh += ch * (uint32_t)nq;
+        o[e] = csub(((u64)xh << 32) | (uint32_t)x, q);
+    }
 }
 
 // Values between rounds: forward below 6.5q and at least 0.49q (or canonical,
@@ -622,7 +685,8 @@ __device__ __forceinline__ void ntt_pass(u64* sm, const PrimeTables& pt, const L
     constexpr bool DIRECT_IN = COL || R::rb(0) > 0, DIRECT_OUT = COL || R::rb(NR - 1) > 0;
     const uint32_t z = blockIdx.z;
     u64* const mp = mid + zb.mid.at(z) + job.dst;
-    const PrimeConst pc = pt.pc[job.prime];
+    PrimeConst pc = pt.pc[job.prime];
+    pc.fp = A::kSecond ? 0 : 1;             // (known where prologue and epilogue branch on it)
     const u64* const fin = pt.pc[job.prime].nv;
     const typename A::C c = A::consts(pc);
     const TwRow tw = tw_row<INV>(pt, job.prime, LOGN);
@@ -634,7 +698,7 @@ __device__ __forceinline__ void ntt_pass(u64* sm, const PrimeTables& pt, const L
         return ((u64)b << LO) + tile0 + col;
     };
     auto fetch = [&](u64 x) -> u64 {
-        if constexpr (first) return A::store(A::of(pro(job, zb, z, x, pc)));
+        if constexpr (first && !Pro::kMany) return A::store(A::of(pro(job, zb, z, x, pc)));
         else return mp[x];
     };
     auto put = [&](u64 x, u64 v, bool canonical) {
@@ -649,8 +713,19 @@ __device__ __forceinline__ void ntt_pass(u64* sm, const PrimeTables& pt, const L
             const typename Rd::Group gr = Rd::group(gi, tile0);
             const u64 x = gidx(gr.base_e);
             typename A::V v[Rd::NK];
+            if constexpr (first && Pro::kMany) {
+                constexpr uint32_t M = Rd::NK < 4 ? Rd::NK : 4;
 #pragma unroll
-            for (uint32_t j = 0; j < Rd::NK; ++j) v[j] = A::load(fetch(x + j * Rd::STEP_X));
+                for (uint32_t j = 0; j < Rd::NK; j += M) {
+                    u64 o[M];
+                    pro.template many<M>(o, job, zb, z, x + j * Rd::STEP_X, Rd::STEP_X, pc);
+#pragma unroll
+                    for (uint32_t i = 0; i < M; ++i) v[j + i] = A::of(o[i]);
+                }
+            } else {
+#pragma unroll
+                for (uint32_t j = 0; j < Rd::NK; ++j) v[j] = A::load(fetch(x + j * Rd::STEP_X));
+            }
             Rd::run_regs(v, tw, gr.blk, c, fin, !first, false);
             u64* const sp = sm + padix(gr.base_e);
 #pragma unroll
@@ -658,6 +733,7 @@ __device__ __forceinline__ void ntt_pass(u64* sm, const PrimeTables& pt, const L
         }
         __syncthreads();
     } else {
+        static_assert(!Pro::kMany, "a prologue of several values needs a first round from memory");
         const u64 x = gidx(threadIdx.x);
 #pragma unroll 8
         for (uint32_t k = 0; k < EPT; ++k) sm[padix(threadIdx.x) + padix(k * T)] = fetch(x + (u64)k * T);

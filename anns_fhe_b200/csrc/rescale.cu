@@ -12,33 +12,34 @@ namespace afhe {
 //           last limb times QlQlInvModqlDivqlModq[i], and whose epilogue is
 //           a_i * qlInvModq[i] + NTT(...)
 // ---------------------------------------------------------------------------
+// The lift times the constant as one product: where the coefficient is above
+// q_l / 2 (rescale.cpp:50 tie rule), -q_l mod q_i is added to it first (a sum
+// below 2^62, which the split product takes as it is).
 struct RescaleLoad {
+    static constexpr bool kMany = false;
     const u64* scratch;
     const u64* qlql;
-    const u64* qlql_sh;
     const PrimeConst* pc_last;   // q_l, the prime being dropped
     __device__ __forceinline__ u64 operator()(const LimbJob& j, const ZBases& zb, uint32_t z, u64 x,
                                               const PrimeConst& pc) const {
-        const u64 q = pc.q;
-        const u64 ql = pc_last->q, ql_half = ql >> 1;
+        const u64 q = pc.q, nq = (u64)0 - q;
+        const u64 ql = pc_last->q;
+        const u64 minus = q - csub(mul_shoup_lazy(ql, 1, pc.one_sh, q), q);
+        const ulonglong2 w = __ldg((const ulonglong2*)(qlql + 4ull * j.aux));
+        const ulonglong2 s = __ldg((const ulonglong2*)(qlql + 4ull * j.aux) + 1);
         u64 v = scratch[zb.aux.at(z) + x];                           // last limb coefficient, [0, q_l)
-        u64 vm = csub(mul_shoup_lazy(v, 1, pc.one_sh, q), q);         // v mod q_i
-        u64 qlm = csub(mul_shoup_lazy(ql, 1, pc.one_sh, q), q);       // q_l mod q_i
-        u64 val = (v > ql_half) ? sub_mod(vm, qlm, q) : vm;           // rescale.cpp:50 tie rule
-        return mul_shoup(val, __ldg(qlql + j.aux), __ldg(qlql_sh + j.aux), q);
+        v += v > (ql >> 1) ? minus : 0;
+        return csub(sp_mul(v, w.x, w.y, as_double(s.x), as_double(s.y), nq, sp_start(nq)), q);
     }
 };
 
 struct RescaleStore {
     u64* arena;
     const u64* qlinv;
-    const u64* qlinv_sh;
     __device__ __forceinline__ void operator()(const LimbJob& j, const ZBases& zb, uint32_t z, u64 x, u64 v,
                                                const PrimeConst& pc) const {
-        const u64 q = pc.q;
-        u64 a = arena[zb.src.at(z) + j.src + x];
-        u64 s = mul_shoup(a, __ldg(qlinv + j.aux), __ldg(qlinv_sh + j.aux), q);
-        arena[zb.out.at(z) + j.out + x] = add_mod(s, v, q);
+        const u64 a = arena[zb.src.at(z) + j.src + x];
+        arena[zb.out.at(z) + j.out + x] = add_mod(mul_tc(a, qlinv + 4ull * j.aux, pc), v, pc.q);
     }
 };
 
@@ -62,8 +63,8 @@ cudaError_t launch_rescale(int log_n, const OpTabs& t, const LimbJob* jobs_q, ui
     ZBases z2 = zb_in;
     z2.aux = zb_in.mid;                      // coefficients of the last limb
     z2.mid = zf_plus(zb_in.mid, n);          // intermediates
-    RescaleLoad pro{scratch, t.qlql, t.qlql_sh, t.pt.pc + last};
-    RescaleStore epi{arena, t.qlinv, t.qlinv_sh};
+    RescaleLoad pro{scratch, t.qlql_sp, t.pt.pc + last};
+    RescaleStore epi{arena, t.qlinv_tc};
     return launch_ntt<false>(log_n, t.pt, jobs_q, last, nz, scratch, z2, pro, epi, st);
 }
 
