@@ -579,10 +579,6 @@ struct NttRound {
         uint32_t c, brest;
         if (COL) { c = r & (C - 1u); brest = r >> LOGC; }
         else { brest = r & ((1u << (P - K)) - 1u); c = r >> (P - K); }
-        // The round at bit 3 has runs of eight neighbours, 2^6 or 2^7 apart; a
-        // half warp takes two runs 2^7 apart, whose padded places (8 banks of
-        // 16 apart, not 4) do not share banks.
-        if (!COL && RB == 3 && P - K >= 5) brest = (brest & ~24u) | ((brest & 8u) << 1) | ((brest & 16u) >> 1);
         const uint32_t base_b = ((brest >> RB) << (RB + K)) | (brest & ((1u << RB) - 1u));
         const uint32_t hb = COL ? 0u : (tile0 + c);     // index bits above the pass
         return Group{COL ? ((base_b << LOGC) | c) : ((c << P) | base_b), (hb << (P - RB - K)) | (brest >> RB)};
