@@ -423,14 +423,12 @@ int afhe_ctx_create(const afhe_params* prm, afhe_ctx** out) {
         {
             const char* v = std::getenv("AFHE_KS_FUSED");
             ctx->ks_fused = key_switch_fused_supported(ctx->log_n) && !(v && v[0] == '0');
-            // the one-kernel path carries a ciphertext per CTA (per cluster of
-            // N / 2^13 CTAs above N = 2^13): below half a wave of SMs a launch
-            // leaves most of the GPU idle, and the limb-parallel multi-kernel
-            // path is faster
+            // (below N = 2^13; above it the line is drawn by level, and this
+            // value stands for that)
             int sms = 148;
             cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
             const int cl = ctx->log_n > 13 ? 1 << (ctx->log_n - 13) : 1;
-            ctx->fused_min = (uint32_t)std::max(1, sms / (2 * cl));
+            ctx->fused_min = ctx->fused_default = (uint32_t)std::max(1, sms / (2 * cl));
             const char* m = std::getenv("AFHE_FUSED_MIN");
             if (m && std::atoi(m) >= 1) ctx->fused_min = (uint32_t)std::atoi(m);
         }

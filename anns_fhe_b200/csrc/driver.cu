@@ -92,6 +92,55 @@ int cached_map(afhe_ctx* ctx, uint32_t galois, const uint32_t** out) {
         if (_rc != AFHE_OK) return _rc;                                                 \
     } while (0)
 
+// How many of nz ciphertexts at level `limbs` the one-kernel key switch takes;
+// the kernel pipeline takes the rest. The one-kernel path runs `capacity`
+// ciphertexts at once and a partial wave costs nearly a whole one, the pipeline's
+// time grows with the count: whole waves and a remainder that nearly fills one
+// go to the former. The line lies where both took the same time (microseconds,
+// one kernel / pipeline): N = 2^13, three digits: 40: 203 / 164, 56: 205 / 215,
+// 148: 317 / 429, 160: 533 / 477; N = 2^14, three digits: 56: 1306 / 1179, 71: 1329
+// / 1476, 80: 2231 / 1653; N = 2^15, one digit (four limbs): 20: 416 / 390, 22: 418
+// / 420, 33: 441 / 603, 40: 797 / 716; three digits: 33: 1646 / 1627, 45: 3004 /
+// 2188; N = 2^16, one digit: 12: 783 / 754, 15: 803 / 934; two or more (8 limbs,
+// 24): 12: 1325 / 1072, 4521 / 3204.
+uint32_t ks_fused_part(afhe_ctx* ctx, uint32_t nz, uint32_t limbs) {
+    const bool by_level = ctx->fused_min == ctx->fused_default && ctx->log_n >= 13;
+    if (!ctx->ks_fused || nz < (by_level ? 2 : ctx->fused_min)) return 0;
+    if (ctx->fused_min == 1) return nz;
+    if (!ctx->ks_capacity) ctx->ks_capacity = std::max(1, key_switch_fused_capacity(ctx->log_n));
+    const uint32_t cap = ctx->ks_capacity;
+    uint32_t line = ctx->fused_min;
+    if (ctx->log_n >= 13) {
+        static const uint8_t percent[4][3] = {{5, 27, 35}, {63, 85, 90}, {65, 92, 255}, {85, 255, 255}};
+        const uint32_t share = percent[ctx->log_n - 13][std::min(ctx->lv[limbs].parts, 3u) - 1];
+        if (by_level && share == 255) return 0;
+        line = std::max(1u, cap * share / 100);
+        if (!by_level) line = std::min(line, ctx->fused_min);       // (nz is at least fused_min)
+    }
+    const uint32_t rest = nz % cap;
+    if (rest >= line || (rest == nz && !by_level)) return nz;
+    return nz - rest;
+}
+
+// nz key switches at one level: the first `fused` on the one-kernel path, the
+// others on the kernel pipeline.
+int ks_launch(afhe_ctx* ctx, ZBases zb, uint32_t fused, uint32_t nz, u64 evk, uint32_t limbs, const KsFuse* fuse,
+              const ulonglong2* prep, const ZField* lvz) {
+    const u64 S = (u64)ctx->L + ctx->K, evk_b = evk + (u64)ctx->dnum * S * ctx->n;
+    if (fused) {
+        CK(launch_key_switch_fused(ctx->log_n, ctx->lv_dev, ctx->alpha, limbs, ctx->K, ctx->key, evk, evk_b, (uint32_t)S,
+                                   ctx->L, ctx->poly, ctx->scr, fused, zb, ctx->st, fuse, prep, lvz));
+        if (fused == nz) return AFHE_OK;
+    }
+    KsFuse f{};
+    if (fuse) f = *fuse;
+    for (ZField* z : {&zb.src, &zb.out, &zb.aux, &zb.mid, &f.c0, &f.acc0, &f.acc1, &f.mapz, &f.keyz}) *z = zf_skip(*z, fused);
+    const LevelJobs& lj = ctx->lvjobs[limbs];
+    CK(launch_key_switch(ctx->log_n, ctx->lv[limbs], ctx->jobs_qp, lj.modup, lj.n_modup, ctx->L, limbs, ctx->K, ctx->key,
+                         evk, evk_b, (uint32_t)S, ctx->L, ctx->poly, ctx->scr, nz - fused, zb, ctx->st, fuse ? &f : nullptr));
+    return AFHE_OK;
+}
+
 // Key switch nz polynomials (poly_gmem-relative offsets) with one key, with
 // optional fusion (automorphism gather, c0 add, accumulate; see KsFuse).
 // `fused_ok` is false when an entry's outputs may overlap another entry's
@@ -101,24 +150,13 @@ int cached_map(afhe_ctx* ctx, uint32_t galois, const uint32_t** out) {
 int ks_batch(afhe_ctx* ctx, const ZField& in, const ZField& out0, const ZField& out1, uint32_t nz, u64 evk,
              uint32_t limbs, const KsFuse* fuse = nullptr, bool fused_ok = true, const ulonglong2* prep = nullptr,
              const ZField* lvz = nullptr) {
-    const u64 n = ctx->n, S = (u64)ctx->L + ctx->K;
-    const OpTabs& t = ctx->lv[limbs];
-    const LevelJobs& lj = ctx->lvjobs[limbs];
     ZBases zb{};
     zb.src = in;
     zb.out = out0;
     zb.aux = out1;
     zb.mid = lane_field(ctx, &Lane::ks);
     if (lvz && !(ctx->ks_fused && fused_ok)) return fail(ctx, AFHE_E_STATE, "mixed levels need the one-kernel key switch");
-    if (ctx->ks_fused && fused_ok && (lvz || nz >= ctx->fused_min)) {
-        CK(launch_key_switch_fused(ctx->log_n, ctx->lv_dev, ctx->alpha, limbs, ctx->K, ctx->key, evk, evk + (u64)ctx->dnum * S * n,
-                                   (uint32_t)S, ctx->L, ctx->poly, ctx->scr, nz, zb, ctx->st, fuse, prep, lvz));
-        return AFHE_OK;
-    }
-    CK(launch_key_switch(ctx->log_n, t, ctx->jobs_qp, lj.modup, lj.n_modup, ctx->L, limbs, ctx->K, ctx->key, evk,
-                         evk + (u64)ctx->dnum * S * n, (uint32_t)S, ctx->L, ctx->poly, ctx->scr, nz, zb, ctx->st,
-                         fuse));
-    return AFHE_OK;
+    return ks_launch(ctx, zb, lvz ? nz : fused_ok ? ks_fused_part(ctx, nz, limbs) : 0, nz, evk, limbs, fuse, prep, lvz);
 }
 
 // Rescale nz ciphertexts (in0, in1) -> (out0, out1), level limbs -> limbs - 1.
@@ -700,9 +738,7 @@ int afhe_eval_rotate_steps_batch(afhe_ctx* ctx, const afhe_ct_ref* in, const afh
     for (uint32_t i = 0; i < count; ++i)
         if (!ctx->rot.count(steps[i]))
             return fail(ctx, AFHE_E_NOKEY, "rotation key not found for step " + std::to_string(steps[i]));
-    const u64 n = ctx->n, S = (u64)ctx->L + ctx->K;
-    const OpTabs& t = ctx->lv[limbs];
-    const LevelJobs& lj = ctx->lvjobs[limbs];
+    const u64 n = ctx->n;
     // eval_rotate_single_step per entry (fhe_host_driver.cpp:331-359), each
     // with its own key and automorphism, in one key switch launch sequence.
     // The multi-kernel key switch reads every input before it writes any
@@ -732,19 +768,14 @@ int afhe_eval_rotate_steps_batch(afhe_ctx* ctx, const afhe_ct_ref* in, const afh
         ZF(zb.out, o0);
         ZF(zb.aux, o1);
         zb.mid = lane_field(ctx, &Lane::ks);
-        if (ctx->ks_fused && m >= ctx->fused_min && fused_rotation_safe(i0, i1, o0, o1, (u64)limbs * n)) {
-            const ulonglong2* prep = nullptr;
-            if (all_prep) {
-                ZF(f.prepz, preps);
-                prep = ctx->rot.at(steps[s]).prep;
-            }
-            CK(launch_key_switch_fused(ctx->log_n, ctx->lv_dev, ctx->alpha, limbs, ctx->K, ctx->key, 0, (u64)ctx->dnum * S * n, (uint32_t)S,
-                                       ctx->L, ctx->poly, ctx->scr, m, zb, ctx->st, &f, prep));
-            return AFHE_OK;
+        uint32_t fused = ks_fused_part(ctx, m, limbs);
+        if (fused && !fused_rotation_safe(i0, i1, o0, o1, (u64)limbs * n)) fused = 0;
+        const ulonglong2* prep = nullptr;
+        if (fused && all_prep) {
+            ZF(f.prepz, preps);
+            prep = ctx->rot.at(steps[s]).prep;
         }
-        CK(launch_key_switch(ctx->log_n, t, ctx->jobs_qp, lj.modup, lj.n_modup, ctx->L, limbs, ctx->K, ctx->key, 0,
-                             (u64)ctx->dnum * S * n, (uint32_t)S, ctx->L, ctx->poly, ctx->scr, m, zb, ctx->st, &f));
-        return AFHE_OK;
+        return ks_launch(ctx, zb, fused, m, 0, limbs, &f, prep, nullptr);
     });
 }
 

@@ -119,7 +119,10 @@ struct afhe_ctx {
     afhe::DescRing ring;
     bool ks_fused = true;   // one-kernel key switch where supported (AFHE_KS_FUSED=0 turns it off)
     uint32_t chunk = 0;     // ciphertexts per launch of a batched call (0: all lanes)
-    uint32_t fused_min = 1; // launches of fewer ciphertexts take the multi-kernel key switch
+    // launches (and remainders of whole waves) of fewer ciphertexts take the
+    // kernel pipeline; the same as fused_default: by level (ks_fused_part)
+    uint32_t fused_min = 1, fused_default = 0;
+    uint32_t ks_capacity = 0;   // ciphertexts the one-kernel key switch runs at once
     uint32_t ks_ept = 8;    // AFHE_OPT_KS_EPT and AFHE_OPT_KS_SLICE: kept for callers that set them
     uint32_t ks_slice = 13;
     // afhe_fence: fence f is event fences[f % size], recorded on st

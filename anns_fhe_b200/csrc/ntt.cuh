@@ -170,6 +170,12 @@ struct ZField {
 inline ZField zf_const(u64 v) { ZField f{}; f.base = v; return f; }
 inline ZField zf_stride(u64 base, u64 stride) { ZField f{}; f.base = base; f.stride = stride; return f; }
 inline ZField zf_plus(ZField f, u64 add) { f.add += add; return f; }
+// entries z0 and on (of a field without zf_pair)
+inline ZField zf_skip(ZField f, uint32_t z0) {
+    if (f.arr) f.arr += z0;
+    else f.base += (u64)z0 * f.stride;
+    return f;
+}
 inline ZField zf_pair(ZField f, u64 hdelta) { f.shift = 1; f.hdelta = hdelta; return f; }
 
 // The operands of one batched launch: meaning of src / out / aux is the

@@ -176,34 +176,33 @@ int afhe_copy_poly(afhe_ctx* ctx, uint64_t dst_offset, uint64_t src_offset, uint
 /* Run-time options of a context (no counterpart in the reference; the
  * autotuner, anns_fhe_b200/autotune.py, picks them per GPU and parameter set):
  *   AFHE_OPT_KS_FUSED  1: the one-kernel key switch (one CTA per ciphertext
- *                      at N <= 2^13, a cluster of N / 2^13 CTAs above), 0: the
- *                      multi-kernel pipeline. Same residues either way.
+ *                      at N <= 2^12, a cluster of N / 2^12 CTAs above, of
+ *                      eight at N = 2^16), 0: the multi-kernel pipeline. Same residues either way.
  *   AFHE_OPT_CHUNK     ciphertexts per launch of a batched call, 1..lanes
  *                      (0: all lanes). Same residues for any value. */
 #define AFHE_OPT_KS_FUSED 1u
 #define AFHE_OPT_CHUNK 2u
 /*   AFHE_OPT_FUSED_MIN launches of fewer ciphertexts than this take the
  *                      multi-kernel key switch even where the one-kernel path
- *                      is on (it carries one ciphertext per CTA, or per
- *                      cluster above N = 2^13, so a small launch leaves most
- *                      SMs idle). Default: half a wave of SMs. Same residues. */
+ *                      is on (a small launch leaves most SMs idle), and so does
+ *                      what is left of a larger launch after whole waves
+ *                      (AFHE_OPT_KS_CAPACITY) where a wave of its own would take
+ *                      longer; 1: every launch is one kernel. The default (half
+ *                      a wave of SMs, by one CTA per 2^13 coefficients) stands,
+ *                      from N = 2^13 on, for a line drawn by level. Same
+ *                      residues. */
 #define AFHE_OPT_FUSED_MIN 3u
 /*   AFHE_OPT_KS_CAPACITY (read only) ciphertexts the one-kernel key switch
  *                      runs at once on this GPU (CTAs, or clusters above
- *                      N = 2^13, resident together): a launch of a multiple
+ *                      N = 2^12, resident together): a launch of a multiple
  *                      of it fills its waves; 0 where it cannot run. */
 #define AFHE_OPT_KS_CAPACITY 4u
-/*   AFHE_OPT_KS_EPT    values per thread of the one-kernel key switch: 8
- *                      (N / 8 threads per CTA slice, the default) or 16 (half
- *                      the threads, twice the registers each). Same residues. */
+/*   AFHE_OPT_KS_EPT    8 or 16, AFHE_OPT_KS_SLICE 12 or 13: launch shapes of
+ *                      earlier one-kernel key switches. It has one shape now (16
+ *                      values per thread, slices of 2^12 coefficients, of 2^13 at
+ *                      N = 2^16); the values are kept for callers that set and
+ *                      read them and change nothing. */
 #define AFHE_OPT_KS_EPT 5u
-/*   AFHE_OPT_KS_SLICE  log2 of the slice each CTA of a cluster holds in the
- *                      one-kernel key switch at N = 2^14 and 2^15: 13 (the
- *                      default: clusters of N / 2^13 CTAs of 1024 threads, one
- *                      per SM) or 12 (clusters of N / 2^12 CTAs, two per SM:
- *                      512 threads with 8 values each, or 256 threads with 16
- *                      values each in radix-16 rounds). Ignored at other N.
- *                      Same residues. */
 #define AFHE_OPT_KS_SLICE 6u
 int afhe_ctx_set_option(afhe_ctx* ctx, uint32_t option, int64_t value);
 int afhe_ctx_get_option(afhe_ctx* ctx, uint32_t option, int64_t* value);
@@ -342,7 +341,7 @@ int afhe_decrypt_batch(afhe_ctx* ctx, const afhe_ct_ref* cts, uint32_t count, ui
  * context of that degree, from the next launch). Plans change only launch
  * shapes; every plan gives the same residues. N <= 2^13 (one pass over the
  * limb): 2 plans, values per thread 8 or 16. N >= 2^14 (two passes): 6 plans,
- * columns per CTA of the column pass (16, 8, 32) x words per tile of the
+ * columns per CTA of the column pass (32, 16, 64) x words per tile of the
  * chunk pass (4096, 8192). Plan 0 is the default. The autotuner
  * (anns_fhe_b200/autotune.py) times them. The one-kernel key switch has its
  * own transform and ignores the plan. */
