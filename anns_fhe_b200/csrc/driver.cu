@@ -160,9 +160,10 @@ int ks_batch(afhe_ctx* ctx, const ZField& in, const ZField& out0, const ZField& 
 }
 
 // Rescale nz ciphertexts (in0, in1) -> (out0, out1), level limbs -> limbs - 1.
-// The two polynomials of ciphertext z run as z' = 2z, 2z + 1.
+// The two polynomials of ciphertext z run as z' = 2z, 2z + 1. With pt: times
+// the plaintexts there.
 int rescale_batch(afhe_ctx* ctx, const Offs& in0, const Offs& in1, const Offs& out0, const Offs& out1,
-                  uint32_t limbs) {
+                  uint32_t limbs, const Offs* pt = nullptr) {
     const uint32_t nz = (uint32_t)in0.size();
     Offs src(2 * nz), out(2 * nz);
     for (uint32_t z = 0; z < nz; ++z) {
@@ -173,7 +174,13 @@ int rescale_batch(afhe_ctx* ctx, const Offs& in0, const Offs& in1, const Offs& o
     ZF(zb.src, src);
     ZF(zb.out, out);
     zb.mid = zf_pair(lane_field(ctx, &Lane::resc), (u64)ctx->L * ctx->n);
-    CK(launch_rescale(ctx->log_n, ctx->lv[limbs], ctx->jobs_qp, limbs, ctx->poly, ctx->scr, 2 * nz, zb, ctx->st));
+    ZField factor{};
+    if (pt) {
+        ZF(factor, *pt);
+        factor = zf_pair(factor, 0);
+    }
+    CK(launch_rescale(ctx->log_n, ctx->lv[limbs], ctx->jobs_qp, limbs, ctx->poly, ctx->scr, 2 * nz, zb, ctx->st,
+                      pt ? &factor : nullptr));
     return AFHE_OK;
 }
 
@@ -275,8 +282,9 @@ bool fused_rotation_safe(const Offs& i0, const Offs& i1, const Offs& o0, const O
 
 // Whether a rescale may read its inputs where they are: every output polynomial
 // is disjoint from every input polynomial (inputs span w words, outputs less),
-// or starts where its own input does.
-bool rescale_in_place_safe(const Offs& i0, const Offs& i1, const Offs& o0, const Offs& o1, u64 w) {
+// or starts where its own input does; and disjoint from the plaintexts, if any.
+bool rescale_in_place_safe(const Offs& i0, const Offs& i1, const Offs& o0, const Offs& o1, u64 w,
+                           const Offs* pt = nullptr) {
     const size_t nz = i0.size();
     std::vector<std::pair<u64, size_t>> outs;       // (start, polynomial)
     outs.reserve(2 * nz);
@@ -286,12 +294,12 @@ bool rescale_in_place_safe(const Offs& i0, const Offs& i1, const Offs& o0, const
     }
     std::sort(outs.begin(), outs.end());
     for (size_t z = 0; z < nz; ++z)
-        for (size_t h = 0; h < 2; ++h) {
-            const u64 a = h ? i1[z] : i0[z];
+        for (size_t h = 0; h < (pt ? 3 : 2); ++h) {
+            const u64 a = h == 2 ? (*pt)[z] : h ? i1[z] : i0[z];
             const u64 lo = a >= w ? a - w + 1 : 0;
             for (auto it = std::lower_bound(outs.begin(), outs.end(), std::make_pair(lo, (size_t)0));
                  it != outs.end() && it->first < a + w; ++it)
-                if (it->first != a || it->second != 2 * z + h) return false;
+                if (h == 2 || it->first != a || it->second != 2 * z + h) return false;
         }
     return true;
 }
@@ -579,8 +587,20 @@ int afhe_eval_mult_plain_rescale_batch(afhe_ctx* ctx, const afhe_ct_ref* a, cons
         return rc;
     for (uint32_t i = 0; i < count; ++i)
         if ((rc = check_poly(ctx, pt[i], limbs))) return rc;
-    // fhe_host_driver.cpp:308-329: (c0 * pt, c1 * pt), then rescale
+    // fhe_host_driver.cpp:308-329: (c0 * pt, c1 * pt), then rescale. The products
+    // are formed inside the rescale, unless an output overlaps what they are
+    // formed of (other than its own input): then they go to lane temps first.
     return for_chunks(ctx, count, [&](uint32_t s, uint32_t m) {
+        {
+            Offs i0(m), i1(m), o0(m), o1(m), f(m);
+            for (uint32_t z = 0; z < m; ++z) {
+                i0[z] = a[s + z].c0_offset; i1[z] = a[s + z].c1_offset;
+                o0[z] = d[s + z].c0_offset; o1[z] = d[s + z].c1_offset;
+                f[z] = pt[s + z];
+            }
+            if (rescale_in_place_safe(i0, i1, o0, o1, (u64)limbs * ctx->n, &f))
+                return rescale_batch(ctx, i0, i1, o0, o1, limbs, &f);
+        }
         Offs A(2 * m), P(2 * m), T(2 * m), t0(m), t1(m), o0(m), o1(m);
         for (uint32_t z = 0; z < m; ++z) {
             t0[z] = lane_temp(ctx, z, 0);

@@ -236,9 +236,10 @@ cudaError_t launch_ntt_plain(bool inverse, int log_n, const PrimeTables& pt, con
 // Rescale of nz polynomials at level sizeQl: zb.src = input polys (arena),
 // zb.out = outputs (arena), zb.mid = scratch for the last limb's coefficients
 // (scratch arena, N words each), zb.aux = scratch for pass intermediates
-// ((sizeQl - 1) * N words each).
+// ((sizeQl - 1) * N words each). With pt: of the products with the polynomials
+// at pt (arena).
 cudaError_t launch_rescale(int log_n, const OpTabs& t, const LimbJob* jobs_q, uint32_t sizeQl, u64* arena,
-                           u64* scratch, uint32_t nz, const ZBases& zb, cudaStream_t st);
+                           u64* scratch, uint32_t nz, const ZBases& zb, cudaStream_t st, const ZField* pt = nullptr);
 
 // Key switch of nz polynomials at level sizeQl. Per z: zb.src = input poly
 // (arena), zb.out = ks0 output, zb.aux = ks1 output (arena), zb.mid = scratch

@@ -43,11 +43,37 @@ struct RescaleStore {
     }
 };
 
+// The same of the product with a plaintext (pt.at(z): its polynomial), which is
+// formed where the transforms read it and written nowhere.
+__device__ __forceinline__ u64 product(u64 a, u64 b, const PrimeConst& pc) {
+    if (pc.fp) return fp_canon(fp_mul2(fp_of(a), fp_of(b), pc.qd, pc.qi), pc.qd);
+    return mul_mod(a, b, modconst_of(pc));
+}
+struct LoadProduct {
+    static constexpr bool kMany = false;
+    const u64* arena;
+    ZField pt;
+    __device__ __forceinline__ u64 operator()(const LimbJob& j, const ZBases& zb, uint32_t z, u64 x,
+                                              const PrimeConst& pc) const {
+        return product(arena[zb.src.at(z) + j.src + x], arena[pt.at(z) + j.src + x], pc);
+    }
+};
+struct RescaleProductStore {
+    u64* arena;
+    const u64* qlinv;
+    ZField pt;
+    __device__ __forceinline__ void operator()(const LimbJob& j, const ZBases& zb, uint32_t z, u64 x, u64 v,
+                                               const PrimeConst& pc) const {
+        const u64 a = product(arena[zb.src.at(z) + j.src + x], arena[pt.at(z) + j.src + x], pc);
+        arena[zb.out.at(z) + j.out + x] = add_mod(mul_tc(a, qlinv + 4ull * j.aux, pc), v, pc.q);
+    }
+};
+
 // zb.src = input poly (arena), zb.out = output poly (arena), zb.mid = scratch
 // region of sizeQl * N words per z: words [0, N) hold the last limb's
 // coefficients, words [N, sizeQl * N) the step-2 intermediates.
 cudaError_t launch_rescale(int log_n, const OpTabs& t, const LimbJob* jobs_q, uint32_t sizeQl, u64* arena,
-                           u64* scratch, uint32_t nz, const ZBases& zb_in, cudaStream_t st) {
+                           u64* scratch, uint32_t nz, const ZBases& zb_in, cudaStream_t st, const ZField* pt) {
     if (sizeQl < 2 || nz == 0) return cudaSuccess;
     const u64 n = 1ull << log_n;
     const uint32_t last = sizeQl - 1;
@@ -56,16 +82,19 @@ cudaError_t launch_rescale(int log_n, const OpTabs& t, const LimbJob* jobs_q, ui
     ZBases z1 = zb_in;
     z1.mid = zf_plus(zb_in.mid, (u64)0 - (u64)last * n);
     z1.out = z1.mid;
-    cudaError_t e = launch_ntt<true>(log_n, t.pt, jobs_q + last, 1, nz, scratch, z1, LoadPlain{arena},
-                                     StorePlain{scratch}, st);
+    cudaError_t e = pt ? launch_ntt<true>(log_n, t.pt, jobs_q + last, 1, nz, scratch, z1, LoadProduct{arena, *pt},
+                                          StorePlain{scratch}, st)
+                       : launch_ntt<true>(log_n, t.pt, jobs_q + last, 1, nz, scratch, z1, LoadPlain{arena},
+                                          StorePlain{scratch}, st);
     if (e != cudaSuccess) return e;
     // step 2
     ZBases z2 = zb_in;
     z2.aux = zb_in.mid;                      // coefficients of the last limb
     z2.mid = zf_plus(zb_in.mid, n);          // intermediates
     RescaleLoad pro{scratch, t.qlql_sp, t.pt.pc + last};
-    RescaleStore epi{arena, t.qlinv_tc};
-    return launch_ntt<false>(log_n, t.pt, jobs_q, last, nz, scratch, z2, pro, epi, st);
+    if (pt)
+        return launch_ntt<false>(log_n, t.pt, jobs_q, last, nz, scratch, z2, pro, RescaleProductStore{arena, t.qlinv_tc, *pt}, st);
+    return launch_ntt<false>(log_n, t.pt, jobs_q, last, nz, scratch, z2, pro, RescaleStore{arena, t.qlinv_tc}, st);
 }
 
 }  // namespace afhe

@@ -101,3 +101,41 @@ def test_rescale_over_its_inputs(log_n, limbs):
                 assert np.array_equal(x, y), name
     finally:
         ctx.close()
+
+
+@pytest.mark.parametrize("log_n,limbs,q_bits", [(11, 2, 40), (13, 3, 55), (14, 3, 40)])
+def test_plaintext_product_over_its_operands(log_n, limbs, q_bits):
+    """The product formed inside the rescale equals the one through temporaries
+    (outputs over the plaintexts or another input), shared plaintexts included."""
+    q, p = primes_for(log_n, limbs, q_bits, 1, 60)
+    n = 1 << log_n
+    w = limbs * n
+    ctx = FheContext(CkksParams(log_n, q, p, 1), poly_words=64 * w, key_words=1024)
+    count = 5
+    try:
+        rng = np.random.default_rng([log_n, limbs])
+        data = [uniform_residues(rng, q, n) for _ in range(3 * count)]
+        data[0] = np.repeat(np.array(q, dtype=np.uint64) - 1, n)
+        data[2 * count] = data[0]
+        ins = [(2 * i * w, (2 * i + 1) * w) for i in range(count)]
+        pts = [(2 * count + i % 3) * w for i in range(count)]
+
+        def run(outs):
+            ctx.write_poly(0, np.concatenate(data))
+            a = (L.CtRef * count)(*[L.CtRef(*c) for c in ins])
+            d = (L.CtRef * count)(*[L.CtRef(*c) for c in outs])
+            f = (L.u64 * count)(*pts)
+            L.check(ctx.lib.afhe_eval_mult_plain_rescale_batch(ctx.h, a, f, d, count, limbs), "mult_plain_rescale")
+            return [ctx.read_poly(o, w - n) for c in outs for o in c]
+
+        over = run([((2 * count) * w, (2 * count + 1) * w)] + [((32 + 2 * i) * w, (33 + 2 * i) * w) for i in range(1, count)])
+        arrangements = {
+            "apart": [((32 + 2 * i) * w, (33 + 2 * i) * w) for i in range(count)],
+            "in place": ins,
+            "turned": ins[1:] + ins[:1],
+        }
+        for name, outs in arrangements.items():
+            for x, y in zip(over, run(outs)):
+                assert np.array_equal(x, y), name
+    finally:
+        ctx.close()
