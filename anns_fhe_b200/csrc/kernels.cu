@@ -54,8 +54,7 @@ __global__ void __launch_bounds__(256) elementwise_kernel(const PrimeConst* __re
         u64 r = x[k];
         if (OP == EW_ADD) r = add_mod(x[k], y[k], p.q);
         else if (OP == EW_SUB) r = sub_mod(x[k], y[k], p.q);
-        else if (OP == EW_MUL) r = p.fp ? fp_canon(fp_mul2(fp_of(x[k]), fp_of(y[k]), p.qd, p.qi), p.qd)
-                                        : mul_mod(x[k], y[k], modconst_of(p));
+        else if (OP == EW_MUL) r = mul_words(x[k], y[k], p);
         if (i0 + 256 * k < n) o[256 * k] = r;
     }
 }
@@ -93,7 +92,7 @@ __global__ void __launch_bounds__(256) tensor_kernel(const PrimeConst* __restric
     u64* d2 = arena + ta.d2.at(z) + off;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         u64 x0 = a0[i], x1 = a1[i], y0 = b0[i], y1 = b1[i];
-        if (p.fp) {
+        if (p.fp && x0 < p.q && x1 < p.q && y0 < p.q && y1 < p.q) {
             const double f0 = fp_of(x0), f1 = fp_of(x1), g0 = fp_of(y0), g1 = fp_of(y1);
             const double c = __dadd_rn(fp_mul2(f0, g1, p.qd, p.qi), fp_mul2(f1, g0, p.qd, p.qi));
             d0[i] = fp_canon(fp_mul2(f0, g0, p.qd, p.qi), p.qd);

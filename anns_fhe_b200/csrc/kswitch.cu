@@ -82,7 +82,8 @@ struct StoreSlot {   // plain store into scratch
 // Inner product with the evaluation key. One thread per (slot, coefficient).
 // slot s < sizeQl is Q limb s, slot slots_q + k is special limb k. The operands
 // of up to four digits are on their way before the first is used; products of
-// primes below 2^50 in doubles, else summed in 128 bits and reduced once.
+// residues of primes below 2^50 in doubles, else (also where a key's word is no
+// residue) summed in 128 bits and reduced once.
 __global__ void __launch_bounds__(256) ks_mac_kernel(OpTabs t, uint32_t n, uint32_t slots_q, uint32_t sizeQl,
                                                      uint32_t K, const u64* __restrict__ key, u64 evk_a, u64 evk_b,
                                                      uint32_t key_stride, uint32_t key_pbase,
@@ -111,6 +112,7 @@ __global__ void __launch_bounds__(256) ks_mac_kernel(OpTabs t, uint32_t n, uint3
         acc_init(ab);
         acc_init(aa);
         double fb = 0, fa = 0;
+        bool words = !pc.fp;                    // something in ab, aa
         constexpr uint32_t D = 4;
         for (uint32_t part0 = 0; part0 < t.parts; part0 += D) {
             u64 d[D], kb[D], ka[D];
@@ -133,18 +135,24 @@ __global__ void __launch_bounds__(256) ks_mac_kernel(OpTabs t, uint32_t n, uint3
 #pragma unroll
             for (uint32_t e = 0; e < D; ++e) {
                 if (part0 + e >= t.parts) break;
-                if (pc.fp) {
+                if (pc.fp && d[e] < pc.q && kb[e] < pc.q && ka[e] < pc.q) {
                     const double f = fp_of(d[e]);
                     fb = fp_center(__dadd_rn(fb, fp_mul2(f, fp_of(kb[e]), pc.qd, pc.qi)), pc.qd, pc.qi);
                     fa = fp_center(__dadd_rn(fa, fp_mul2(f, fp_of(ka[e]), pc.qd, pc.qi)), pc.qd, pc.qi);
                 } else {
+                    words = true;
                     acc_mad(ab, d[e], kb[e]);
                     acc_mad(aa, d[e], ka[e]);
                 }
             }
         }
-        scratch[base_scr + ext0_off + (u64)slot * n + x] = pc.fp ? fp_canon(fb, pc.qd) : acc_reduce(ab, mc);
-        scratch[base_scr + ext1_off + (u64)slot * n + x] = pc.fp ? fp_canon(fa, pc.qd) : acc_reduce(aa, mc);
+        u64 r0 = pc.fp ? fp_canon(fb, pc.qd) : 0, r1 = pc.fp ? fp_canon(fa, pc.qd) : 0;
+        if (words) {
+            r0 = add_mod(r0, acc_reduce(ab, mc), pc.q);
+            r1 = add_mod(r1, acc_reduce(aa, mc), pc.q);
+        }
+        scratch[base_scr + ext0_off + (u64)slot * n + x] = r0;
+        scratch[base_scr + ext1_off + (u64)slot * n + x] = r1;
     }
 }
 

@@ -303,6 +303,13 @@ __device__ __forceinline__ double fp_mul2(double a, double b, double q, double q
     return __dadd_rn(__fma_rn(-c, q, h), l);
 }
 
+// The product of any two words, canonical: in doubles where both are residues
+// of a prime below 2^50, else 128 bits and their reduction.
+__device__ __forceinline__ u64 mul_words(u64 a, u64 b, const PrimeConst& pc) {
+    if (pc.fp && a < pc.q && b < pc.q) return fp_canon(fp_mul2(fp_of(a), fp_of(b), pc.qd, pc.qi), pc.qd);
+    return mul_mod(a, b, modconst_of(pc));
+}
+
 // Base conversions of M values at a time: o[e] = sum over i < size of y(i, e) w_i
 // mod q, canonical, w_i = split constants at tab + 4 i row (any q < 2^61). The
 // products' low words are summed mod 2^64 and the quotient by q in doubles

@@ -38,24 +38,21 @@ struct RescaleStore {
     const u64* qlinv;
     __device__ __forceinline__ void operator()(const LimbJob& j, const ZBases& zb, uint32_t z, u64 x, u64 v,
                                                const PrimeConst& pc) const {
-        const u64 a = arena[zb.src.at(z) + j.src + x];
+        u64 a = arena[zb.src.at(z) + j.src + x];
+        if (a >= pc.q) a = reduce128(0, a, modconst_of(pc));        // (a word that is no residue)
         arena[zb.out.at(z) + j.out + x] = add_mod(mul_tc(a, qlinv + 4ull * j.aux, pc), v, pc.q);
     }
 };
 
 // The same of the product with a plaintext (pt.at(z): its polynomial), which is
 // formed where the transforms read it and written nowhere.
-__device__ __forceinline__ u64 product(u64 a, u64 b, const PrimeConst& pc) {
-    if (pc.fp) return fp_canon(fp_mul2(fp_of(a), fp_of(b), pc.qd, pc.qi), pc.qd);
-    return mul_mod(a, b, modconst_of(pc));
-}
 struct LoadProduct {
     static constexpr bool kMany = false;
     const u64* arena;
     ZField pt;
     __device__ __forceinline__ u64 operator()(const LimbJob& j, const ZBases& zb, uint32_t z, u64 x,
                                               const PrimeConst& pc) const {
-        return product(arena[zb.src.at(z) + j.src + x], arena[pt.at(z) + j.src + x], pc);
+        return mul_words(arena[zb.src.at(z) + j.src + x], arena[pt.at(z) + j.src + x], pc);
     }
 };
 struct RescaleProductStore {
@@ -64,7 +61,7 @@ struct RescaleProductStore {
     ZField pt;
     __device__ __forceinline__ void operator()(const LimbJob& j, const ZBases& zb, uint32_t z, u64 x, u64 v,
                                                const PrimeConst& pc) const {
-        const u64 a = product(arena[zb.src.at(z) + j.src + x], arena[pt.at(z) + j.src + x], pc);
+        const u64 a = mul_words(arena[zb.src.at(z) + j.src + x], arena[pt.at(z) + j.src + x], pc);
         arena[zb.out.at(z) + j.out + x] = add_mod(mul_tc(a, qlinv + 4ull * j.aux, pc), v, pc.q);
     }
 };

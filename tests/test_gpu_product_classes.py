@@ -51,3 +51,24 @@ def test_products_against_oracle(log_n, alpha, orc):
                 want = ora.eval_mult_relin_rescale((x[0], x[1]), (x[2], x[3]), (key[:kw // 2], key[kw // 2:]), lv)
                 for h in range(2):
                     assert np.array_equal(ctx.read_poly((4 + h) * w, (lv - 1) * n), want[h]), (lv, top, h)
+
+
+@pytest.mark.parametrize("bits", [36, 50, 61])
+def test_products_of_words_that_are_no_residues(bits):
+    """Pointwise products reduce any two words exactly, whatever the prime's form."""
+    log_n = 11
+    q = find_ntt_primes(log_n, bits, 1, [])
+    n = 1 << log_n
+    p = CkksParams(log_n, q, find_ntt_primes(log_n, 60, 1, q), 1)
+    rng = np.random.default_rng(bits)
+    a = rng.integers(0, 1 << 64, n, dtype=np.uint64)
+    b = rng.integers(0, 1 << 64, n, dtype=np.uint64)
+    a[::3] %= np.uint64(q[0])
+    b[::2] %= np.uint64(q[0])
+    with FheContext(p, poly_words=3 * n, key_words=1024, max_batch=1) as ctx:
+        ctx.write_poly(0, a)
+        ctx.write_poly(n, b)
+        FHEHostDriver(ctx).poly_mul_ntt(0, n, 2 * n, 1)
+        got = ctx.read_poly(2 * n, n)
+    want = (a.astype(object) * b.astype(object)) % q[0]
+    assert np.array_equal(got, want.astype(np.uint64))
