@@ -36,8 +36,8 @@ class KsChoice:
     fused: bool
     chunk: int
     us_per_ct: float
-    ept: int = 8          # values per thread of the one-kernel key switch (AFHE_OPT_KS_EPT)
-    slice: int = 13       # log2 of a cluster CTA's slice (AFHE_OPT_KS_SLICE; 12 at N = 2^14, 2^15)
+    ept: int = 8          # AFHE_OPT_KS_EPT and AFHE_OPT_KS_SLICE: set and reported, without effect
+    slice: int = 13       # (the one-kernel key switch has one shape per ring degree)
     fused_min: int = 0    # launches of fewer ciphertexts take the multi-kernel path (0: context default)
 
 
@@ -76,7 +76,7 @@ TIE = 0.10   # candidates within this fraction of the fastest count as ties
 # Version of the key-switch kernels a cache was tuned against: a cache from
 # other kernels (e.g. before the one-kernel path existed at this ring degree)
 # is tuned again.
-KERNELS = 8
+KERNELS = 9
 
 
 def ntt_plan_count(log_n: int) -> int:
@@ -213,14 +213,7 @@ def tune(params: CkksParams, levels, lanes: int, device: int = 0, verbose: bool 
             ctx.write_poly(i * w_max, np.concatenate([rng.integers(0, q, n, dtype=np.uint64)
                                                       for q in params.q[:max(levels)]]))
         fused_ok = ctx.get_option(L.OPT_KS_FUSED) == 1    # the context enables it where the GPU can run it
-        shapes = [(True, 8, 13), (True, 16, 13), (False, 8, 13)] if fused_ok else [(False, 8, 13)]
-        if fused_ok and params.log_n in (14, 15):
-            try:
-                ctx.set_option(L.OPT_KS_SLICE, 12)
-                shapes[2:2] = [(True, 8, 12), (True, 16, 12)]
-            except L.AfheError:
-                pass                     # two CTAs per SM cannot be placed in clusters here
-            ctx.set_option(L.OPT_KS_SLICE, 13)
+        shapes = [(True, 8, 13), (False, 8, 13)] if fused_ok else [(False, 8, 13)]
         out = {}
         for lv in sorted(set(levels)):
             timings = {}

@@ -21,24 +21,15 @@ import time
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
-# DRAM traffic and integer-pipe use of the key switch from ncu captures of the
-# current kernels (`--set full`, clocks not locked), per (N, l, K, slice): the
-# traffic of one launch sequence per ciphertext (its scratch and I/O grow with
-# the ciphertexts), the key's bytes read once, the kernel, and the busiest
-# integer pipe's utilisation. The captures are summarised under profiles/.
+# DRAM traffic and the busiest arithmetic pipe of the key switch from an ncu
+# capture of the current kernel (clocks not locked), per (N, l, K): the traffic
+# of one launch per ciphertext (its scratch and I/O grow with the ciphertexts),
+# the key's bytes read once, the kernel, and the pipe's utilisation. The
+# capture is summarised under profiles/.
 KS_CAPTURES: dict = {
-    (8192, 3, 1, 13): {"kernel": "ks_fused_kernel<13, 1>", "ciphertexts": 148, "dram_bytes": 175.3e6,
-                       "pipe": "fmaheavy (IMAD)", "util": 0.580},
-    # clusters of 4 CTAs of 2^13-value slices, one per SM; 37 clusters ran as
-    # two waves (33 resident at once)
-    (32768, 3, 4, 13): {"kernel": "ks_fused_kernel<13, 2, 1>", "ciphertexts": 37, "dram_bytes": 402.9e6,
-                        "pipe": "alu", "util": 0.387},
-    # clusters of 8 CTAs of 2^12-value slices, two per SM; 66 = two full waves
-    (32768, 3, 4, 12): {"kernel": "ks_fused_kernel<12, 3, 1, 8>", "ciphertexts": 66, "dram_bytes": 715.8e6,
-                        "pipe": "alu", "util": 0.370},
-    # the diagonal chain's evaluation level (2 + 4 limbs), same shape
-    (32768, 2, 4, 12): {"kernel": "ks_fused_kernel<12, 3, 1, 8>", "ciphertexts": 66, "dram_bytes": 522.2e6,
-                        "pipe": "alu", "util": 0.371},
+    # the diagonal chain's evaluation level: clusters of 8 CTAs, 33 resident
+    (32768, 2, 4): {"kernel": "ks_fused_kernel<12, 3, 1, 1>", "ciphertexts": 240, "dram_bytes": 2506e6,
+                    "pipe": "fmaheavy (IMAD)", "util": 0.344},
 }
 
 
@@ -82,7 +73,6 @@ def ks_roofline(params, lanes: int, reps: int = 20, level: int = 0, nbuf: int = 
             ctx.set_option(2, min(int(choice.chunk), lanes))
             ctx.set_option(5, int(getattr(choice, "ept", 8)))
             ctx.set_option(6, int(getattr(choice, "slice", 13)))
-        ept, slc = ctx.get_option(5), ctx.get_option(6)
         limb = np.concatenate([rng.integers(0, q, n, dtype=np.uint64) for q in p.q[:L]])
         for i in range((nbuf + 1) * lanes * 2):
             ctx.write_poly(i * w, limb)
@@ -114,15 +104,14 @@ def ks_roofline(params, lanes: int, reps: int = 20, level: int = 0, nbuf: int = 
     bytes_per_call = lanes * 4 * w * 8 + key_bytes
     achieved = bytes_per_call / (ms * 1e-3) / 1e9
     peak, src = load_peaks()
-    cap = KS_CAPTURES.get((n, L, K, slc if n >= 1 << 14 else 13))
+    cap = KS_CAPTURES.get((n, L, K))
     traffic = int_pipe = None
-    if cap and launches == 1 and fused and ept == cap.get("ept", 8):
+    if cap and launches == 1 and fused:
         # the capture's per-ciphertext traffic scaled to this launch, the key once
         traffic = (cap["dram_bytes"] - key_bytes) * lanes / cap["ciphertexts"] + key_bytes
         int_pipe = {"pipe": cap["pipe"], "frac": cap["util"], "kernel": cap["kernel"],
                     "captured_ciphertexts": cap["ciphertexts"]}
-    shape = f", 2^{slc}-value slices" if n >= 1 << 14 else ""
-    kind = f"one-kernel, {ept} values per thread{shape}" if fused and launches == 1 else f"{launches:g}-launch"
+    kind = "one kernel" if fused and launches == 1 else f"{launches:g} launches"
     return {"bound": "hbm", "kernel": f"rotation key switch, {kind} (N={n}, {L} + {K} limbs, "
                                       f"{lanes} ciphertexts per call)",
             "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
