@@ -32,6 +32,10 @@ int cuda_fail(afhe_ctx* ctx, cudaError_t e, const char* where) {
     return fail(ctx, AFHE_E_CUDA, std::string(where) + ": " + cudaGetErrorString(e));
 }
 
+cudaError_t upload(afhe_ctx* ctx, void* dst, const void* src, size_t bytes) {
+    return bytes ? cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, ctx->st) : cudaSuccess;
+}
+
 u64 host_shoup(u64 w, u64 q) { return (u64)(((unsigned __int128)w << 64) / q); }
 
 // The primitive 2N-th root behind prime i's twiddles (Q primes first, then
@@ -212,14 +216,14 @@ int build_native_tables(afhe_ctx* ctx) {
     CK(dalloc(&s.itw2, (size_t)np * n));
     CK(dalloc(&s.tw2b, (size_t)np * n));
     CK(dalloc(&s.itw2b, (size_t)np * n));
-    CK(cudaMemcpy(s.pc, pc.data(), np * sizeof(PrimeConst), cudaMemcpyHostToDevice));
+    CK(upload(ctx, s.pc, pc.data(), np * sizeof(PrimeConst)));
     {
         u64* raw = nullptr;
         const size_t w = (size_t)np * n;
         CK(dalloc(&raw, 2 * w + np));
-        cudaError_t e = cudaMemcpy(raw, tw.data(), w * 8, cudaMemcpyHostToDevice);
-        if (e == cudaSuccess) e = cudaMemcpy(raw + w, itw.data(), w * 8, cudaMemcpyHostToDevice);
-        if (e == cudaSuccess) e = cudaMemcpy(raw + 2 * w, primes.data(), np * 8, cudaMemcpyHostToDevice);
+        cudaError_t e = upload(ctx, raw, tw.data(), w * 8);
+        if (e == cudaSuccess) e = upload(ctx, raw + w, itw.data(), w * 8);
+        if (e == cudaSuccess) e = upload(ctx, raw + 2 * w, primes.data(), np * 8);
         if (e == cudaSuccess) e = launch_twiddles(raw, raw + 2 * w, s.tw2, s.tw2b, np, ctx->log_n, ctx->st);
         if (e == cudaSuccess) e = launch_twiddles(raw + w, raw + 2 * w, s.itw2, s.itw2b, np, ctx->log_n, ctx->st);
         if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->st);
@@ -306,7 +310,7 @@ int build_native_tables(afhe_ctx* ctx) {
         R.qlinv = push_tc(qlinv, mr);
     }
     CK(dalloc(&ctx->lvbuf, buf.size()));
-    CK(cudaMemcpy(ctx->lvbuf, buf.data(), buf.size() * 8, cudaMemcpyHostToDevice));
+    CK(upload(ctx, ctx->lvbuf, buf.data(), buf.size() * 8));
     ctx->lv.assign(L + 1, OpTabs{});
     for (uint32_t lvl = 1; lvl <= L; ++lvl) {
         OpTabs& t = ctx->lv[lvl];
@@ -333,7 +337,7 @@ int build_native_tables(afhe_ctx* ctx) {
     // the same tables as one device array, for launches whose entries run at
     // different levels
     CK(dalloc(&ctx->lv_dev, L + 1));
-    CK(cudaMemcpy(ctx->lv_dev, ctx->lv.data(), (L + 1) * sizeof(OpTabs), cudaMemcpyHostToDevice));
+    CK(upload(ctx, ctx->lv_dev, ctx->lv.data(), (L + 1) * sizeof(OpTabs)));
 
     // job templates
     std::vector<LimbJob> jq(np);
@@ -345,7 +349,7 @@ int build_native_tables(afhe_ctx* ctx) {
         jq[i] = j;
     }
     CK(dalloc(&ctx->jobs_qp, np));
-    CK(cudaMemcpy(ctx->jobs_qp, jq.data(), np * sizeof(LimbJob), cudaMemcpyHostToDevice));
+    CK(upload(ctx, ctx->jobs_qp, jq.data(), np * sizeof(LimbJob)));
     ctx->lvjobs.assign(L + 1, LevelJobs{});
     const u64 S = (u64)L + K;
     for (uint32_t lvl = 1; lvl <= L; ++lvl) {
@@ -370,8 +374,9 @@ int build_native_tables(afhe_ctx* ctx) {
         LevelJobs& lj = ctx->lvjobs[lvl];
         lj.n_modup = (uint32_t)jm.size();
         CK(dalloc(&lj.modup, jm.size()));
-        CK(cudaMemcpy(lj.modup, jm.data(), jm.size() * sizeof(LimbJob), cudaMemcpyHostToDevice));
+        CK(upload(ctx, lj.modup, jm.data(), jm.size() * sizeof(LimbJob)));
     }
+    CK(cudaStreamSynchronize(ctx->st));
     return AFHE_OK;
 }
 
@@ -439,8 +444,8 @@ int afhe_ctx_create(const afhe_params* prm, afhe_ctx** out) {
         ctx->scr = ctx->poly + prm->poly_words;
         e = dalloc(&ctx->key, prm->key_words);
         if (e != cudaSuccess) { rc = cuda_fail(ctx, e, "alloc key_gmem"); break; }
-        e = cudaMemset(ctx->poly, 0, (prm->poly_words + ctx->scr_words) * 8);
-        if (e == cudaSuccess) e = cudaMemset(ctx->key, 0, std::max<u64>(prm->key_words, 1) * 8);
+        e = cudaMemsetAsync(ctx->poly, 0, (prm->poly_words + ctx->scr_words) * 8, ctx->st);
+        if (e == cudaSuccess) e = cudaMemsetAsync(ctx->key, 0, std::max<u64>(prm->key_words, 1) * 8, ctx->st);
         if (e != cudaSuccess) { rc = cuda_fail(ctx, e, "clear arenas"); break; }
         rc = build_native_tables(ctx);
         if (rc != AFHE_OK) break;

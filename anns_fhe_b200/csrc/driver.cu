@@ -73,7 +73,7 @@ int cached_map(afhe_ctx* ctx, uint32_t galois, const uint32_t** out) {
     automorphism_map(ctx->log_n, galois, map.data());
     uint32_t* d = nullptr;
     CK(cudaMalloc(&d, (size_t)ctx->n * sizeof(uint32_t)));
-    cudaError_t e = cudaMemcpy(d, map.data(), (size_t)ctx->n * sizeof(uint32_t), cudaMemcpyHostToDevice);
+    cudaError_t e = upload(ctx, d, map.data(), (size_t)ctx->n * sizeof(uint32_t));
     if (e != cudaSuccess) {
         cudaFree(d);
         return cuda_fail(ctx, e, "automorphism map upload");
@@ -440,7 +440,7 @@ int afhe_add_rotation_key(afhe_ctx* ctx, int32_t step, uint64_t evk) {
     } else {
         CK(cudaMalloc((void**)&rk.map, ctx->n * sizeof(uint32_t)));
     }
-    CK(cudaMemcpy(rk.map, map.data(), ctx->n * sizeof(uint32_t), cudaMemcpyHostToDevice));
+    CK(upload(ctx, rk.map, map.data(), ctx->n * sizeof(uint32_t)));
     rc = prep_key(ctx, evk, &rk.prep);
     ctx->rot[step] = rk;
     return rc;

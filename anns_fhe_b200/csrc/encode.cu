@@ -540,11 +540,11 @@ int afhe_pq_create(afhe_ctx* ctx, const afhe_pq_index* ix, afhe_pq** out) {
     if (e == cudaSuccess) e = cudaMalloc(&p->codebooks, bbytes);
     if (e == cudaSuccess) e = cudaMalloc(&p->codes, ix->n * ix->M + 1);
     if (e == cudaSuccess) e = cudaMalloc(&p->assign, ix->n * sizeof(uint32_t) + 4);
-    if (e == cudaSuccess) e = cudaMemcpy(p->centroids, ix->centroids, cbytes, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemcpy(p->codebooks, ix->codebooks, bbytes, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess && ix->n) e = cudaMemcpy(p->codes, ix->codes, ix->n * ix->M, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess && ix->n)
-        e = cudaMemcpy(p->assign, ix->assignments, ix->n * sizeof(uint32_t), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = upload(ctx, p->centroids, ix->centroids, cbytes);
+    if (e == cudaSuccess) e = upload(ctx, p->codebooks, ix->codebooks, bbytes);
+    if (e == cudaSuccess) e = upload(ctx, p->codes, ix->codes, ix->n * ix->M);
+    if (e == cudaSuccess) e = upload(ctx, p->assign, ix->assignments, ix->n * sizeof(uint32_t));
+    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->st);    // (the caller's arrays may be pinned)
     if (e != cudaSuccess) {
         afhe_pq_destroy(p);
         return cuda_fail(ctx, e, "index upload");
@@ -624,9 +624,10 @@ int pq_encode(afhe_pq* p, const uint32_t* vids, const uint32_t* first, const uin
     if (e == cudaSuccess) e = cudaMalloc(&vids_d, (total + 1) * sizeof(uint32_t));
     if (e == cudaSuccess) e = cudaMalloc(&first_d, ((size_t)batches + 1) * sizeof(uint32_t));
     if (e == cudaSuccess) e = cudaMalloc(&cnt_d, ((size_t)batches + 1) * sizeof(uint32_t));
-    if (e == cudaSuccess && total) e = cudaMemcpy(vids_d, ids.data(), total * sizeof(uint32_t), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess && batches) e = cudaMemcpy(first_d, first, batches * sizeof(uint32_t), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess && batches) e = cudaMemcpy(cnt_d, cnt, batches * sizeof(uint32_t), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = upload(ctx, vids_d, ids.data(), total * sizeof(uint32_t));
+    if (e == cudaSuccess) e = upload(ctx, first_d, first, batches * sizeof(uint32_t));
+    if (e == cudaSuccess) e = upload(ctx, cnt_d, cnt, batches * sizeof(uint32_t));
+    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->st);    // (the caller's arrays may be pinned)
     if (e != cudaSuccess) {
         release();
         return cuda_fail(ctx, e, "batch upload");

@@ -15,6 +15,12 @@ extern thread_local std::string g_last_error;
 int fail(afhe_ctx* ctx, int code, const std::string& msg);
 int cuda_fail(afhe_ctx* ctx, cudaError_t e, const char* where);
 u64 host_shoup(u64 w, u64 q);
+// Copy host memory to the device on the context's stream, where what
+// reads it is launched: the stream is non-blocking, so nothing on it waits for a
+// copy on the legacy stream, which may return before its data has arrived.
+// Pageable sources have been staged on return; a source that may be pinned needs
+// the stream waited for.
+cudaError_t upload(afhe_ctx* ctx, void* dst, const void* src, size_t bytes);
 // Re-derive the prepared copies of registered keys that overlap key words
 // [off, off + count) after they were overwritten (driver.cu).
 int refresh_key_preps(afhe_ctx* ctx, u64 off, u64 count);
