@@ -1062,9 +1062,11 @@ int afhe_eval_diag_inner_batch(afhe_ctx* ctx, const afhe_ct_ref* out, uint32_t c
     const unsigned __int128 room = ~(unsigned __int128)0 / (sq ? sq : 1);
     const uint32_t reduce_every = room > 0x7fffffff ? 0x7fffffffu : (uint32_t)room;
     if (reduce_every < nb + 1) return fail(ctx, AFHE_E_ARG, "primes too large for the accumulators; use afhe_eval_mac_plain_batch");
-    // the shared-memory form: tiles of 256 words stay put under every map,
-    // 16-byte aligned plaintext tiles
+    // the shared-memory form: tiles of 256 words stay put under every map, and
+    // the plaintexts' and the baby steps' tiles, which come in 16-byte copies,
+    // are 16-byte aligned
     bool staged = ctx->n % 256 == 0 && pt_stride % 2 == 0;
+    for (u64 k = 0; k < (u64)count * nb && staged; ++k) staged = (src[k].c0_offset | src[k].c1_offset) % 2 == 0;
     for (uint32_t j = 0; j < count && staged; ++j)
         for (uint32_t k = first_unit[j]; k < first_unit[j + 1] && staged; ++k) {
             const uint32_t* map = nullptr;

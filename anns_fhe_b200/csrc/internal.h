@@ -203,7 +203,7 @@ struct MacTerm {
 // in `add` (the giant step). Neighbouring jobs run side by side on the same
 // coefficients.
 // staged: every map keeps 256-word tiles within themselves, every plaintext
-// offset and the stride are even and N is a multiple of 256 (the
+// and source offset and the stride are even and N is a multiple of 256 (the
 // shared-memory form); halves: every prime is below 2^50 (25-bit split
 // products).
 struct DiagJob {

@@ -1,0 +1,62 @@
+"""Operands of afhe_eval_diag_inner_batch that its shared-memory form does not take.
+
+Where a source polynomial starts at an odd word, its 16-byte copies would not be
+aligned: the call takes the form that reads word by word. One odd polynomial
+among even ones, first, last and in the middle, c0 or c1; equal word for word
+to afhe_eval_mac_plain_batch.
+"""
+import numpy as np
+import pytest
+
+from anns_fhe_b200 import _lib as L
+from anns_fhe_b200.driver import CkksParams, FheContext, galois_elt
+from tests.helpers import primes_for, uniform_residues
+from tests.test_gpu_mac_plain import call
+
+pytestmark = pytest.mark.gpu
+
+LOG_N, LIMBS = 11, 2
+
+
+def diag(ctx, outs, srcs, nb, units, gals, stride, limbs, accumulate=0):
+    """One call: outs[j] from sources srcs[j] (nb of them) and units[j] (plaintext offsets)."""
+    oa = (L.CtRef * len(outs))(*[L.CtRef(*c) for c in outs])
+    src = (L.CtRef * (len(outs) * nb))(*[L.CtRef(*c) for s in srcs for c in s])
+    upt = np.array([u for us in units for u in us] or [0], dtype=np.uint64)
+    ugal = np.array([gals[k % len(gals)] for us in units for k in range(len(us))] or [1], dtype=np.uint32)
+    first = np.concatenate([[0], np.cumsum([len(us) for us in units])]).astype(np.uint32)
+    return ctx.lib.afhe_eval_diag_inner_batch(ctx.h, oa, len(outs), src, nb, upt.ctypes.data_as(L.P64),
+                                              ugal.ctypes.data_as(L.P32), first.ctypes.data_as(L.P32), stride, limbs,
+                                              accumulate)
+
+
+@pytest.mark.parametrize("nb,q_bits", [(1, 50), (4, 50), (16, 50), (2, 60), (16, 60)])
+@pytest.mark.parametrize("which", ["c0 of the first", "c1 of the last", "c0 in the middle"])
+def test_sources_at_odd_words(nb, q_bits, which):
+    q, p = primes_for(LOG_N, LIMBS, q_bits, 1, 61 if q_bits == 60 else 60)
+    n = 1 << LOG_N
+    w = LIMBS * n
+    ctx = FheContext(CkksParams(LOG_N, q, p, 1), poly_words=160 * w, key_words=1024)
+    try:
+        rng = np.random.default_rng([nb, q_bits])
+        srcs = [[(2 * b * w, (2 * b + 1) * w) for b in range(nb)] for _ in range(2)]
+        j, b = {"c0 of the first": (0, 0), "c1 of the last": (1, nb - 1), "c0 in the middle": (1, nb // 2)}[which]
+        odd = 40 * w + 1
+        srcs[j][b] = (srcs[j][b][0], odd) if which.startswith("c1") else (odd, srcs[j][b][1])
+        for at in {o for s in srcs for c in s for o in c}:
+            ctx.write_poly(at, uniform_residues(rng, q, n))
+        for k in range(48, 48 + 4 * nb):
+            ctx.write_poly(k * w, uniform_residues(rng, q, n))
+        gals = [1, galois_elt(LOG_N, -64), galois_elt(LOG_N, -256)]
+        units = [[(48 + nb * k) * w for k in range(3)], [(48 + nb * k) * w for k in range(1, 4)]]
+        outs = [((120 + 2 * j) * w, (121 + 2 * j) * w) for j in range(2)]
+        outs_b = [((130 + 2 * j) * w, (131 + 2 * j) * w) for j in range(2)]
+        assert diag(ctx, outs, srcs, nb, units, gals, w, LIMBS) == L.OK, ctx.lib.afhe_last_error()
+        mac = [[(srcs[j][b], [(u + b * w, gals[k]) for k, u in enumerate(units[j])]) for b in range(nb)]
+               for j in range(2)]
+        assert call(ctx, outs_b, mac, LIMBS) == L.OK, ctx.lib.afhe_last_error()
+        for a, b in zip(outs, outs_b):
+            assert np.array_equal(ctx.read_poly(a[0], w), ctx.read_poly(b[0], w))
+            assert np.array_equal(ctx.read_poly(a[1], w), ctx.read_poly(b[1], w))
+    finally:
+        ctx.close()
