@@ -168,7 +168,7 @@ __device__ __forceinline__ void fwd_rounds(u64* const (&bufs)[NB], const TwRow& 
     typedef Rounds<false, LOGQ> R;
     if constexpr (I < R::NR - 1) {
         KsRound<A, false, LOGQ, R::rb(I), R::k(I), G::LOGN>::R::template run_n<NB>(bufs, tw, c, nullptr, G::rank(),
-                                                                                    I > 0 || LOGCL > 0, false);
+                                                                                    I > 0 || LOGCL > 0 ? kEarlier : kResidues, false);
         sync_round<R::rb(I), G::T>();
         fwd_rounds<A, LOGQ, LOGCL, NB, I + 1>(bufs, tw, c);
     }
@@ -183,7 +183,7 @@ __device__ __forceinline__ void inv_rounds(u64* const (&bufs)[NB], const TwRow& 
     typedef Rounds<true, LOGQ> R;
     if constexpr (I < R::NR) {
         sync_round<R::rb(I), G::T>();
-        KsRound<A, true, LOGQ, R::rb(I), R::k(I), G::LOGN>::R::template run_n<NB>(bufs, tw, c, fin, G::rank(), true,
+        KsRound<A, true, LOGQ, R::rb(I), R::k(I), G::LOGN>::R::template run_n<NB>(bufs, tw, c, fin, G::rank(), kEarlier,
                                                                                 LOGCL == 0 && I == R::NR - 1);
         inv_rounds<A, LOGQ, LOGCL, NB, I + 1>(bufs, tw, c, fin);
     }
@@ -238,7 +238,7 @@ __device__ __forceinline__ void fwd_enter(typename A::V* v, uint32_t g, u64* W, 
         const uint32_t base = smem_u32(W);
 #pragma unroll
         for (uint32_t q = 0; q < 8 / G::CL; ++q) {
-            fwd_stages<A, LOGCL>(v + q * G::CL, cross, c, false);
+            fwd_stages<A, LOGCL>(v + q * G::CL, cross, c, kResidues);
             const uint32_t at = 8 * padix(G::column(8 * g + q * G::CL));
 #pragma unroll
             for (uint32_t k = 0; k < G::CL; ++k) st_cluster(map_rank(base, k) + at, A::store(v[q * G::CL + k]));
@@ -296,7 +296,7 @@ __device__ __forceinline__ void fwd_last(typename A::V* v, uint32_t g, const u64
     const u64* const sp = W + padix(gr.base_e);
 #pragma unroll
     for (uint32_t j = 0; j < 8; ++j) v[j] = A::load(sp[j]);
-    R::run_regs(v, tw, gr.blk, c, nullptr, true, false);
+    R::run_regs(v, tw, gr.blk, c, nullptr, kEarlier, false);
 }
 // The first inverse round on eight adjacent values, stored to buf.
 template <class A, int LOGQ, int LOGCL>
@@ -305,7 +305,7 @@ __device__ __forceinline__ void inv_first(typename A::V* v, uint32_t g, u64* buf
     using G = Geo<LOGQ, LOGCL>;
     typedef typename KsRound<A, true, LOGQ, 0, 3, G::LOGN>::R R;
     const typename R::Group gr = R::group(g, G::rank());
-    R::run_regs(v, tw, gr.blk, c, nullptr, true, false);
+    R::run_regs(v, tw, gr.blk, c, nullptr, kEarlier, false);
     u64* const sp = buf + padix(gr.base_e);
 #pragma unroll
     for (uint32_t j = 0; j < 8; ++j) sp[j] = A::store(v[j]);
@@ -554,6 +554,7 @@ __device__ AFHE_KS_FN void input_limb(const Slot<LOGQ, LOGCL, SINGLE> S, uint32_
         for (uint32_t e = 0; e < kE; ++e) g[e] = gpos(map, G::rank() * G::QN + (uint32_t)G::lpos(e));
 #pragma unroll
         for (uint32_t e = 0; e < kE; ++e) x[e] = src[g[e]];
+        residues<kE, A::kSecond>(x, S.pt()->pc[i]);
 #pragma unroll
         for (uint32_t e = 0; e < kE; ++e) buf[G::spos(e)] = A::store(A::of(x[e]));
     }
@@ -630,10 +631,9 @@ __device__ __forceinline__ void special_slot(const Slot<LOGQ, LOGCL, SINGLE>& S,
 
 // The ModDown combine at one position: (sum - y) P^-1, plus acc, canonical.
 __device__ __forceinline__ u64 moddown_value(double s, double y, const ulonglong2& pinv, const ulonglong2&,
-                                             const ArFp::C& c, bool has_acc, u64 acc, u64) {
-    double r = fp_mul(__dadd_rn(s, -y), as_double(pinv.x), as_double(pinv.y), c.q);
-    if (has_acc) r = fp_center(__dadd_rn(r, fp_of(acc)), c.q, c.qi);
-    return fp_canon(r, c.q);
+                                             const ArFp::C& c, bool has_acc, u64 acc, u64 q) {
+    const u64 r = fp_canon(fp_mul(__dadd_rn(s, -y), as_double(pinv.x), as_double(pinv.y), c.q), c.q);
+    return has_acc ? add_mod(r, acc, q) : r;
 }
 __device__ __forceinline__ u64 moddown_value(u64 s, u64 y, const ulonglong2& pinv, const ulonglong2& pinv2,
                                              const ArSp::C& c, bool has_acc, u64 acc, u64 q) {
@@ -647,7 +647,7 @@ __device__ __forceinline__ u64 moddown_value(u64 s, u64 y, const ulonglong2& pin
 // halves, c0 joining the first as c0 P (it comes out of the product with P^-1).
 // OwnGather reads input and c0 at lpos(e0) .. lpos(e0 + 7) through the
 // automorphism, own_products makes the products of four of them.
-template <int LOGQ, int LOGCL>
+template <class A, int LOGQ, int LOGCL>
 struct OwnGather {
     u64 d[8], cv[8];
     template <bool SINGLE>
@@ -664,6 +664,10 @@ struct OwnGather {
         for (uint32_t e = 0; e < 8; ++e) {
             d[e] = src[g[e]];
             cv[e] = a.f.has_c0 ? cb[g[e]] : 0;
+        }
+        if (!A::kSecond) {              // (split and 128-bit products take any word)
+            residues<8, false>(d, S.pt()->pc[i]);
+            residues<8, false>(cv, S.pt()->pc[i]);
         }
     }
 };
@@ -735,7 +739,7 @@ __device__ AFHE_KS_FN void own_sums(const Slot<LOGQ, LOGCL, false> S, uint32_t i
     const EntryKey ek = entry_key(S.a, S.z());
 #pragma unroll 1
     for (uint32_t e0 = 0; e0 < kE; e0 += 8) {
-        OwnGather<LOGQ, LOGCL> og;
+        OwnGather<A, LOGQ, LOGCL> og;
         og.load(S, ek, i, e0);
 #pragma unroll
         for (uint32_t f = 0; f < 8; f += 4) {
@@ -808,7 +812,7 @@ __device__ AFHE_KS_FN void combine_both(const Slot<LOGQ, LOGCL, true> S, uint32_
     const ulonglong2 pi0 = __ldg(pi), pi1 = A::kSecond ? __ldg(pi + 1) : ulonglong2{};
 #pragma unroll 1
     for (uint32_t e0 = 0; e0 < kE; e0 += 8) {
-        OwnGather<LOGQ, LOGCL> og;
+        OwnGather<A, LOGQ, LOGCL> og;
         og.load(S, ek, i, e0);
 #pragma unroll
         for (uint32_t f = 0; f < 8; f += 4) {

@@ -26,6 +26,7 @@ size_t ks_scratch_words(uint32_t n, uint32_t slots_q, uint32_t K, uint32_t parts
 // c1[map[x]] (the reference applies automorphism() first, fhe_host_driver.cpp:342-350).
 struct LoadGather {
     static constexpr bool kMany = false;
+    static constexpr bool kWords = true;
     const u64* base;
     const uint32_t* map;
     ZField mapz;        // per-entry map addresses (per_z)
@@ -55,6 +56,7 @@ struct StoreQhatInv {
 // y_i = [x_i * qHatInv_i]_{q_i} (StoreQhatInv) and sums y_i * [qHat_i]_p.
 struct ModUpLoad {
     static constexpr bool kMany = true;
+    static constexpr bool kWords = false;
     const u64* scratch;   // coef region at zb.aux[z]
     OpTabs t;
     uint32_t K;

@@ -21,6 +21,7 @@ struct StorePhatInv {
 // [x_k * PHatInv_k]_{p_k} (StorePhatInv) and sums it times [PHat_k]_{q_i}.
 struct ModDownLoad {
     static constexpr bool kMany = true;
+    static constexpr bool kWords = false;
     const u64* scratch;  // ext region at zb.aux[z]
     OpTabs t;
     uint32_t slots_q, K, n;
@@ -70,7 +71,7 @@ cudaError_t launch_ks_moddown(int log_n, const OpTabs& t, const LimbJob* jobs_qp
         a.mid = a.src;
         a.out = a.src;
         // 4a. INTT of the special limbs, in place, times PHatInv
-        cudaError_t e = launch_ntt<true>(log_n, t.pt, jobs_qp + slots_q, K, 2 * nz, scratch, a, LoadPlain{scratch},
+        cudaError_t e = launch_ntt<true>(log_n, t.pt, jobs_qp + slots_q, K, 2 * nz, scratch, a, LoadResidue{{scratch}},
                              StorePhatInv{scratch, t}, st);
         if (e != cudaSuccess) return e;
         // 4b. NTT over Q limbs with base-conversion prologue and ModDown epilogue

@@ -53,7 +53,7 @@ struct PrimeConst {
     u64 r64, r64_sh, one_sh;  // reduce128 constants
     u64 fp;                   // q < kFpLimit
     double qd, qi;            // q and 1/q as doubles (fp)
-    u64 pad;
+    u64 over;                 // the bits above q's own
     u64 nv[4], w1nv[4];       // ninv and w1ninv as transform constants
 };
 
@@ -98,7 +98,8 @@ AFHE_HD void set_transform_constants(PrimeConst& c) {
     c.fp = c.q < kFpLimit ? 1 : 0;
     c.qd = (double)c.q;
     c.qi = 1.0 / c.qd;
-    c.pad = 0;
+    c.over = ~0ull;
+    while (c.q & c.over) c.over <<= 1;
     transform_constant(c.ninv, c.q, c.nv);
     transform_constant(c.w1ninv, c.q, c.w1nv);
 }
@@ -185,14 +186,43 @@ struct ZBases {
     ZField src, mid, out, aux;
 };
 
-// Plain prologue / epilogue.
+// x mod q, any x
+__device__ __forceinline__ u64 residue(u64 x, const PrimeConst& pc) {
+    return x < pc.q ? x : csub(mul_shoup_lazy(x, 1, pc.one_sh, pc.q), pc.q);
+}
+// Words from outside as residues: one branch, rarely taken, behind all their
+// loads. Unless EXACT, words below the next power of two (so below 2q) stay as
+// they are.
+template <int M, bool EXACT>
+__device__ __forceinline__ void residues(u64* v, const PrimeConst& pc) {
+    u64 bits = 0;
+    bool words = false;
+#pragma unroll
+    for (int i = 0; i < M; ++i) {
+        if (EXACT) words |= v[i] >= pc.q;
+        else bits |= v[i];
+    }
+    if (EXACT ? words : (bits & pc.over) != 0) {
+#pragma unroll
+        for (int i = 0; i < M; ++i) v[i] = residue(v[i], pc);
+    }
+}
+
+// Plain prologues / epilogue. Words of outside (kWords) may be no residues: a
+// transform takes them below 4q forward and below 2q inverse, by its bounds alone
+// (checking the words before their use keeps loads and arithmetic apart, which
+// costs 13% of a forward transform at N = 2^16).
 struct LoadPlain {
     static constexpr bool kMany = false;      // one value a call
+    static constexpr bool kWords = true;
     const u64* base;
     __device__ __forceinline__ u64 operator()(const LimbJob& j, const ZBases& zb, uint32_t z, u64 x,
                                               const PrimeConst&) const {
         return base[zb.src.at(z) + j.src + x];
     }
+};
+struct LoadResidue : LoadPlain {
+    static constexpr bool kWords = false;
 };
 struct StorePlain {
     u64* base;
@@ -244,6 +274,10 @@ struct ArFp {
     static __device__ __forceinline__ V load(u64 bits) { return as_double(bits); }
     static __device__ __forceinline__ u64 store(V v) { return as_bits(v); }
     static __device__ __forceinline__ V of(u64 canonical) { return fp_of(canonical); }
+    // a word below 4q, less 2q
+    static __device__ __forceinline__ V outside(u64 word, const C& c) {
+        return __dadd_rn(as_double(word | 0x4330000000000000ull), -__fma_rn(2, c.q, 0x1p52));
+    }
     static __device__ __forceinline__ V mul(V a, const ulonglong2& w, const ulonglong2&, const C& c) {
         return fp_mul(a, as_double(w.x), as_double(w.y), c.q);
     }
@@ -371,6 +405,7 @@ struct ArSp {
     static __device__ __forceinline__ V load(u64 bits) { return bits; }
     static __device__ __forceinline__ u64 store(V v) { return v; }
     static __device__ __forceinline__ V of(u64 canonical) { return canonical; }
+    static __device__ __forceinline__ V outside(u64 word, const C&) { return word; }
     static __device__ __forceinline__ V mul(V a, const ulonglong2& w, const ulonglong2& s, const C& c) {
         return sp_mul(a, w.x, w.y, as_double(s.x), as_double(s.y), c.nq, c.start);
     }
@@ -388,10 +423,11 @@ struct ArSp {
 
 // K forward stages (bits high to low) on 2^K values: y = value 2^s apart times
 // its twiddle, (x + y, x - y). tw.first(s, m), tw.second(s, m): the constants of
-// twiddle m of stage s. center (ArFp): inputs may be up to 2.8 q (any earlier
-// round), else they are canonical.
+// twiddle m of stage s. from: what the inputs are: residues (below q (1 + 2^-6));
+// words below 4q (A::outside); values of an earlier round.
+enum Inputs { kResidues, kOutside, kEarlier };
 template <class A, int K, int NB = 1, class Tw>
-__device__ __forceinline__ void fwd_stages(typename A::V* v, const Tw& tw, const typename A::C& c, bool center) {
+__device__ __forceinline__ void fwd_stages(typename A::V* v, const Tw& tw, const typename A::C& c, Inputs from) {
     constexpr uint32_t NK = 1u << K;
     // the half that the first stage does not multiply
 #pragma unroll
@@ -400,10 +436,10 @@ __device__ __forceinline__ void fwd_stages(typename A::V* v, const Tw& tw, const
         for (uint32_t j = 0; j < NK / 2; ++j) {
             typename A::V& x = v[b * NK + j];
             if constexpr (A::kSecond) {
-                x = center ? A::low(x, c) : x + c.q;
+                x = from == kEarlier ? A::low(x, c) : from == kOutside ? A::low(x + c.q, c) : x + c.q;
             } else {
-                // the bound grows by less than 0.7 a stage: 1/2 (or 1) -> at most 2.8 after three
-                if (center) x = fp_center(x, c.q, c.qi);
+                // the bound grows by less than 0.75 a stage: 1/2 (1, 2) -> at most 2.8 (4) after three
+                if (from == kEarlier) x = fp_center(x, c.q, c.qi);
             }
         }
     }
@@ -433,7 +469,8 @@ __device__ __forceinline__ void fwd_stages(typename A::V* v, const Tw& tw, const
 }
 
 // K inverse stages (bits low to high): (x + y, (x - y) times the twiddle). Inputs
-// and outputs within 1 (canonical, products, reduced sums): the bounds are
+// and outputs within 1 (canonical, products, reduced sums; inputs from outside
+// within 2, which is as well within ArFp's exact range): the bounds are
 // tracked per value (they fold away when unrolled), and a sum is brought down
 // only where it could pass 2 before another stage of the round (ArSp: 4, by
 // 2q), or 1 at the end. last: the last stage multiplies its sums and
@@ -442,11 +479,11 @@ __device__ __forceinline__ void fwd_stages(typename A::V* v, const Tw& tw, const
 // the transform.
 template <class A, int K, int NB = 1, class Tw>
 __device__ __forceinline__ void inv_stages(typename A::V* v, const Tw& tw, const typename A::C& c, bool last,
-                                           const u64* fin_consts) {
+                                           const u64* fin_consts, Inputs from = kEarlier) {
     constexpr uint32_t NK = 1u << K;
     float bound[NK];
 #pragma unroll
-    for (uint32_t j = 0; j < NK; ++j) bound[j] = 1.0f;
+    for (uint32_t j = 0; j < NK; ++j) bound[j] = A::kSecond && from == kOutside ? 2.0f : 1.0f;
 #pragma unroll
     for (int s = 0; s < K; ++s) {
 #pragma unroll
@@ -600,32 +637,32 @@ struct NttRound {
 
     template <int NB, class W>
     __device__ __forceinline__ static void stages(V* v, const W& tw, const typename A::C& c, const u64* fin,
-                                                  bool center, bool last) {
-        if constexpr (INV) inv_stages<A, K, NB>(v, tw, c, last, fin);
-        else fwd_stages<A, K, NB>(v, tw, c, center);
+                                                  Inputs from, bool last) {
+        if constexpr (INV) inv_stages<A, K, NB>(v, tw, c, last, fin, from);
+        else fwd_stages<A, K, NB>(v, tw, c, from);
     }
 
     // NB sets of values in registers, twiddles from where they lie
     template <int NB = 1>
     __device__ __forceinline__ static void run_regs(V* v, const TwRow& row, uint32_t blk, const typename A::C& c,
-                                                    const u64* fin, bool center, bool last) {
+                                                    const u64* fin, Inputs from, bool last) {
         const Tw at(row, blk);
         if constexpr (A::kSecond) {
-            stages<NB>(v, at, c, fin, center, last);
+            stages<NB>(v, at, c, fin, from, last);
         } else {
             const TwHeld<K> held(at, INV && last);
-            stages<NB>(v, held, c, fin, center, last);
+            stages<NB>(v, held, c, fin, from, last);
         }
     }
 
     // The round over NB buffers of the same prime in shared memory: each
-    // group's twiddles and addresses serve every buffer. center: the values
-    // come from an earlier round (forward); last: the round holds the
+    // group's twiddles and addresses serve every buffer. from: where the values
+    // come from; last: the round holds the
     // transform's last stage (inverse), and the values are stored as canonical
     // residues.
     template <int NB>
     __device__ __forceinline__ static void run_n(u64* const (&sms)[NB], const TwRow& tw, const typename A::C& c,
-                                                 const u64* fin, uint32_t tile0, bool center, bool last) {
+                                                 const u64* fin, uint32_t tile0, Inputs from, bool last) {
 #pragma unroll(K == 3 ? 1 : GROUPS)      // (whole groups one after another: code size, registers)
         for (uint32_t gi = 0; gi < GROUPS; ++gi) {
             const Group g = group(gi, tile0);
@@ -637,7 +674,7 @@ struct NttRound {
             for (int b = 0; b < NB; ++b)
 #pragma unroll
                 for (uint32_t j = 0; j < NK; ++j) v[b * NK + j] = A::load(sms[b][padix(g.base_e) + padix(j * STEP_E)]);
-            run_regs<NB>(v, tw, g.blk, c, fin, center, last);
+            run_regs<NB>(v, tw, g.blk, c, fin, from, last);
 #pragma unroll
             for (int b = 0; b < NB; ++b)
 #pragma unroll
@@ -658,18 +695,18 @@ struct Rounds {
 };
 
 // Rounds [FROM, TO) of a pass over NB tiles in shared memory (same prime),
-// each followed by a barrier. center0: the first of the pass's rounds reads
-// values of an earlier pass (forward); finish: the pass ends the transform
+// each followed by a barrier. from0: what the first of the pass's rounds reads;
+// finish: the pass ends the transform
 // (inverse).
 template <class A, bool INV, int LOGN, int LO, int P, int LOGC, bool COL, int FROM, int TO, int EPT, int NB>
 __device__ __forceinline__ void ntt_rounds_n(u64* const (&sms)[NB], const TwRow& tw, const typename A::C& c,
-                                             const u64* fin, uint32_t tile0, bool center0, bool finish) {
+                                             const u64* fin, uint32_t tile0, Inputs from0, bool finish) {
     if constexpr (FROM < TO) {
         typedef Rounds<INV, P> R;
         NttRound<A, INV, LOGN, LO, P, LOGC, COL, R::rb(FROM), R::k(FROM), EPT>::template run_n<NB>(
-            sms, tw, c, fin, tile0, FROM > 0 || center0, finish && FROM == R::NR - 1);
+            sms, tw, c, fin, tile0, FROM > 0 ? kEarlier : from0, finish && FROM == R::NR - 1);
         __syncthreads();
-        ntt_rounds_n<A, INV, LOGN, LO, P, LOGC, COL, FROM + 1, TO, EPT, NB>(sms, tw, c, fin, tile0, center0, finish);
+        ntt_rounds_n<A, INV, LOGN, LO, P, LOGC, COL, FROM + 1, TO, EPT, NB>(sms, tw, c, fin, tile0, from0, finish);
     }
 }
 
@@ -696,6 +733,7 @@ __device__ __forceinline__ void ntt_pass(u64* sm, const PrimeTables& pt, const L
     constexpr bool TOP = LO + P == LOGN, first = INV ? LO == 0 : TOP, last = INV ? TOP : LO == 0;
     static_assert(NR >= 2, "a pass has a first and a last round");
     constexpr bool DIRECT_IN = COL || R::rb(0) > 0, DIRECT_OUT = COL || R::rb(NR - 1) > 0;
+    constexpr Inputs FROM = !first ? kEarlier : Pro::kWords ? kOutside : kResidues;
     const uint32_t z = blockIdx.z;
     u64* const mp = mid + zb.mid.at(z) + job.dst;
     PrimeConst pc = pt.pc[job.prime];
@@ -711,7 +749,10 @@ __device__ __forceinline__ void ntt_pass(u64* sm, const PrimeTables& pt, const L
         return ((u64)b << LO) + tile0 + col;
     };
     auto fetch = [&](u64 x) -> u64 {
-        if constexpr (first && !Pro::kMany) return A::store(A::of(pro(job, zb, z, x, pc)));
+        if constexpr (first && !Pro::kMany) {
+            const u64 w = pro(job, zb, z, x, pc);
+            return A::store(FROM == kOutside && !INV ? A::outside(w, c) : A::of(w));
+        }
         else return mp[x];
     };
     auto put = [&](u64 x, u64 v, bool canonical) {
@@ -739,7 +780,7 @@ __device__ __forceinline__ void ntt_pass(u64* sm, const PrimeTables& pt, const L
 #pragma unroll
                 for (uint32_t j = 0; j < Rd::NK; ++j) v[j] = A::load(fetch(x + j * Rd::STEP_X));
             }
-            Rd::run_regs(v, tw, gr.blk, c, fin, !first, false);
+            Rd::run_regs(v, tw, gr.blk, c, fin, FROM, false);
             u64* const sp = sm + padix(gr.base_e);
 #pragma unroll
             for (uint32_t j = 0; j < Rd::NK; ++j) sp[padix(j * Rd::STEP_E)] = A::store(v[j]);
@@ -754,7 +795,7 @@ __device__ __forceinline__ void ntt_pass(u64* sm, const PrimeTables& pt, const L
     }
     u64* const one[1] = {sm};
     ntt_rounds_n<A, INV, LOGN, LO, P, LOGC, COL, DIRECT_IN ? 1 : 0, DIRECT_OUT ? NR - 1 : NR, EPT, 1>(
-        one, tw, c, fin, tile0, !first, last);
+        one, tw, c, fin, tile0, FROM, last);
     if constexpr (DIRECT_OUT) {
         typedef NttRound<A, INV, LOGN, LO, P, LOGC, COL, R::rb(NR - 1), R::k(NR - 1), EPT> Rd;
 #pragma unroll
@@ -765,7 +806,7 @@ __device__ __forceinline__ void ntt_pass(u64* sm, const PrimeTables& pt, const L
             const u64* const sp = sm + padix(gr.base_e);
 #pragma unroll
             for (uint32_t j = 0; j < Rd::NK; ++j) v[j] = A::load(sp[padix(j * Rd::STEP_E)]);
-            Rd::run_regs(v, tw, gr.blk, c, fin, true, last);
+            Rd::run_regs(v, tw, gr.blk, c, fin, kEarlier, last);
 #pragma unroll
             for (uint32_t j = 0; j < Rd::NK; ++j)
                 put(x + j * Rd::STEP_X, (INV && last) ? A::canon_inv(v[j], c) : A::store(v[j]), INV && last);

@@ -17,6 +17,7 @@ namespace afhe {
 // below 2^62, which the split product takes as it is).
 struct RescaleLoad {
     static constexpr bool kMany = false;
+    static constexpr bool kWords = false;
     const u64* scratch;
     const u64* qlql;
     const PrimeConst* pc_last;   // q_l, the prime being dropped
@@ -48,6 +49,7 @@ struct RescaleStore {
 // formed where the transforms read it and written nowhere.
 struct LoadProduct {
     static constexpr bool kMany = false;
+    static constexpr bool kWords = false;
     const u64* arena;
     ZField pt;
     __device__ __forceinline__ u64 operator()(const LimbJob& j, const ZBases& zb, uint32_t z, u64 x,

@@ -15,6 +15,12 @@
  * afhe_status and never throws; work is queued on the context's CUDA stream
  * and ordered; afhe_sync() waits for it. One context is not safe to drive from
  * two host threads at once; separate contexts are independent.
+ *
+ * Limbs hold residues, words below their prime q; results are residues where the
+ * operands are. Other words are taken modulo q by products (any word), forward
+ * transforms (words below 4q), inverse transforms, rescales and key switches
+ * (below 2q); where words are only added or subtracted (a rotation's c0, an
+ * accumulated ciphertext too), a result may be no residue either.
  */
 #ifndef AFHE_H
 #define AFHE_H
