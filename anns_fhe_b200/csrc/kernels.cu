@@ -237,7 +237,7 @@ constexpr uint32_t kDiagTile = 256, kDiagUnits = 128;
 // in 64-bit registers by single 32 x 32 + 64 multiply-adds (products of
 // halves below 2^57: room for 32 of the middle ones, used for at most 16 of
 // them twice); recombined in 128 bits.
-constexpr uint32_t kHalfBits = 25, kHalfMask = (1u << kHalfBits) - 1;
+constexpr uint32_t kHalfBits = 25, kHalfMask = (1u << kHalfBits) - 1, kWordBits = 2 * kHalfBits;
 __device__ __forceinline__ void mad_wide(u64& acc, uint32_t a, uint32_t b) {
     asm("mad.wide.u32 %0, %1, %2, %0;" : "+l"(acc) : "r"(a), "r"(b));
 }
@@ -272,7 +272,10 @@ __device__ __forceinline__ u64 halves_reduce(const Halves& h, const ModConst& m)
 // neighbouring CTAs share their baby steps.
 // HALVES: primes below 2^50; sums of up to kDiagUnits residues are below 2^57, a
 // 25-bit half and a 32-bit one, and multiply as they are. Else the sums have
-// 96 bits and are reduced once. One coefficient per thread, tile t =
+// 96 bits and are reduced once. Words that are no residues: ANY looks at each and
+// reduces those from 2^50 on; without it (the shared-memory form, where that
+// look costs 10% of the kernel) plaintexts may be below 2^57 and baby steps
+// below 2^53. One coefficient per thread, tile t =
 // coefficients [256 t, 256 t + 256); groups vary fastest across the grid, so
 // consecutive CTAs are other groups of the same tile.
 template <int NB, bool HALVES>
@@ -285,36 +288,70 @@ struct DiagSums {
 #pragma unroll
         for (int b = 0; b < (HALVES ? 1 : NB); ++b) hi[b] = 0;
     }
+    // the array moves on by one, `first` to its end: a loop over it with one copy
+    // of its body and no more registers
+    __device__ __forceinline__ void turn(u64 first) {
+#pragma unroll
+        for (int c = 0; c + 1 < NB; ++c) p[c] = p[c + 1];
+        p[NB - 1] = first;
+    }
     // unit k's plaintexts, `stride` words apart
+    template <bool ANY>
     __device__ __forceinline__ void add(uint32_t k, const u64* t, u64 stride, const ModConst& m) {
+        uint32_t high = 0;
 #pragma unroll
         for (int b = 0; b < NB; ++b) {
             const u64 v = t[b * stride];
             p[b] += v;
+            if (HALVES && ANY) high |= (uint32_t)(v >> 32);
             if (!HALVES) hi[b] += p[b] < v ? 1u : 0u;
+        }
+        if (HALVES && ANY && high >> (kWordBits - 32)) {     // (words that are no residues)
+#pragma unroll 1
+            for (int b = 0; b < NB; ++b) {
+                const u64 v = t[b * stride];
+                turn(p[0] + reduce128(0, v, m) - v);
+            }
         }
         if (HALVES && k % (kDiagUnits - 1) == kDiagUnits - 2) {
 #pragma unroll 1
-            for (int b = 0; b < NB; ++b) {      // rotates through the array: one copy of the reduction
-                const u64 r = reduce128(0, p[0], m);
-#pragma unroll
-                for (int c = 0; c + 1 < NB; ++c) p[c] = p[c + 1];
-                p[NB - 1] = r;
-            }
+            for (int b = 0; b < NB; ++b) turn(reduce128(0, p[0], m));
         }
     }
     // after the last unit: residues, or their halves side by side
     __device__ __forceinline__ void close(const ModConst& m) {
+        if (HALVES) {
+            uint32_t high = 0;
+#pragma unroll
+            for (int b = 0; b < NB; ++b) high |= (uint32_t)(p[b] >> 32);
+            if (high >> kHalfBits) {                    // a sum from 2^57 on (words that are no residues)
+#pragma unroll 1
+                for (int b = 0; b < NB; ++b) turn(reduce128(0, p[0], m));
+            }
+        }
 #pragma unroll
         for (int b = 0; b < NB; ++b)
             p[b] = HALVES ? (p[b] >> kHalfBits << 32 | ((uint32_t)p[b] & kHalfMask)) : reduce128(hi[HALVES ? 0 : b], p[b], m);
     }
-    template <typename X>
-    __device__ __forceinline__ u64 times(X&& x, const ModConst& m) const {
+    template <bool ANY, typename X>
+    __device__ __forceinline__ u64 times(X&& x, const ModConst& m) {
         if (HALVES) {
             Halves c{0, 0, 0};
+            uint32_t high = 0;
 #pragma unroll
-            for (int b = 0; b < NB; ++b) halves_mad(c, (uint32_t)p[b], (uint32_t)(p[b] >> 32), x(b));
+            for (int b = 0; b < NB; ++b) {
+                const u64 v = x(b);
+                if (ANY) high |= (uint32_t)(v >> 32);
+                halves_mad(c, (uint32_t)p[b], (uint32_t)(p[b] >> 32), v);
+            }
+            if (ANY && high >> (kWordBits - 32)) {      // (words that are no residues)
+                c = Halves{0, 0, 0};
+#pragma unroll 1
+                for (int b = 0; b < NB; ++b) {
+                    halves_mad(c, (uint32_t)p[0], (uint32_t)(p[0] >> 32), reduce128(0, x(b), m));
+                    turn(p[0]);
+                }
+            }
             return halves_reduce(c, m);
         }
         Acc128 a;
@@ -341,7 +378,7 @@ __global__ void __launch_bounds__(kDiagTile) diag_inner_kernel(
     const DiagJob J = jobs[G.first];
     for (uint32_t k = J.u0; k < J.u1; ++k) {
         const DiagUnit U = units[k];
-        sums.add(k - J.u0, arena + U.pt + J.add + (U.map ? __ldg(U.map + i) : i), stride, m);
+        sums.template add<true>(k - J.u0, arena + U.pt + J.add + (U.map ? __ldg(U.map + i) : i), stride, m);
     }
     sums.close(m);
     for (uint32_t z = G.first; z < G.first + G.count; ++z) {
@@ -349,7 +386,7 @@ __global__ void __launch_bounds__(kDiagTile) diag_inner_kernel(
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             u64* out = arena + (h ? jobs[z].out1 : jobs[z].out0) + i;
-            const u64 r = sums.times([&](int b) { return arena[s[2 * b + h] + i]; }, m);
+            const u64 r = sums.template times<true>([&](int b) { return arena[s[2 * b + h] + i]; }, m);
             *out = accumulate ? add_mod(r, *out, m.q) : r;
         }
     }
@@ -429,7 +466,7 @@ __global__ void __launch_bounds__(kDiagTile, HALVES ? 3 : 2) diag_inner_staged_k
         } else {
             issue_baby(nu);
         }
-        sums.add(k, stage + (k & 1u) * NB * kDiagTile + j, kDiagTile, m);
+        sums.template add<false>(k, stage + (k & 1u) * NB * kDiagTile + j, kDiagTile, m);
         j = jn;
     }
     sums.close(m);
@@ -441,7 +478,7 @@ __global__ void __launch_bounds__(kDiagTile, HALVES ? 3 : 2) diag_inner_staged_k
         if (!(e & 1u) && z + 1 < G.first + G.count && tid < 2 * NB) from[~(e >> 1) & 1u][tid] = srcs[2ull * jobs[z + 1].s + tid];
         u64* out = arena + ((e & 1u) ? jobs[z].out1 : jobs[z].out0) + tid;
         const u64* t = stage + (k & 1u) * NB * kDiagTile + tid;
-        const u64 r = sums.times([&](int b) { return t[b * kDiagTile]; }, m);
+        const u64 r = sums.template times<false>([&](int b) { return t[b * kDiagTile]; }, m);
         *out = accumulate ? add_mod(r, *out, m.q) : r;
     }
 }

@@ -17,10 +17,11 @@
  * two host threads at once; separate contexts are independent.
  *
  * Limbs hold residues, words below their prime q; results are residues where the
- * operands are. Other words are taken modulo q by products (any word), forward
- * transforms (words below 4q), inverse transforms, rescales and key switches
- * (below 2q); where words are only added or subtracted (a rotation's c0, an
- * accumulated ciphertext too), a result may be no residue either.
+ * operands are. Other words are taken modulo q by products (any word; by
+ * afhe_eval_diag_inner_batch plaintexts below 2^57 and sources below 2^53),
+ * forward transforms (words below 4q), inverse transforms, rescales and key
+ * switches (below 2q); where words are only added or subtracted (a rotation's c0,
+ * an accumulated ciphertext too), a result may be no residue either.
  */
 #ifndef AFHE_H
 #define AFHE_H

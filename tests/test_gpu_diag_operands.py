@@ -1,9 +1,9 @@
-"""Operands of afhe_eval_diag_inner_batch that its shared-memory form does not take.
+"""Operands of afhe_eval_diag_inner_batch at the edges of its shared-memory form.
 
 Where a source polynomial starts at an odd word, its 16-byte copies would not be
 aligned: the call takes the form that reads word by word. One odd polynomial
 among even ones, first, last and in the middle, c0 or c1; equal word for word
-to afhe_eval_mac_plain_batch.
+to afhe_eval_mac_plain_batch. Words that are no residues, in either form.
 """
 import numpy as np
 import pytest
@@ -58,5 +58,54 @@ def test_sources_at_odd_words(nb, q_bits, which):
         for a, b in zip(outs, outs_b):
             assert np.array_equal(ctx.read_poly(a[0], w), ctx.read_poly(b[0], w))
             assert np.array_equal(ctx.read_poly(a[1], w), ctx.read_poly(b[1], w))
+    finally:
+        ctx.close()
+
+
+@pytest.mark.parametrize("nb", [1, 4, 16])
+@pytest.mark.parametrize("what", ["plaintexts", "sources", "both"])
+@pytest.mark.parametrize("local", [True, False])
+def test_words_that_are_no_residues(nb, what, local):
+    """Below 2^50 the products split words in halves: other words are taken modulo
+    their prime, any by the form for any placement, plaintexts below 2^57 and
+    sources below 2^53 by the shared-memory form."""
+    q = primes_for(LOG_N, LIMBS, 50, 1, 60)[0][:1] + primes_for(LOG_N, LIMBS, 36, 1, 60)[0][:1]
+    p = primes_for(LOG_N, LIMBS, 50, 1, 60)[1]
+    n = 1 << LOG_N
+    w = LIMBS * n
+    ctx = FheContext(CkksParams(LOG_N, q, p, 1), poly_words=200 * w, key_words=1024)
+    try:
+        rng = np.random.default_rng([nb, local])
+
+        def poly(words, most):
+            x = uniform_residues(rng, q, n)
+            y = x.copy()
+            if words:
+                y[::3] = rng.integers(0, most, y[::3].size, dtype=np.uint64)
+                y[1::7] = np.uint64(most - 1)
+                y[2::11] = np.uint64(2 ** 50)
+                y[5::13] = np.uint64(2 ** 50 - 1)
+                x = np.concatenate([y[l * n:(l + 1) * n] % np.uint64(q[l]) for l in range(LIMBS)])
+            return x, y
+
+        srcs = [[(2 * b * w, (2 * b + 1) * w) for b in range(nb)]]
+        gals = [1, galois_elt(LOG_N, -64), galois_elt(LOG_N, 128 if local else 5)]
+        units = [[(40 + nb * k) * w for k in range(5)]]
+        most = (1 << 53, 1 << 57) if local else (1 << 64, 1 << 64)
+        data = {k: poly(what != "plaintexts", most[0]) if k < 32 else poly(what != "sources", most[1])
+                for k in [*range(2 * nb), *range(40, 40 + 5 * nb)]}
+        got = []
+        for form in range(2):              # residues through the sums of products, then the words
+            for k, v in data.items():
+                ctx.write_poly(k * w, v[form])
+            out = [((150 + 2 * form) * w, (151 + 2 * form) * w)]
+            if form == 0:
+                mac = [[(srcs[0][b], [(u + b * w, gals[k % 3]) for k, u in enumerate(units[0])]) for b in range(nb)]]
+                assert call(ctx, out, mac, LIMBS) == L.OK, ctx.lib.afhe_last_error()
+            else:
+                assert diag(ctx, out, srcs, nb, units, gals, w, LIMBS) == L.OK, ctx.lib.afhe_last_error()
+            got.append([ctx.read_poly(o, w) for o in out[0]])
+        assert np.array_equal(got[0][0], got[1][0])
+        assert np.array_equal(got[0][1], got[1][1])
     finally:
         ctx.close()
