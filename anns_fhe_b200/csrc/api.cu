@@ -432,6 +432,7 @@ int afhe_ctx_create(const afhe_params* prm, afhe_ctx** out) {
             // value stands for that)
             int sms = 148;
             cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
+            ctx->sms = (uint32_t)std::max(1, sms);
             const int cl = ctx->log_n > 13 ? 1 << (ctx->log_n - 13) : 1;
             ctx->fused_min = ctx->fused_default = (uint32_t)std::max(1, sms / (2 * cl));
             const char* m = std::getenv("AFHE_FUSED_MIN");

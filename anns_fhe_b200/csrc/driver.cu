@@ -1058,14 +1058,11 @@ int afhe_eval_diag_inner_batch(afhe_ctx* ctx, const afhe_ct_ref* out, uint32_t c
     }
     u64 qmax = 0;
     for (uint32_t l = 0; l < limbs; ++l) qmax = std::max<u64>(qmax, ctx->prm.q[l]);
-    const unsigned __int128 sq = (unsigned __int128)(qmax - 1) * (qmax - 1);
-    const unsigned __int128 room = ~(unsigned __int128)0 / (sq ? sq : 1);
-    const uint32_t reduce_every = room > 0x7fffffff ? 0x7fffffffu : (uint32_t)room;
-    if (reduce_every < nb + 1) return fail(ctx, AFHE_E_ARG, "primes too large for the accumulators; use afhe_eval_mac_plain_batch");
     // the shared-memory form: tiles of 256 words stay put under every map, and
     // the plaintexts' and the baby steps' tiles, which come in 16-byte copies,
     // are 16-byte aligned
-    bool staged = ctx->n % 256 == 0 && pt_stride % 2 == 0;
+    const bool halves = qmax < (1ull << 50);
+    bool staged = halves && nb >= 8 && ctx->n % 256 == 0 && pt_stride % 2 == 0;
     for (u64 k = 0; k < (u64)count * nb && staged; ++k) staged = (src[k].c0_offset | src[k].c1_offset) % 2 == 0;
     for (uint32_t j = 0; j < count && staged; ++j)
         for (uint32_t k = first_unit[j]; k < first_unit[j + 1] && staged; ++k) {
@@ -1089,26 +1086,45 @@ int afhe_eval_diag_inner_batch(afhe_ctx* ctx, const afhe_ct_ref* out, uint32_t c
     };
     const size_t seg = ctx->ring.seg_words - 96;
     const u64 tiles = (u64)limbs * ((ctx->n + 255) / 256);
+    constexpr size_t jw = sizeof(DiagJob) / sizeof(u64);
+    std::vector<u64> D;
     std::vector<DiagJob> J;
     std::vector<uint32_t> step;             // output's place in its run
     std::vector<u64> S;
     std::vector<DiagUnit> U;
-    std::multimap<u64, std::pair<uint32_t, uint32_t>> lists;    // hash of a run's units -> their [u0, u1) in U
+    // the runs' units, [u0, u1) in U, by their hash (open addressing; twice as
+    // many places as outputs)
+    struct List {
+        u64 hash;
+        uint32_t u0, u1;
+    };
+    std::vector<List> lists;
+    const size_t outputs = std::min<size_t>(count, seg / (jw + 1));      // of one launch, at most
+    size_t places = 4;
+    while (places < 2 * outputs) places *= 2;
+    std::vector<uint32_t> place(places, 0);                             // a list's number + 1
+    J.reserve(outputs);
+    step.reserve(outputs);
+    S.reserve(std::min<size_t>((size_t)count * 2 * nb, seg));
+    U.reserve(std::min<size_t>(count ? first_unit[count] - first_unit[0] : 0, seg / 2) + 1);
     auto flush = [&]() -> int {
         if (J.empty()) return AFHE_OK;
         // Outputs at the same place of their runs side by side: a run's
         // sources stay in L2 from one place to the next. Among them those
         // with the same plaintexts (queries that scan the same list) form
         // groups, whose plaintexts are read and added up once; a group ends
-        // where larger ones would leave too few blocks (4 an SM).
+        // where larger ones would leave too few blocks (four an SM).
         std::vector<uint32_t> by(J.size());
         for (uint32_t i = 0; i < by.size(); ++i) by[i] = i;
-        std::stable_sort(by.begin(), by.end(), [&](uint32_t x, uint32_t y) {
+        auto before = [&](uint32_t x, uint32_t y) {
             return std::tie(step[x], J[x].u0, J[x].add) < std::tie(step[y], J[y].u0, J[y].add);
-        });
-        const u64 most = std::max<u64>(1, J.size() * tiles / (4 * 148));
+        };
+        if (!std::is_sorted(by.begin(), by.end(), before)) std::stable_sort(by.begin(), by.end(), before);
+        const u64 most = std::max<u64>(1, J.size() * tiles / (4 * ctx->sms));
         std::vector<DiagJob> ordered;
         std::vector<DiagGroup> G;
+        ordered.reserve(J.size());
+        G.reserve(J.size());
         for (uint32_t i : by) {
             const DiagJob& p = J[i];
             if (G.empty() || G.back().count >= most || ordered.back().u0 != p.u0 || ordered.back().u1 != p.u1 ||
@@ -1117,28 +1133,49 @@ int afhe_eval_diag_inner_batch(afhe_ctx* ctx, const afhe_ct_ref* out, uint32_t c
             ++G.back().count;
             ordered.push_back(p);
         }
-        u64 *dg = nullptr, *dj = nullptr, *ds = nullptr, *du = nullptr;
-        int r;
+        // Which form (N = 2^15, two limbs, 64 outputs; microseconds). Up to three
+        // units and no plaintexts shared, or one unit: reading straight through
+        // (60 bits, 8 baby steps, one unit: 146, through sums 209; two: 171 / 234; 50
+        // bits, 4, one: 97 / 123; one shared, 16: 264 / 342), unless the
+        // shared-memory form is open (50 bits, 16, one: 229, straight 288; 8, one:
+        // 161 / 150, two: 193 / 197). That form is for primes below 2^50 and eight
+        // baby steps or more; elsewhere the one for any placement is as fast or
+        // faster (50 bits, 4 baby steps, four units: 180 / 212; 8: 262 / 249; 16: 520
+        // / 318; 60 bits, 16: 557 / 581).
+        uint32_t few = ordered[0].u1 - ordered[0].u0;
+        for (const DiagJob& j : ordered)
+            if (j.u1 - j.u0 != few) few = 0;
+        if (few > 3 || (staged && !(nb == 8 && few == 1)) || (few > 1 && G.size() < ordered.size())) few = 0;
+        const uint32_t blocks = (uint32_t)(few ? ordered.size() : G.size());
         if (U.empty()) U.push_back(DiagUnit{0, nullptr});
-        if ((r = ring_put(ctx, G.data(), G.size() * sizeof(DiagGroup) / sizeof(u64), &dg))) return r;
-        if ((r = ring_put(ctx, ordered.data(), J.size() * sizeof(DiagJob) / sizeof(u64), &dj))) return r;
-        if ((r = ring_put(ctx, S.data(), S.size(), &ds))) return r;
-        if ((r = ring_put(ctx, U.data(), U.size() * sizeof(DiagUnit) / sizeof(u64), &du))) return r;
-        CK(launch_diag_inner(ctx->nat.pc, ctx->poly, ctx->n, limbs, (uint32_t)G.size(), nb, (const DiagGroup*)dg,
-                             (const DiagJob*)dj, ds, (const DiagUnit*)du, pt_stride, accumulate ? 1 : 0, staged,
-                             qmax < (1ull << 50), ctx->st));
+        // one copy to the device: groups, outputs, sources, units
+        D.clear();
+        D.reserve(J.size() * (jw + 1) + S.size() + 2 * U.size());
+        auto put = [&](const void* v, size_t words) {
+            const size_t at = D.size();
+            D.insert(D.end(), (const u64*)v, (const u64*)v + words);
+            return at;
+        };
+        const size_t ag = put(G.data(), G.size() * sizeof(DiagGroup) / sizeof(u64)), aj = put(ordered.data(), ordered.size() * jw),
+                     as = put(S.data(), S.size()), au = put(U.data(), U.size() * sizeof(DiagUnit) / sizeof(u64));
+        u64* d = nullptr;
+        int r;
+        if ((r = ring_put(ctx, D.data(), D.size(), &d))) return r;
+        CK(launch_diag_inner(ctx->nat.pc, ctx->poly, ctx->n, limbs, blocks, nb, (const DiagGroup*)(d + ag),
+                             (const DiagJob*)(d + aj), d + as, (const DiagUnit*)(d + au), pt_stride, accumulate ? 1 : 0,
+                             staged, halves, few, ctx->st));
         J.clear();
         step.clear();
         S.clear();
         U.clear();
         lists.clear();
+        std::fill(place.begin(), place.end(), 0u);
         return AFHE_OK;
     };
-    constexpr size_t jw = sizeof(DiagJob) / sizeof(u64);
     for (uint32_t j = 0; j < count; ++j) {
         const size_t nu = first_unit[j + 1] - first_unit[j];
-        if (jw + 2 * nb + 2 * nu + 2 > seg) return fail(ctx, AFHE_E_ARG, "too many units in one output for the descriptor ring");
-        if ((J.size() + 1) * jw > seg || S.size() + 2 * nb > seg || (U.size() + nu + 1) * 2 > seg)
+        if (3 + 2 * nb + 2 * nu + 2 > seg / 3) return fail(ctx, AFHE_E_ARG, "too many units in one output for the descriptor ring");
+        if ((J.size() + 1) * (jw + 1) + S.size() + 2 * nb + (U.size() + nu + 1) * 2 > seg)
             if ((rc = flush())) return rc;
         if (!J.empty() && follows(j)) {
             DiagJob n = J.back();
@@ -1158,19 +1195,22 @@ int afhe_eval_diag_inner_batch(afhe_ctx* ctx, const afhe_ct_ref* out, uint32_t c
         }
         // a run's units that an earlier run has too are kept once
         uint32_t u1 = (uint32_t)U.size(), u0 = u1 - (uint32_t)nu;
-        bool found = false;
-        for (auto it = lists.lower_bound(hash); it != lists.end() && it->first == hash && !found; ++it) {
-            const uint32_t a = it->second.first;
-            found = it->second.second - a == nu && std::equal(U.begin() + u0, U.end(), U.begin() + a, [](const DiagUnit& x, const DiagUnit& y) {
-                return x.pt == y.pt && x.map == y.map;
-            });
-            if (found) {
+        for (size_t at = hash >> 32 & (places - 1);; at = (at + 1) & (places - 1)) {
+            if (!place[at]) {
+                lists.push_back(List{hash, u0, u1});
+                place[at] = (uint32_t)lists.size();
+                break;
+            }
+            const List& t = lists[place[at] - 1];
+            if (t.hash == hash && t.u1 - t.u0 == nu &&
+                std::equal(U.begin() + u0, U.end(), U.begin() + t.u0,
+                           [](const DiagUnit& x, const DiagUnit& y) { return x.pt == y.pt && x.map == y.map; })) {
                 U.resize(u0);
-                u0 = a;
-                u1 = a + (uint32_t)nu;
+                u0 = t.u0;
+                u1 = t.u1;
+                break;
             }
         }
-        if (!found) lists.insert({hash, {u0, u1}});
         J.push_back(DiagJob{out[j].c0_offset, out[j].c1_offset, 0, u0, u1, (uint32_t)(S.size() / 2), 0});
         step.push_back(0);
         for (uint32_t b = 0; b < nb; ++b) {

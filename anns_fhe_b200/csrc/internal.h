@@ -85,6 +85,7 @@ struct afhe_ctx {
     int log_n;
     uint32_t n, L, K, alpha, dnum;
     int device;
+    uint32_t sms = 148;      // multiprocessors of the device
     cudaStream_t st = nullptr;
     afhe::u64* poly = nullptr;
     afhe::u64* key = nullptr;
@@ -202,10 +203,11 @@ struct MacTerm {
 // srcs[2 (s + b)]. Jobs of one result share their units and sources and differ
 // in `add` (the giant step). Neighbouring jobs run side by side on the same
 // coefficients.
-// staged: every map keeps 256-word tiles within themselves, every plaintext
-// and source offset and the stride are even and N is a multiple of 256 (the
-// shared-memory form); halves: every prime is below 2^50 (25-bit split
-// products).
+// staged (the shared-memory form; halves, nb 8 or 16): every map keeps 256-word
+// tiles within themselves, every plaintext and source offset and the stride are
+// even and N is a multiple of 256; halves: every prime is below 2^50 (25-bit
+// split products); few: 1, 2 or 3 where every group is one output of that many
+// units, to be read straight through, else 0.
 struct DiagJob {
     u64 out0, out1;
     u64 add;
@@ -222,7 +224,7 @@ struct DiagGroup {
 };
 cudaError_t launch_diag_inner(const PrimeConst* pc, u64* arena, uint32_t n, uint32_t limbs, uint32_t groups,
                               uint32_t nb, const DiagGroup* group, const DiagJob* job, const u64* srcs,
-                              const DiagUnit* unit, u64 stride, int accumulate, bool staged, bool halves,
+                              const DiagUnit* unit, u64 stride, int accumulate, bool staged, bool halves, uint32_t few,
                               cudaStream_t st);
 cudaError_t launch_mac_plain(const PrimeConst* pc, u64* arena, uint32_t n, uint32_t limbs, uint32_t jobs,
                              const MacJob* job, const MacGroup* group, const MacTerm* term, uint32_t reduce_every,

@@ -392,8 +392,8 @@ __global__ void __launch_bounds__(kDiagTile) diag_inner_kernel(
     }
 }
 
-// Every placement map of the launch keeps each 256-coefficient tile within
-// itself (a slot rotation by a multiple of D permutes the evaluation form
+// Primes below 2^50, eight baby steps or more, and every placement map of the
+// launch keeps each 256-coefficient tile within itself (a slot rotation by a multiple of D permutes the evaluation form
 // inside blocks of N / 2D words): tiles of nb rows, a unit's plaintexts or one
 // half of an output's baby steps, come by cp.async into one of two buffers
 // while the other is worked on. 64 KB a CTA at nb = 16, three on an SM.
@@ -403,8 +403,8 @@ __global__ void __launch_bounds__(kDiagTile) diag_inner_kernel(
 // slower: four buffers of eight rows (3.7 ms: the instructions of a deeper
 // ring), the products with a baby step for each unit in double precision
 // (9.0 ms).
-template <int NB, bool HALVES>
-__global__ void __launch_bounds__(kDiagTile, HALVES ? 3 : 2) diag_inner_staged_kernel(
+template <int NB>
+__global__ void __launch_bounds__(kDiagTile, 3) diag_inner_staged_kernel(
     const PrimeConst* __restrict__ pc, u64* __restrict__ arena, uint32_t n, const DiagGroup* __restrict__ groups,
     const DiagJob* __restrict__ jobs, const u64* __restrict__ srcs, const DiagUnit* __restrict__ units, u64 stride,
     int accumulate) {
@@ -424,22 +424,18 @@ __global__ void __launch_bounds__(kDiagTile, HALVES ? 3 : 2) diag_inner_staged_k
     const u64 first = J.add + row * stride + col;
     const u64 step = 2 * stride;
     auto issue_unit = [&](uint32_t k, u64 pt) {
-        if (NB > 1 || row == 0) {
-            const u64* g = arena + (first + pt);
-            u64* d = stage + ((k & 1u) * NB + row) * kDiagTile + col;
+        const u64* g = arena + (first + pt);
+        u64* d = stage + ((k & 1u) * NB + row) * kDiagTile + col;
 #pragma unroll
-            for (uint32_t r = 0; r < (NB + 1) / 2; ++r, g += step) cp_async16(d + 2 * r * kDiagTile, g);
-        }
+        for (uint32_t r = 0; r < NB / 2; ++r, g += step) cp_async16(d + 2 * r * kDiagTile, g);
         cp_async_commit();
     };
     auto issue_baby = [&](uint32_t k) {
         const uint32_t e = k - nu;
-        if (NB > 1 || row == 0) {
-            const u64* f = &from[e >> 1 & 1u][2 * row + (e & 1u)];
-            u64* d = stage + ((k & 1u) * NB + row) * kDiagTile + col;
+        const u64* f = &from[e >> 1 & 1u][2 * row + (e & 1u)];
+        u64* d = stage + ((k & 1u) * NB + row) * kDiagTile + col;
 #pragma unroll
-            for (uint32_t r = 0; r < (NB + 1) / 2; ++r) cp_async16(d + 2 * r * kDiagTile, arena + f[4 * r] + col);
-        }
+        for (uint32_t r = 0; r < NB / 2; ++r) cp_async16(d + 2 * r * kDiagTile, arena + f[4 * r] + col);
         cp_async_commit();
     };
     // the next unit's descriptor and automorphism index are loaded while the
@@ -455,7 +451,7 @@ __global__ void __launch_bounds__(kDiagTile, HALVES ? 3 : 2) diag_inner_staged_k
         __syncthreads();
         issue_baby(0);
     }
-    DiagSums<NB, HALVES> sums;
+    DiagSums<NB, true> sums;
     for (uint32_t k = 0; k < nu; ++k) {
         cp_async_wait<0>();
         __syncthreads();                    // item k is here, the other buffer free
@@ -483,17 +479,96 @@ __global__ void __launch_bounds__(kDiagTile, HALVES ? 3 : 2) diag_inner_staged_k
     }
 }
 
+// Up to three units an output, and no plaintexts shared between outputs (or one
+// unit): the sums above would only put the plaintexts' loads before the baby
+// steps'. Four baby steps at a time with all their loads in flight, products in 128
+// bits (they fit: 48 of below 2^61 squared; 25-bit halves are slower, 292 against
+// 253 us for 64 outputs of one shared unit at nb = 16, N = 2^15, two limbs). Any
+// placement, any alignment, any words. 64 outputs of one unit each at nb = 8, 60-bit
+// primes: 146 us (209 through the sums).
+template <int NB, int NU>
+__global__ void __launch_bounds__(kDiagTile) diag_inner_few_kernel(
+    const PrimeConst* __restrict__ pc, u64* __restrict__ arena, uint32_t n, const DiagJob* __restrict__ jobs,
+    const u64* __restrict__ srcs, const DiagUnit* __restrict__ units, u64 stride, int accumulate) {
+    constexpr int C = NB < 4 ? NB : 4;
+    const uint32_t l = blockIdx.z, i = blockIdx.y * kDiagTile + threadIdx.x;
+    if (i >= n) return;
+    const DiagJob J = jobs[blockIdx.x];
+    const ModConst m = modconst_of(pc[l]);
+    arena += (u64)l * n;
+    const u64* pt[NU];
+#pragma unroll
+    for (int u = 0; u < NU; ++u) {
+        const DiagUnit U = units[J.u0 + u];
+        pt[u] = arena + (U.pt + J.add + (U.map ? __ldg(U.map + i) : i));
+    }
+    srcs += 2ull * J.s;
+    Acc128 a0, a1;
+    acc_init(a0);
+    acc_init(a1);
+    u64 high = 0;
+#pragma unroll 2
+    for (int b = 0; b < NB; b += C) {
+        u64 p[C], x0[C], x1[C];
+#pragma unroll
+        for (int e = 0; e < C; ++e) {
+            x0[e] = arena[srcs[2 * (b + e)] + i];
+            x1[e] = arena[srcs[2 * (b + e) + 1] + i];
+            p[e] = 0;
+        }
+#pragma unroll
+        for (int u = 0; u < NU; ++u)
+#pragma unroll
+            for (int e = 0; e < C; ++e) {
+                const u64 v = pt[u][(b + e) * stride];
+                high |= v;
+                p[e] += v;
+            }
+#pragma unroll
+        for (int e = 0; e < C; ++e) {
+            high |= x0[e] | x1[e];
+            acc_mad(a0, p[e], x0[e]);
+            acc_mad(a1, p[e], x1[e]);
+        }
+    }
+    if (high >> 61) {                       // (words that are no residues)
+        acc_init(a0);
+        acc_init(a1);
+#pragma unroll 1
+        for (int b = 0; b < NB; ++b) {
+            u64 p = 0;
+            for (int u = 0; u < NU; ++u) p += reduce128(0, pt[u][b * stride], m);
+            acc_mad(a0, p, reduce128(0, arena[srcs[2 * b] + i], m));
+            acc_mad(a1, p, reduce128(0, arena[srcs[2 * b + 1] + i], m));
+        }
+    }
+    u64 r0 = acc_reduce(a0, m), r1 = acc_reduce(a1, m);
+    if (accumulate) {
+        r0 = add_mod(r0, arena[J.out0 + i], m.q);
+        r1 = add_mod(r1, arena[J.out1 + i], m.q);
+    }
+    arena[J.out0 + i] = r0;
+    arena[J.out1 + i] = r1;
+}
+
 template <int NB, bool HALVES>
 cudaError_t launch_diag(const PrimeConst* pc, u64* arena, uint32_t n, uint32_t limbs, uint32_t groups,
                         const DiagGroup* group, const DiagJob* job, const u64* srcs, const DiagUnit* unit, u64 stride,
-                        int accumulate, bool staged, cudaStream_t st) {
+                        int accumulate, bool staged, uint32_t few, cudaStream_t st) {
     const dim3 grid(groups, (n + kDiagTile - 1) / kDiagTile, limbs);
-    if (staged) {
-        const size_t smem = 2ull * NB * kDiagTile * sizeof(u64);
-        auto kern = diag_inner_staged_kernel<NB, HALVES>;
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-        kern<<<grid, kDiagTile, smem, st>>>(pc, arena, n, group, job, srcs, unit, stride, accumulate);
+    if (few) {
+        auto kern = few == 1 ? diag_inner_few_kernel<NB, 1> : few == 2 ? diag_inner_few_kernel<NB, 2> : diag_inner_few_kernel<NB, 3>;
+        kern<<<grid, kDiagTile, 0, st>>>(pc, arena, n, job, srcs, unit, stride, accumulate);
+    } else if (staged) {
+        if constexpr (HALVES && NB >= 8) {
+            const size_t smem = 2ull * NB * kDiagTile * sizeof(u64);
+            auto kern = diag_inner_staged_kernel<NB>;
+            cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            if (e != cudaSuccess) return e;
+            kern<<<grid, kDiagTile, smem, st>>>(pc, arena, n, group, job, srcs, unit, stride, accumulate);
+        } else {
+            return cudaErrorInvalidValue;
+        }
     } else {
         diag_inner_kernel<NB, HALVES><<<grid, kDiagTile, 0, st>>>(pc, arena, n, group, job, srcs, unit, stride, accumulate);
     }
@@ -503,26 +578,26 @@ cudaError_t launch_diag(const PrimeConst* pc, u64* arena, uint32_t n, uint32_t l
 
 cudaError_t launch_diag_inner(const PrimeConst* pc, u64* arena, uint32_t n, uint32_t limbs, uint32_t groups,
                               uint32_t nb, const DiagGroup* group, const DiagJob* job, const u64* srcs,
-                              const DiagUnit* unit, u64 stride, int accumulate, bool staged, bool halves,
+                              const DiagUnit* unit, u64 stride, int accumulate, bool staged, bool halves, uint32_t few,
                               cudaStream_t st) {
     if (limbs == 0 || groups == 0) return cudaSuccess;
-    if (limbs > 65535 || (staged && n % kDiagTile)) return cudaErrorInvalidValue;
+    if (limbs > 65535 || (staged && n % kDiagTile) || few > 3) return cudaErrorInvalidValue;
     switch (nb) {
     case 1:
-        return halves ? launch_diag<1, true>(pc, arena, n, limbs, groups, group, job, srcs, unit, stride, accumulate, staged, st)
-                      : launch_diag<1, false>(pc, arena, n, limbs, groups, group, job, srcs, unit, stride, accumulate, staged, st);
+        return halves ? launch_diag<1, true>(pc, arena, n, limbs, groups, group, job, srcs, unit, stride, accumulate, staged, few, st)
+                      : launch_diag<1, false>(pc, arena, n, limbs, groups, group, job, srcs, unit, stride, accumulate, staged, few, st);
     case 2:
-        return halves ? launch_diag<2, true>(pc, arena, n, limbs, groups, group, job, srcs, unit, stride, accumulate, staged, st)
-                      : launch_diag<2, false>(pc, arena, n, limbs, groups, group, job, srcs, unit, stride, accumulate, staged, st);
+        return halves ? launch_diag<2, true>(pc, arena, n, limbs, groups, group, job, srcs, unit, stride, accumulate, staged, few, st)
+                      : launch_diag<2, false>(pc, arena, n, limbs, groups, group, job, srcs, unit, stride, accumulate, staged, few, st);
     case 4:
-        return halves ? launch_diag<4, true>(pc, arena, n, limbs, groups, group, job, srcs, unit, stride, accumulate, staged, st)
-                      : launch_diag<4, false>(pc, arena, n, limbs, groups, group, job, srcs, unit, stride, accumulate, staged, st);
+        return halves ? launch_diag<4, true>(pc, arena, n, limbs, groups, group, job, srcs, unit, stride, accumulate, staged, few, st)
+                      : launch_diag<4, false>(pc, arena, n, limbs, groups, group, job, srcs, unit, stride, accumulate, staged, few, st);
     case 8:
-        return halves ? launch_diag<8, true>(pc, arena, n, limbs, groups, group, job, srcs, unit, stride, accumulate, staged, st)
-                      : launch_diag<8, false>(pc, arena, n, limbs, groups, group, job, srcs, unit, stride, accumulate, staged, st);
+        return halves ? launch_diag<8, true>(pc, arena, n, limbs, groups, group, job, srcs, unit, stride, accumulate, staged, few, st)
+                      : launch_diag<8, false>(pc, arena, n, limbs, groups, group, job, srcs, unit, stride, accumulate, staged, few, st);
     case 16:
-        return halves ? launch_diag<16, true>(pc, arena, n, limbs, groups, group, job, srcs, unit, stride, accumulate, staged, st)
-                      : launch_diag<16, false>(pc, arena, n, limbs, groups, group, job, srcs, unit, stride, accumulate, staged, st);
+        return halves ? launch_diag<16, true>(pc, arena, n, limbs, groups, group, job, srcs, unit, stride, accumulate, staged, few, st)
+                      : launch_diag<16, false>(pc, arena, n, limbs, groups, group, job, srcs, unit, stride, accumulate, staged, few, st);
     default: return cudaErrorInvalidValue;
     }
 }

@@ -32,11 +32,12 @@ def diag(ctx, outs, srcs, nb, units, gals, stride, limbs, accumulate=0):
 
 @pytest.mark.parametrize("nb,q_bits", [(1, 50), (4, 50), (16, 50), (2, 60), (16, 60)])
 @pytest.mark.parametrize("which", ["c0 of the first", "c1 of the last", "c0 in the middle"])
-def test_sources_at_odd_words(nb, q_bits, which):
+@pytest.mark.parametrize("nu", [3, 5])
+def test_sources_at_odd_words(nb, q_bits, which, nu):
     q, p = primes_for(LOG_N, LIMBS, q_bits, 1, 61 if q_bits == 60 else 60)
     n = 1 << LOG_N
     w = LIMBS * n
-    ctx = FheContext(CkksParams(LOG_N, q, p, 1), poly_words=160 * w, key_words=1024)
+    ctx = FheContext(CkksParams(LOG_N, q, p, 1), poly_words=180 * w, key_words=1024)
     try:
         rng = np.random.default_rng([nb, q_bits])
         srcs = [[(2 * b * w, (2 * b + 1) * w) for b in range(nb)] for _ in range(2)]
@@ -45,14 +46,14 @@ def test_sources_at_odd_words(nb, q_bits, which):
         srcs[j][b] = (srcs[j][b][0], odd) if which.startswith("c1") else (odd, srcs[j][b][1])
         for at in {o for s in srcs for c in s for o in c}:
             ctx.write_poly(at, uniform_residues(rng, q, n))
-        for k in range(48, 48 + 4 * nb):
+        for k in range(48, 48 + (nu + 1) * nb):
             ctx.write_poly(k * w, uniform_residues(rng, q, n))
         gals = [1, galois_elt(LOG_N, -64), galois_elt(LOG_N, -256)]
-        units = [[(48 + nb * k) * w for k in range(3)], [(48 + nb * k) * w for k in range(1, 4)]]
-        outs = [((120 + 2 * j) * w, (121 + 2 * j) * w) for j in range(2)]
-        outs_b = [((130 + 2 * j) * w, (131 + 2 * j) * w) for j in range(2)]
+        units = [[(48 + nb * k) * w for k in range(nu)], [(48 + nb * k) * w for k in range(1, nu + 1)]]
+        outs = [((160 + 2 * j) * w, (161 + 2 * j) * w) for j in range(2)]
+        outs_b = [((170 + 2 * j) * w, (171 + 2 * j) * w) for j in range(2)]
         assert diag(ctx, outs, srcs, nb, units, gals, w, LIMBS) == L.OK, ctx.lib.afhe_last_error()
-        mac = [[(srcs[j][b], [(u + b * w, gals[k]) for k, u in enumerate(units[j])]) for b in range(nb)]
+        mac = [[(srcs[j][b], [(u + b * w, gals[k % 3]) for k, u in enumerate(units[j])]) for b in range(nb)]
                for j in range(2)]
         assert call(ctx, outs_b, mac, LIMBS) == L.OK, ctx.lib.afhe_last_error()
         for a, b in zip(outs, outs_b):
@@ -64,8 +65,9 @@ def test_sources_at_odd_words(nb, q_bits, which):
 
 @pytest.mark.parametrize("nb", [1, 4, 16])
 @pytest.mark.parametrize("what", ["plaintexts", "sources", "both"])
+@pytest.mark.parametrize("nu", [2, 5])
 @pytest.mark.parametrize("local", [True, False])
-def test_words_that_are_no_residues(nb, what, local):
+def test_words_that_are_no_residues(nb, what, local, nu):
     """Below 2^50 the products split words in halves: other words are taken modulo
     their prime, any by the form for any placement, plaintexts below 2^57 and
     sources below 2^53 by the shared-memory form."""
@@ -89,11 +91,11 @@ def test_words_that_are_no_residues(nb, what, local):
             return x, y
 
         srcs = [[(2 * b * w, (2 * b + 1) * w) for b in range(nb)]]
-        gals = [1, galois_elt(LOG_N, -64), galois_elt(LOG_N, 128 if local else 5)]
-        units = [[(40 + nb * k) * w for k in range(5)]]
+        gals = [galois_elt(LOG_N, 128 if local else 5), 1, galois_elt(LOG_N, -64)]
+        units = [[(40 + nb * k) * w for k in range(nu)]]
         most = (1 << 53, 1 << 57) if local else (1 << 64, 1 << 64)
         data = {k: poly(what != "plaintexts", most[0]) if k < 32 else poly(what != "sources", most[1])
-                for k in [*range(2 * nb), *range(40, 40 + 5 * nb)]}
+                for k in [*range(2 * nb), *range(40, 40 + nu * nb)]}
         got = []
         for form in range(2):              # residues through the sums of products, then the words
             for k, v in data.items():
@@ -107,5 +109,37 @@ def test_words_that_are_no_residues(nb, what, local):
             got.append([ctx.read_poly(o, w) for o in out[0]])
         assert np.array_equal(got[0][0], got[1][0])
         assert np.array_equal(got[0][1], got[1][1])
+    finally:
+        ctx.close()
+
+
+@pytest.mark.parametrize("nb", [1, 2, 4, 8, 16])
+@pytest.mark.parametrize("q_bits", [50, 61])
+@pytest.mark.parametrize("nu,shared", [(1, False), (2, False), (3, False), (4, False), (1, True), (3, True)])
+def test_few_units(nb, q_bits, nu, shared):
+    """Outputs of one to three units are read straight through, unless they share
+    their plaintexts; plaintexts and sources of all q - 1 among them."""
+    q, p = primes_for(LOG_N, LIMBS, q_bits, 1, 60)
+    n = 1 << LOG_N
+    w = LIMBS * n
+    top = np.repeat(np.array(q, dtype=np.uint64) - 1, n)
+    ctx = FheContext(CkksParams(LOG_N, q, p, 1), poly_words=260 * w, key_words=1024)
+    try:
+        rng = np.random.default_rng([nb, q_bits, nu])
+        for k in range(40 + 3 * nu * nb):
+            ctx.write_poly(k * w, top if k % 5 < 2 else uniform_residues(rng, q, n))
+        gals = [1, galois_elt(LOG_N, -64), galois_elt(LOG_N, 256)]
+        srcs = [[((2 * b + j) * w, (2 * b + 1 + j) * w) for b in range(nb)] for j in range(3)]
+        units = [[(40 + nb * (k + (0 if shared else j) * nu)) * w for k in range(nu)] for j in range(3)]
+        outs = [((240 + 2 * j) * w, (241 + 2 * j) * w) for j in range(3)]
+        outs_b = [((250 + 2 * j) * w, (251 + 2 * j) * w) for j in range(3)]
+        for accumulate in (0, 1):
+            assert diag(ctx, outs, srcs, nb, units, gals, w, LIMBS, accumulate) == L.OK, ctx.lib.afhe_last_error()
+            mac = [[(srcs[j][b], [(u + b * w, gals[k % 3]) for k, u in enumerate(units[j])]) for b in range(nb)]
+                   for j in range(3)]
+            assert call(ctx, outs_b, mac, LIMBS, accumulate) == L.OK, ctx.lib.afhe_last_error()
+            for a, b in zip(outs, outs_b):
+                assert np.array_equal(ctx.read_poly(a[0], w), ctx.read_poly(b[0], w)), accumulate
+                assert np.array_equal(ctx.read_poly(a[1], w), ctx.read_poly(b[1], w)), accumulate
     finally:
         ctx.close()
