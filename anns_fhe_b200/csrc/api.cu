@@ -193,6 +193,12 @@ const char* afhe_last_error(void) { return g_last_error.c_str(); }
 // ===========================================================================
 namespace {
 
+// The first prime whose transforms read a second pair for each twiddle (none: their
+// number).
+uint32_t first_split_prime(const std::vector<u64>& primes) {
+    return (uint32_t)(std::find_if(primes.begin(), primes.end(), [](u64 q) { return q >= kFpLimit; }) - primes.begin());
+}
+
 int build_native_tables(afhe_ctx* ctx) {
     const uint32_t n = ctx->n, L = ctx->L, K = ctx->K, np = L + K;
     std::vector<u64> primes(np);
@@ -214,8 +220,11 @@ int build_native_tables(afhe_ctx* ctx) {
     CK(dalloc(&s.pc, np));
     CK(dalloc(&s.tw2, (size_t)np * n));
     CK(dalloc(&s.itw2, (size_t)np * n));
-    CK(dalloc(&s.tw2b, (size_t)np * n));
-    CK(dalloc(&s.itw2b, (size_t)np * n));
+    s.first_b = first_split_prime(primes);
+    if (s.first_b < np) {
+        CK(dalloc(&s.tw2b, (size_t)(np - s.first_b) * n));
+        CK(dalloc(&s.itw2b, (size_t)(np - s.first_b) * n));
+    }
     CK(upload(ctx, s.pc, pc.data(), np * sizeof(PrimeConst)));
     {
         u64* raw = nullptr;
@@ -224,8 +233,8 @@ int build_native_tables(afhe_ctx* ctx) {
         cudaError_t e = upload(ctx, raw, tw.data(), w * 8);
         if (e == cudaSuccess) e = upload(ctx, raw + w, itw.data(), w * 8);
         if (e == cudaSuccess) e = upload(ctx, raw + 2 * w, primes.data(), np * 8);
-        if (e == cudaSuccess) e = launch_twiddles(raw, raw + 2 * w, s.tw2, s.tw2b, np, ctx->log_n, ctx->st);
-        if (e == cudaSuccess) e = launch_twiddles(raw + w, raw + 2 * w, s.itw2, s.itw2b, np, ctx->log_n, ctx->st);
+        if (e == cudaSuccess) e = launch_twiddles(raw, raw + 2 * w, s.tw2, s.tw2b, s.first_b, np, ctx->log_n, ctx->st);
+        if (e == cudaSuccess) e = launch_twiddles(raw + w, raw + 2 * w, s.itw2, s.itw2b, s.first_b, np, ctx->log_n, ctx->st);
         if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->st);
         cudaFree(raw);
         if (e != cudaSuccess) return cuda_fail(ctx, e, "twiddle tables");
@@ -316,7 +325,7 @@ int build_native_tables(afhe_ctx* ctx) {
         OpTabs& t = ctx->lv[lvl];
         const LvlRefs& R = refs[lvl];
         const u64* b = ctx->lvbuf;
-        t.pt = s.view();
+        t.pt = s.view(ctx->log_n);
         t.p_base = L;
         t.sizeQl = lvl;
         t.parts = R.parts;
@@ -819,8 +828,6 @@ int load_context(afhe_ctx* ctx, const afhe_accel_args* a) {
         CK(dalloc(&s.itw, (size_t)(AFHE_MAX_Q + AFHE_MAX_P) * n));
         CK(dalloc(&s.tw2, (size_t)(AFHE_MAX_Q + AFHE_MAX_P) * n));
         CK(dalloc(&s.itw2, (size_t)(AFHE_MAX_Q + AFHE_MAX_P) * n));
-        CK(dalloc(&s.tw2b, (size_t)(AFHE_MAX_Q + AFHE_MAX_P) * n));
-        CK(dalloc(&s.itw2b, (size_t)(AFHE_MAX_Q + AFHE_MAX_P) * n));
         s.count = AFHE_MAX_Q + AFHE_MAX_P;
     }
     cudaStream_t st = ctx->st;
@@ -833,14 +840,18 @@ int load_context(afhe_ctx* ctx, const afhe_accel_args* a) {
         qv[i] = i < L ? a->rns_primes[i] : a->p_primes[i - L];
         ninv[i] = i < L ? a->n_inv_q[i] : a->n_inv_p[i - L];
     }
+    if (first_split_prime(qv) < L + K) {        // (kept for the contexts loaded next)
+        if (!s.tw2b) CK(dalloc(&s.tw2b, (size_t)(AFHE_MAX_Q + AFHE_MAX_P) * n));
+        if (!s.itw2b) CK(dalloc(&s.itw2b, (size_t)(AFHE_MAX_Q + AFHE_MAX_P) * n));
+    }
     u64* dq = nullptr;
     u64* dn = nullptr;
     CK(dalloc(&dq, L + K));
     CK(dalloc(&dn, L + K));
     CK(cudaMemcpyAsync(dq, qv.data(), qv.size() * 8, cudaMemcpyHostToDevice, st));
     CK(cudaMemcpyAsync(dn, ninv.data(), ninv.size() * 8, cudaMemcpyHostToDevice, st));
-    CK(launch_twiddles(s.tw, dq, s.tw2, s.tw2b, L + K, ctx->log_n, st));
-    CK(launch_twiddles(s.itw, dq, s.itw2, s.itw2b, L + K, ctx->log_n, st));
+    CK(launch_twiddles(s.tw, dq, s.tw2, s.tw2b, 0, L + K, ctx->log_n, st));
+    CK(launch_twiddles(s.itw, dq, s.itw2, s.itw2b, 0, L + K, ctx->log_n, st));
     CK(launch_prime_consts(s.pc, dq, dn, s.itw, n, L + K, st));
     CK(cudaStreamSynchronize(st));
     cudaFree(dq); cudaFree(dn);
@@ -916,7 +927,7 @@ int prep_loaded_tables(afhe_ctx* ctx, uint32_t sizeQl, uint32_t parts, uint32_t 
     std::vector<u64> mods(W, 0);
     const u64* q = ctx->ld_q.data();
     const u64* p = ctx->ld_p.data();
-    t->pt = ctx->ld.view();
+    t->pt = ctx->ld.view(ctx->log_n);
     t->p_base = Lld;
     t->sizeQl = sizeQl;
     t->parts = parts;
@@ -1027,7 +1038,7 @@ extern "C" int afhe_dispatch(afhe_ctx* ctx, const afhe_accel_args* a) {
         zb.src = zf_const(src);
         zb.mid = zf_const(a->dst_offset);
         zb.out = zf_const(a->dst_offset);
-        CK(launch_ntt_plain(a->op_code == AFHE_OP_INTT, ctx->log_n, ctx->ld.view(), djobs, L,
+        CK(launch_ntt_plain(a->op_code == AFHE_OP_INTT, ctx->log_n, ctx->ld.view(ctx->log_n), djobs, L,
                             in_scr ? ctx->scr : ctx->poly, ctx->poly, 1, zb, st));
         break;
     }

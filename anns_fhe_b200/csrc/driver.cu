@@ -463,7 +463,7 @@ static int ntt_native(afhe_ctx* ctx, bool inv, uint64_t src, uint64_t dst, uint3
     zb.src = zf_const(s);
     zb.mid = zf_const(dst);
     zb.out = zf_const(dst);
-    CK(launch_ntt_plain(inv, ctx->log_n, ctx->nat.view(), ctx->jobs_qp, limbs, ctx->poly, ctx->poly, 1, zb, ctx->st));
+    CK(launch_ntt_plain(inv, ctx->log_n, ctx->nat.view(ctx->log_n), ctx->jobs_qp, limbs, ctx->poly, ctx->poly, 1, zb, ctx->st));
     return AFHE_OK;
 }
 
@@ -1271,7 +1271,7 @@ int afhe_ntt_batch(afhe_ctx* ctx, const uint64_t* polys, uint32_t count, uint32_
         ZF(zb.src, v);
         zb.mid = zb.src;
         zb.out = zb.src;
-        CK(launch_ntt_plain(inverse != 0, ctx->log_n, ctx->nat.view(), ctx->jobs_qp, limbs, ctx->poly, ctx->poly, m,
+        CK(launch_ntt_plain(inverse != 0, ctx->log_n, ctx->nat.view(ctx->log_n), ctx->jobs_qp, limbs, ctx->poly, ctx->poly, m,
                             zb, ctx->st));
     }
     return AFHE_OK;
@@ -1300,7 +1300,7 @@ int afhe_decrypt_batch(afhe_ctx* ctx, const afhe_ct_ref* cts, uint32_t count, ui
         if ((rc = ew_fields(ctx, EW_ADD, O, f0, O, m, limbs)) != AFHE_OK) return rc;                    // + c0
         ZBases zb{};
         zb.src = zb.mid = zb.out = O;
-        CK(launch_ntt_plain(true, ctx->log_n, ctx->nat.view(), ctx->jobs_qp, limbs, ctx->poly, ctx->poly, m, zb,
+        CK(launch_ntt_plain(true, ctx->log_n, ctx->nat.view(ctx->log_n), ctx->jobs_qp, limbs, ctx->poly, ctx->poly, m, zb,
                             ctx->st));
     }
     return AFHE_OK;

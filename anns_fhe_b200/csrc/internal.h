@@ -40,7 +40,9 @@ struct OpTabs {
 
 // Owned device storage for one twiddle table set. tw / itw hold raw tables
 // (only for tables loaded by OP_LOAD_CONTEXT); tw2 / itw2 (tw2b / itw2b) the
-// transform constants the kernels read.
+// transform constants the kernels read. Primes below 2^50 have no second pair:
+// tw2b / itw2b start at row first_b, that of the first other prime (null where
+// there is none).
 struct DevPrimeSet {
     PrimeConst* pc = nullptr;
     u64* tw = nullptr;
@@ -50,7 +52,13 @@ struct DevPrimeSet {
     ulonglong2* tw2b = nullptr;
     ulonglong2* itw2b = nullptr;
     uint32_t count = 0;
-    PrimeTables view() const { return PrimeTables{pc, tw2, itw2, tw2b, itw2b}; }
+    uint32_t first_b = 0;
+    // (rows below first_b are never read)
+    PrimeTables view(int log_n) const {
+        const uintptr_t back = ((uintptr_t)first_b << log_n) * sizeof(ulonglong2);
+        auto from = [&](const ulonglong2* t) { return t ? (const ulonglong2*)((uintptr_t)t - back) : nullptr; };
+        return PrimeTables{pc, tw2, itw2, from(tw2b), from(itw2b)};
+    }
 };
 
 // Ring of small per-launch descriptor arrays (ZField::arr): pinned host
@@ -298,9 +306,10 @@ cudaError_t launch_key_prep(const u64* key, ulonglong2* prep, const PrimeConst* 
                             uint32_t dnum, uint32_t alpha, u64 words, cudaStream_t st);
 
 // Twiddle rows: raw[r n + j] = psi^bitrev(j) mod q[r] (or its inverse), j < n,
-// as transform constants in the rounds' order (PrimeTables).
-cudaError_t launch_twiddles(const u64* raw, const u64* q, ulonglong2* out2, ulonglong2* out2b, uint32_t rows, int log_n,
-                            cudaStream_t st);
+// as transform constants in the rounds' order (PrimeTables); the second
+// pairs of primes from 2^50 on at out2b, which starts at row first_b.
+cudaError_t launch_twiddles(const u64* raw, const u64* q, ulonglong2* out2, ulonglong2* out2b, uint32_t first_b,
+                            uint32_t rows, int log_n, cudaStream_t st);
 // Table prep: entry v[e] mod m[e] in split form at sp + 4 e and as a transform
 // constant at tc + 4 e (where m[e] is not 0).
 cudaError_t launch_table_constants(const u64* v, const u64* m, u64* sp, u64* tc, size_t count, cudaStream_t st);

@@ -647,7 +647,7 @@ cudaError_t launch_table_constants(const u64* v, const u64* m, u64* sp, u64* tc,
 }
 
 __global__ void twiddles_kernel(const u64* __restrict__ raw, const u64* __restrict__ q, ulonglong2* __restrict__ out2,
-                                ulonglong2* __restrict__ out2b, uint32_t rows, int log_n) {
+                                ulonglong2* __restrict__ out2b, uint32_t first_b, uint32_t rows, int log_n) {
     const size_t total = (size_t)rows << log_n;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
         const size_t row = i >> log_n;
@@ -661,17 +661,17 @@ __global__ void twiddles_kernel(const u64* __restrict__ raw, const u64* __restri
             at = tw_place(log_n, log_n - 1 - lg, j - (1u << lg));
         }
         out2[(row << log_n) + at] = make_ulonglong2(o[0], o[1]);
-        out2b[(row << log_n) + at] = make_ulonglong2(o[2], o[3]);
+        if (m >= kFpLimit) out2b[((row - first_b) << log_n) + at] = make_ulonglong2(o[2], o[3]);
     }
 }
 
-cudaError_t launch_twiddles(const u64* raw, const u64* q, ulonglong2* out2, ulonglong2* out2b, uint32_t rows, int log_n,
-                            cudaStream_t st) {
+cudaError_t launch_twiddles(const u64* raw, const u64* q, ulonglong2* out2, ulonglong2* out2b, uint32_t first_b,
+                            uint32_t rows, int log_n, cudaStream_t st) {
     if (rows == 0) return cudaSuccess;
     const size_t total = (size_t)rows << log_n;
     unsigned blocks = (unsigned)((total + 255) / 256);
     if (blocks > 8192) blocks = 8192;
-    twiddles_kernel<<<blocks, 256, 0, st>>>(raw, q, out2, out2b, rows, log_n);
+    twiddles_kernel<<<blocks, 256, 0, st>>>(raw, q, out2, out2b, first_b, rows, log_n);
     count_launches(1);
     return cudaGetLastError();
 }
