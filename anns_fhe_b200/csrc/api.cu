@@ -437,8 +437,7 @@ int afhe_ctx_create(const afhe_params* prm, afhe_ctx** out) {
         {
             const char* v = std::getenv("AFHE_KS_FUSED");
             ctx->ks_fused = key_switch_fused_supported(ctx->log_n) && !(v && v[0] == '0');
-            // (below N = 2^13; above it the line is drawn by level, and this
-            // value stands for that)
+            // (this value stands for a line drawn by level)
             int sms = 148;
             cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
             ctx->sms = (uint32_t)std::max(1, sms);

@@ -96,27 +96,41 @@ int cached_map(afhe_ctx* ctx, uint32_t galois, const uint32_t** out) {
 // the kernel pipeline takes the rest. The one-kernel path runs `capacity`
 // ciphertexts at once and a partial wave costs nearly a whole one, the pipeline's
 // time grows with the count: whole waves and a remainder that nearly fills one
-// go to the former. The line lies where both took the same time (microseconds,
-// one kernel / pipeline): N = 2^13, three digits: 40: 203 / 164, 56: 205 / 215,
-// 148: 317 / 429, 160: 533 / 477; N = 2^14, three digits: 56: 1306 / 1179, 71: 1329
-// / 1476, 80: 2231 / 1653; N = 2^15, one digit (four limbs): 20: 416 / 390, 22: 418
-// / 420, 33: 441 / 603, 40: 797 / 716; three digits: 33: 1646 / 1627, 45: 3004 /
-// 2188; N = 2^16, one digit: 12: 783 / 754, 15: 803 / 934; two or more (8 limbs,
-// 24): 12: 1325 / 1072, 4521 / 3204.
+// go to the former. The line lies where both took the same time, by ring degree and
+// digits (microseconds, one kernel / pipeline, primes of 50 bits unless said
+// otherwise; L + K limbs):
+//   N = 2^10, one digit (2 + 2): 40: 44 / 45; two (2 + 1): 40: 45 / 45; three (3 + 1):
+//     120: 65 / 62, 148: 66 / 69, (6 + 2): 148: 129 / 113, 220: 150 / 157
+//   N = 2^11, one (2 + 2): 40: 55 / 52, 74: 55 / 58; two (2 + 1): 60: 56 / 53, 74: 56 /
+//     57; three (3 + 1): 90: 84 / 78, 120: 84 / 95, (6 + 2): 120: 176 / 171
+//   N = 2^12, one (2 + 2): 60: 84 / 78, 74: 84 / 83; two (2 + 1): 60: 80 / 74, 74: 80 /
+//     80; three (3 + 1): 74: 129 / 123, 90: 131 / 139, (6 + 2): 74: 291 / 217, 120:
+//     312 / 342, (3 + 1 of 60 bits): 74: 169 / 148, 90: 169 / 170
+//   N = 2^13, one (2 + 2): 20: 121 / 105, 40: 125 / 138, (1 + 1): 2: 65 / 89; two (2 + 1):
+//     20: 130 / 102, 40: 129 / 138; three (3 + 1): 40: 203 / 163, 60: 226 / 221, 100:
+//     292 / 333, six (6 + 1): 100: 772 / 723, 148: 796 / 1009
+//   N = 2^14, one (4 + 4): 40: 396 / 379, 55: 412 / 492, (1 + 1): 10: 67 / 78; two (8 + 4):
+//     55: 898 / 878, 71: 932 / 1121, (2 + 1): 40: 180 / 195; six (6 + 1): 55: 827 / 795,
+//     71: 838 / 1006
+//   N = 2^15, one (4 + 4): 20: 416 / 393, 28: 428 / 529, (1 + 1): 10: 70 / 96; two (8 +
+//     4): 28: 938 / 925, 33: 965 / 1076, (2 + 1): 20: 188 / 201; three (12 + 4): 33:
+//     1646 / 1627, 45: 3004 / 2188, (6 + 2): 33: 706 / 808
+//   N = 2^16, one (8 + 8): 8: 1066 / 720, 15: 1147 / 1302, (1 + 1): 8: 99 / 113; two (4 +
+//     2): 8: 499 / 322, 15: 515 / 550; six (6 + 1): 15: 998 / 999; two of 8 limbs, three
+//     of 24: 12: 1325 / 1072, 4521 / 3204
 uint32_t ks_fused_part(afhe_ctx* ctx, uint32_t nz, uint32_t limbs) {
-    const bool by_level = ctx->fused_min == ctx->fused_default && ctx->log_n >= 13;
+    const bool by_level = ctx->fused_min == ctx->fused_default;
     if (!ctx->ks_fused || nz < (by_level ? 2 : ctx->fused_min)) return 0;
     if (ctx->fused_min == 1) return nz;
     if (!ctx->ks_capacity) ctx->ks_capacity = std::max(1, key_switch_fused_capacity(ctx->log_n));
     const uint32_t cap = ctx->ks_capacity;
-    uint32_t line = ctx->fused_min;
-    if (ctx->log_n >= 13) {
-        static const uint8_t percent[4][3] = {{5, 27, 35}, {63, 85, 90}, {65, 92, 255}, {85, 255, 255}};
-        const uint32_t share = percent[ctx->log_n - 13][std::min(ctx->lv[limbs].parts, 3u) - 1];
-        if (by_level && share == 255) return 0;
-        line = std::max(1u, cap * share / 100);
-        if (!by_level) line = std::min(line, ctx->fused_min);       // (nz is at least fused_min)
-    }
+    // percent of a wave, by digits (255: the pipeline throughout)
+    static const uint8_t percent[7][3] = {{3, 3, 12}, {11, 12, 18}, {25, 25, 32}, {5, 27, 35},
+                                          {63, 85, 90}, {65, 92, 255}, {85, 255, 255}};
+    const uint32_t share = percent[ctx->log_n - 10][std::min(ctx->lv[limbs].parts, 3u) - 1];
+    if (by_level && share == 255) return 0;
+    uint32_t line = std::max(1u, cap * share / 100);
+    if (!by_level) line = std::min(line, ctx->fused_min);       // (nz is at least fused_min)
     const uint32_t rest = nz % cap;
     if (rest >= line || (rest == nz && !by_level)) return nz;
     return nz - rest;

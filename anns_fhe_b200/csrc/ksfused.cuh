@@ -6,7 +6,7 @@
 // polynomial is carried through every step by one CTA (N <= 2^12) or by a
 // thread-block cluster of CL CTAs, each holding a slice of the limb being
 // transformed (2^12 values and CL = 2, 4, 8 at N = 2^13, 2^14, 2^15; 2^13
-// values and CL = 8 at N = 2^16), sixteen values per thread:
+// values and CL = 8 at N = 2^16), sixteen values per thread (or eight, see launch_fused):
 //
 //   phase 0  coef[i] = INTT(in[i]) * qHatInv_i for the input's Q limbs -> lane scratch
 //   phase 1  for every special slot k: per digit BConv(coef) + NTT and the
@@ -80,17 +80,16 @@ struct KsFusedArgs {
 
 // log2 of the values a CTA holds, at ring degree 2^log_n
 inline constexpr int slice_bits(int log_n) { return log_n <= 12 ? log_n : (log_n == 16 ? 13 : 12); }
-constexpr uint32_t kE = 16;    // values per thread: two groups of the rounds' eight (128 registers)
-constexpr uint32_t kG = kE / 8;
 
-template <int LOGQ, int LOGCL>
+template <int LOGQ, int LOGCL, uint32_t E>
 struct Geo {
     static constexpr int LOGN = LOGQ + LOGCL;
     static constexpr uint32_t QN = 1u << LOGQ;
     static constexpr uint32_t CL = 1u << LOGCL;
-    static constexpr uint32_t T = QN / kE;            // threads
+    static constexpr uint32_t KG = E / 8;             // groups of the rounds' eight values a thread
+    static constexpr uint32_t T = QN / E;             // threads
     static constexpr uint32_t PER = QN / CL;          // columns per CTA
-    static constexpr uint32_t CPT = kE / CL;          // columns per thread
+    static constexpr uint32_t CPT = E / CL;           // columns per thread
     static constexpr uint32_t PADQ = QN + QN / 16;
     static_assert(CL <= 8 && PER == T * CPT, "a thread's columns hold its values");
     __device__ __forceinline__ static uint32_t rank() {
@@ -110,7 +109,7 @@ struct Geo {
         arrive();
         wait();
     }
-    // position i < kE of this thread's columns: value k = i % CL of column
+    // position i < E of this thread's columns: value k = i % CL of column
     // i / CL; global index and index in the slice of CTA k
     __device__ __forceinline__ static uint32_t column(uint32_t i) {
         return rank() * PER + threadIdx.x + (i >> LOGCL) * T;
@@ -155,61 +154,61 @@ __device__ __forceinline__ void sync_round() {
     }
 }
 
-template <class A, bool INV, int LOGQ, int RB, int K, int LOGN>
+template <class A, bool INV, int LOGQ, int RB, int K, int LOGN, uint32_t E>
 struct KsRound {
-    typedef NttRound<A, INV, LOGN, 0, LOGQ, 0, false, RB, K, kE> R;
+    typedef NttRound<A, INV, LOGN, 0, LOGQ, 0, false, RB, K, E> R;
 };
 
 // Forward rounds from the top of the slice down to bit 3: on entry the slices
 // are written and visible, on return this thread's groups of adjacent values are.
-template <class A, int LOGQ, int LOGCL, int NB, int I = 0>
+template <class A, int LOGQ, int LOGCL, uint32_t E, int NB, int I = 0>
 __device__ __forceinline__ void fwd_rounds(u64* const (&bufs)[NB], const TwRow& tw, const typename A::C& c) {
-    using G = Geo<LOGQ, LOGCL>;
+    using G = Geo<LOGQ, LOGCL, E>;
     typedef Rounds<false, LOGQ> R;
     if constexpr (I < R::NR - 1) {
-        KsRound<A, false, LOGQ, R::rb(I), R::k(I), G::LOGN>::R::template run_n<NB>(bufs, tw, c, nullptr, G::rank(),
+        KsRound<A, false, LOGQ, R::rb(I), R::k(I), G::LOGN, E>::R::template run_n<NB>(bufs, tw, c, nullptr, G::rank(),
                                                                                     I > 0 || LOGCL > 0 ? kEarlier : kResidues, false);
         sync_round<R::rb(I), G::T>();
-        fwd_rounds<A, LOGQ, LOGCL, NB, I + 1>(bufs, tw, c);
+        fwd_rounds<A, LOGQ, LOGCL, E, NB, I + 1>(bufs, tw, c);
     }
 }
 // Inverse rounds from bit 3 up: on entry every thread has stored its groups of
 // adjacent values; without a cluster fin holds the constants of the transform's
 // last stage and the results are canonical residues.
-template <class A, int LOGQ, int LOGCL, int NB, int I = 1>
+template <class A, int LOGQ, int LOGCL, uint32_t E, int NB, int I = 1>
 __device__ __forceinline__ void inv_rounds(u64* const (&bufs)[NB], const TwRow& tw, const typename A::C& c,
                                            const u64* fin) {
-    using G = Geo<LOGQ, LOGCL>;
+    using G = Geo<LOGQ, LOGCL, E>;
     typedef Rounds<true, LOGQ> R;
     if constexpr (I < R::NR) {
         sync_round<R::rb(I), G::T>();
-        KsRound<A, true, LOGQ, R::rb(I), R::k(I), G::LOGN>::R::template run_n<NB>(bufs, tw, c, fin, G::rank(), kEarlier,
+        KsRound<A, true, LOGQ, R::rb(I), R::k(I), G::LOGN, E>::R::template run_n<NB>(bufs, tw, c, fin, G::rank(), kEarlier,
                                                                                 LOGCL == 0 && I == R::NR - 1);
-        inv_rounds<A, LOGQ, LOGCL, NB, I + 1>(bufs, tw, c, fin);
+        inv_rounds<A, LOGQ, LOGCL, E, NB, I + 1>(bufs, tw, c, fin);
     }
 }
-template <class A, int LOGQ, int LOGCL, int NB>
+template <class A, int LOGQ, int LOGCL, uint32_t E, int NB>
 __device__ AFHE_KS_FN void fwd_rounds_call(u64* b0, u64* b1, const PrimeTables* pt, uint32_t prime) {
     const TwRow tw = tw_row<false>(*pt, prime, LOGQ + LOGCL);
     const typename A::C c = A::consts(pt->pc[prime]);
     if constexpr (NB == 2) {
         u64* const two[2] = {b0, b1};
-        fwd_rounds<A, LOGQ, LOGCL, 2>(two, tw, c);
+        fwd_rounds<A, LOGQ, LOGCL, E, 2>(two, tw, c);
     } else {
         u64* const one[1] = {b0};
-        fwd_rounds<A, LOGQ, LOGCL, 1>(one, tw, c);
+        fwd_rounds<A, LOGQ, LOGCL, E, 1>(one, tw, c);
     }
 }
-template <class A, int LOGQ, int LOGCL, int NB>
+template <class A, int LOGQ, int LOGCL, uint32_t E, int NB>
 __device__ AFHE_KS_FN void inv_rounds_call(u64* b0, u64* b1, const PrimeTables* pt, uint32_t prime, const u64* fin) {
     const TwRow tw = tw_row<true>(*pt, prime, LOGQ + LOGCL);
     const typename A::C c = A::consts(pt->pc[prime]);
     if constexpr (NB == 2) {
         u64* const two[2] = {b0, b1};
-        inv_rounds<A, LOGQ, LOGCL, 2>(two, tw, c, fin);
+        inv_rounds<A, LOGQ, LOGCL, E, 2>(two, tw, c, fin);
     } else {
         u64* const one[1] = {b0};
-        inv_rounds<A, LOGQ, LOGCL, 1>(one, tw, c, fin);
+        inv_rounds<A, LOGQ, LOGCL, E, 1>(one, tw, c, fin);
     }
 }
 
@@ -226,10 +225,10 @@ struct TwCross {
 // its own slice) as the inputs of a forward transform: the stages across the
 // cluster in registers, then the values to their slices' W. A barrier over
 // the polynomial's CTAs (sync_all) has to follow the last group.
-template <class A, int LOGQ, int LOGCL>
+template <class A, int LOGQ, int LOGCL, uint32_t E>
 __device__ __forceinline__ void fwd_enter(typename A::V* v, uint32_t g, u64* W, const TwRow& tw,
                                           const typename A::C& c) {
-    using G = Geo<LOGQ, LOGCL>;
+    using G = Geo<LOGQ, LOGCL, E>;
     if constexpr (LOGCL == 0) {
 #pragma unroll
         for (uint32_t i = 0; i < 8; ++i) W[G::spos(8 * g + i)] = A::store(v[i]);
@@ -250,9 +249,9 @@ __device__ __forceinline__ void fwd_enter(typename A::V* v, uint32_t g, u64* W, 
 // (columns of every CTA's slice of buf), inv_leave runs the stages across the
 // cluster; v[i] = the canonical residue at column_x(8 g + i) (at this thread's
 // lpos(8 g + i) without a cluster).
-template <int LOGQ, int LOGCL>
+template <int LOGQ, int LOGCL, uint32_t E>
 __device__ __forceinline__ void inv_gather(u64* v, uint32_t g, const u64* buf) {
-    using G = Geo<LOGQ, LOGCL>;
+    using G = Geo<LOGQ, LOGCL, E>;
     if constexpr (LOGCL == 0) {
 #pragma unroll
         for (uint32_t i = 0; i < 8; ++i) v[i] = buf[G::spos(8 * g + i)];
@@ -263,9 +262,9 @@ __device__ __forceinline__ void inv_gather(u64* v, uint32_t g, const u64* buf) {
             v[i] = ld_cluster(map_rank(base, i & (G::CL - 1)) + 8 * padix(G::column(8 * g + i)));
     }
 }
-template <class A, int LOGQ, int LOGCL>
+template <class A, int LOGQ, int LOGCL, uint32_t E>
 __device__ __forceinline__ void inv_leave(u64* v, const TwRow& tw, const typename A::C& c, const u64* fin) {
-    using G = Geo<LOGQ, LOGCL>;
+    using G = Geo<LOGQ, LOGCL, E>;
     if constexpr (LOGCL > 0) {
         const TwCross<LOGQ, G::LOGN> cross{tw};
 #pragma unroll
@@ -279,19 +278,19 @@ __device__ __forceinline__ void inv_leave(u64* v, const TwRow& tw, const typenam
         }
     }
 }
-template <int LOGQ, int LOGCL>
+template <int LOGQ, int LOGCL, uint32_t E>
 __device__ __forceinline__ u64 leave_x(uint32_t i) {
-    using G = Geo<LOGQ, LOGCL>;
+    using G = Geo<LOGQ, LOGCL, E>;
     return LOGCL ? G::column_x(i) : (u64)threadIdx.x + i * G::T;
 }
 
 // The eight adjacent values of this thread's group g (at 8 (threadIdx.x + g T)
 // in the slice) through the last forward round.
-template <class A, int LOGQ, int LOGCL>
+template <class A, int LOGQ, int LOGCL, uint32_t E>
 __device__ __forceinline__ void fwd_last(typename A::V* v, uint32_t g, const u64* W, const TwRow& tw,
                                          const typename A::C& c) {
-    using G = Geo<LOGQ, LOGCL>;
-    typedef typename KsRound<A, false, LOGQ, 0, 3, G::LOGN>::R R;
+    using G = Geo<LOGQ, LOGCL, E>;
+    typedef typename KsRound<A, false, LOGQ, 0, 3, G::LOGN, E>::R R;
     const typename R::Group gr = R::group(g, G::rank());
     const u64* const sp = W + padix(gr.base_e);
 #pragma unroll
@@ -299,11 +298,11 @@ __device__ __forceinline__ void fwd_last(typename A::V* v, uint32_t g, const u64
     R::run_regs(v, tw, gr.blk, c, nullptr, kEarlier, false);
 }
 // The first inverse round on eight adjacent values, stored to buf.
-template <class A, int LOGQ, int LOGCL>
+template <class A, int LOGQ, int LOGCL, uint32_t E>
 __device__ __forceinline__ void inv_first(typename A::V* v, uint32_t g, u64* buf, const TwRow& tw,
                                           const typename A::C& c) {
-    using G = Geo<LOGQ, LOGCL>;
-    typedef typename KsRound<A, true, LOGQ, 0, 3, G::LOGN>::R R;
+    using G = Geo<LOGQ, LOGCL, E>;
+    typedef typename KsRound<A, true, LOGQ, 0, 3, G::LOGN, E>::R R;
     const typename R::Group gr = R::group(g, G::rank());
     R::run_regs(v, tw, gr.blk, c, nullptr, kEarlier, false);
     u64* const sp = buf + padix(gr.base_e);
@@ -311,9 +310,9 @@ __device__ __forceinline__ void inv_first(typename A::V* v, uint32_t g, u64* buf
     for (uint32_t j = 0; j < 8; ++j) sp[j] = A::store(v[j]);
 }
 // this thread's group g of eight adjacent values, as an offset in a slice
-template <int LOGQ, int LOGCL>
+template <int LOGQ, int LOGCL, uint32_t E>
 __device__ __forceinline__ uint32_t adjacent(uint32_t g) {
-    return padix(8 * (threadIdx.x + g * Geo<LOGQ, LOGCL>::T));
+    return padix(8 * (threadIdx.x + g * Geo<LOGQ, LOGCL, E>::T));
 }
 
 // gathered position of x: the automorphism's source index, or x itself
@@ -374,10 +373,10 @@ struct KeyMul<ArSp> {
 // split constants at tab + 4 i row (any q < 2^61). The products' low words are
 // summed mod 2^64 and the quotient by q in doubles rounded down (sp_mul's form
 // for a sum), so one reduction serves the whole sum: t in [0, q (1 + 2^-6)).
-template <int LOGQ, int LOGCL>
+template <int LOGQ, int LOGCL, uint32_t E>
 __device__ __forceinline__ void bconv8(u64* t, uint32_t g, const u64* src, uint32_t stride, uint32_t size,
                                        const u64* __restrict__ tab, uint32_t row, u64 q) {
-    using G = Geo<LOGQ, LOGCL>;
+    using G = Geo<LOGQ, LOGCL, E>;
     const u64 nq = (u64)0 - q;
     double m[8];
 #pragma unroll
@@ -388,7 +387,7 @@ __device__ __forceinline__ void bconv8(u64* t, uint32_t g, const u64* src, uint3
     // the next limb's values are on their way while this one's are used
     u64 v[8];
 #pragma unroll
-    for (uint32_t e = 0; e < 8; ++e) v[e] = src[leave_x<LOGQ, LOGCL>(8 * g + e)];
+    for (uint32_t e = 0; e < 8; ++e) v[e] = src[leave_x<LOGQ, LOGCL, E>(8 * g + e)];
 #pragma unroll 1
     for (uint32_t i = 0; i < size; ++i) {
         const ulonglong2 w = __ldg((const ulonglong2*)(tab + 4ull * i * row));
@@ -397,7 +396,7 @@ __device__ __forceinline__ void bconv8(u64* t, uint32_t g, const u64* src, uint3
         const u64* const y = src + ((u64)((i + 1 < size ? i + 1 : i) * stride) << G::LOGN);
         u64 nv[8];
 #pragma unroll
-        for (uint32_t e = 0; e < 8; ++e) nv[e] = y[leave_x<LOGQ, LOGCL>(8 * g + e)];
+        for (uint32_t e = 0; e < 8; ++e) nv[e] = y[leave_x<LOGQ, LOGCL, E>(8 * g + e)];
 #pragma unroll
         for (uint32_t e = 0; e < 8; ++e) {
             const uint32_t a0 = (uint32_t)v[e], a1 = (uint32_t)(v[e] >> 32);
@@ -426,9 +425,9 @@ __device__ __forceinline__ u64 bconv_value(u64 t, const ArSp::C&) { return t; }
 
 // The entry a cluster works on. Only its level and table pointer are held;
 // the rest is read again where it is used (registers).
-template <int LOGQ, int LOGCL, bool SINGLE>
+template <int LOGQ, int LOGCL, uint32_t E, bool SINGLE>
 struct Slot {
-    using G = Geo<LOGQ, LOGCL>;
+    using G = Geo<LOGQ, LOGCL, E>;
     const KsFusedArgs& a;
     const OpTabs* tp;
     uint32_t l;
@@ -451,22 +450,22 @@ struct Slot {
 // limbs apart; constants at tab, `row` entries apart) into a forward transform
 // of prime `prime` in slice W, after the wait that an earlier arrive belongs to
 // (wait; not for the second half of a pair).
-template <class A, int LOGQ, int LOGCL>
+template <class A, int LOGQ, int LOGCL, uint32_t E>
 __device__ AFHE_KS_FN void convert_enter(const u64* src, uint32_t stride, uint32_t size, const u64* tab, uint32_t row,
                                            u64* W, const PrimeTables* pt, uint32_t prime, bool wait) {
-    using G = Geo<LOGQ, LOGCL>;
+    using G = Geo<LOGQ, LOGCL, E>;
     const PrimeConst* const pcp = pt->pc + prime;
     const typename A::C c = A::consts(*pcp);
     const TwRow tw = tw_row<false>(*pt, prime, G::LOGN);
 #pragma unroll 1
-    for (uint32_t g = 0; g < kG; ++g) {
+    for (uint32_t g = 0; g < G::KG; ++g) {
         u64 b[8];
-        bconv8<LOGQ, LOGCL>(b, g, src, stride, size, tab, row, pcp->q);
+        bconv8<LOGQ, LOGCL, E>(b, g, src, stride, size, tab, row, pcp->q);
         typename A::V v[8];
 #pragma unroll
         for (uint32_t e = 0; e < 8; ++e) v[e] = bconv_value(b[e], c);
         if (wait && g == 0) G::wait();
-        fwd_enter<A, LOGQ, LOGCL>(v, g, W, tw, c);
+        fwd_enter<A, LOGQ, LOGCL, E>(v, g, W, tw, c);
     }
 }
 
@@ -474,22 +473,22 @@ __device__ AFHE_KS_FN void convert_enter(const u64* src, uint32_t stride, uint32
 // halves (digit's key limb at offset kofs), on groups of eight adjacent
 // positions. Sums go to A0 / A1 (first: nothing there yet), or, with inverse on
 // the last digit, straight through the first inverse round.
-template <class A, int LOGQ, int LOGCL, bool PREP, bool SINGLE>
-__device__ AFHE_KS_FN void last_products(const Slot<LOGQ, LOGCL, SINGLE> S, uint32_t prime, u64 kofs, bool first,
+template <class A, int LOGQ, int LOGCL, uint32_t E, bool PREP, bool SINGLE>
+__device__ AFHE_KS_FN void last_products(const Slot<LOGQ, LOGCL, E, SINGLE> S, uint32_t prime, u64 kofs, bool first,
                                            bool inverse) {
-    using G = Geo<LOGQ, LOGCL>;
+    using G = Geo<LOGQ, LOGCL, E>;
     constexpr int LOGN = G::LOGN;
     const PrimeConst* const pcp = S.pt()->pc + prime;
     const typename A::C c = A::consts(*pcp);
     const EntryKey ek = entry_key(S.a, S.z());
 #pragma unroll 1
-    for (uint32_t g = 0; g < kG; ++g) {
+    for (uint32_t g = 0; g < G::KG; ++g) {
         typename A::V v[8];
-        fwd_last<A, LOGQ, LOGCL>(v, g, S.buf(0), tw_row<false>(*S.pt(), prime, LOGN), c);
+        fwd_last<A, LOGQ, LOGCL, E>(v, g, S.buf(0), tw_row<false>(*S.pt(), prime, LOGN), c);
         const ulonglong2* const kp = ek.prep + kofs + threadIdx.x + g * G::T;
 #pragma unroll
         for (uint32_t h = 0; h < 2; ++h) {
-            u64* const Ah = S.buf(1 + h) + adjacent<LOGQ, LOGCL>(g);
+            u64* const Ah = S.buf(1 + h) + adjacent<LOGQ, LOGCL, E>(g);
             typename A::V p[8];
             if (PREP) {
                 const ulonglong2* const kh = kp + (h ? 0 : S.a.prep_b);
@@ -507,7 +506,7 @@ __device__ AFHE_KS_FN void last_products(const Slot<LOGQ, LOGCL, SINGLE> S, uint
                 for (uint32_t e = 0; e < 8; ++e) p[e] = KeyMul<A>::add(p[e], A::load(Ah[e]), c);
             }
             if (SINGLE || inverse) {
-                inv_first<A, LOGQ, LOGCL>(p, g, S.buf(1 + h), tw_row<true>(*S.pt(), prime, LOGN), c);
+                inv_first<A, LOGQ, LOGCL, E>(p, g, S.buf(1 + h), tw_row<true>(*S.pt(), prime, LOGN), c);
             } else {
 #pragma unroll
                 for (uint32_t e = 0; e < 8; ++e) Ah[e] = A::store(p[e]);
@@ -520,88 +519,88 @@ __device__ AFHE_KS_FN void last_products(const Slot<LOGQ, LOGCL, SINGLE> S, uint
 // limb s - l): BConv of the digit's coefficients, NTT, products. Enters with an
 // arrive that its first store to other CTAs' slices waits for, and leaves with
 // one where W is read last (not with inverse).
-template <class A, int LOGQ, int LOGCL, bool PREP, bool SINGLE>
-__device__ __forceinline__ void digit_slot(const Slot<LOGQ, LOGCL, SINGLE>& S, uint32_t s, uint32_t j, bool first,
+template <class A, int LOGQ, int LOGCL, uint32_t E, bool PREP, bool SINGLE>
+__device__ __forceinline__ void digit_slot(const Slot<LOGQ, LOGCL, E, SINGLE>& S, uint32_t s, uint32_t j, bool first,
                                            bool inverse) {
-    using G = Geo<LOGQ, LOGCL>;
+    using G = Geo<LOGQ, LOGCL, E>;
     const OpTabs& t = S.t();
     const uint32_t l = S.l, K = S.a.K;
     const bool isq = s < l;
     const uint32_t prime = isq ? s : t.p_base + (s - l);
     const uint32_t start = j * t.alpha, size = (j == t.parts - 1) ? l - start : t.alpha;
     const uint32_t kpos = isq ? (s < start ? s : s - size) : (l - size) + (s - l);
-    convert_enter<A, LOGQ, LOGCL>(S.coef(start), 1, size, t.qhat_modp_sp[j] + 4ull * kpos, l - size + K, S.buf(0), S.pt(),
+    convert_enter<A, LOGQ, LOGCL, E>(S.coef(start), 1, size, t.qhat_modp_sp[j] + 4ull * kpos, l - size + K, S.buf(0), S.pt(),
                                   prime, true);
     G::sync_all();
-    fwd_rounds_call<A, LOGQ, LOGCL, 1>(S.buf(0), nullptr, S.pt(), prime);
+    fwd_rounds_call<A, LOGQ, LOGCL, E, 1>(S.buf(0), nullptr, S.pt(), prime);
     const uint32_t klimb = isq ? s : S.a.key_pbase + (s - l);
-    last_products<A, LOGQ, LOGCL, PREP>(S, prime, (((u64)j * S.a.key_stride + klimb) << G::LOGN) + G::rank() * G::QN,
+    last_products<A, LOGQ, LOGCL, E, PREP>(S, prime, (((u64)j * S.a.key_stride + klimb) << G::LOGN) + G::rank() * G::QN,
                                         first, inverse);
     if (!(SINGLE || inverse)) G::arrive();
 }
 
 // Phase 0, limb i: coef[i] = INTT(input through the automorphism) * qHatInv.
-template <class A, int LOGQ, int LOGCL, bool SINGLE>
-__device__ AFHE_KS_FN void input_limb(const Slot<LOGQ, LOGCL, SINGLE> S, uint32_t i, u64* buf) {
-    using G = Geo<LOGQ, LOGCL>;
+template <class A, int LOGQ, int LOGCL, uint32_t E, bool SINGLE>
+__device__ AFHE_KS_FN void input_limb(const Slot<LOGQ, LOGCL, E, SINGLE> S, uint32_t i, u64* buf) {
+    using G = Geo<LOGQ, LOGCL, E>;
     constexpr int LOGN = G::LOGN;
     const u64* src = S.in() + ((u64)i << LOGN);
     {
         const uint32_t* const map = entry_key(S.a, S.z()).map;
-        uint32_t g[kE];
-        u64 x[kE];
+        uint32_t g[E];
+        u64 x[E];
 #pragma unroll
-        for (uint32_t e = 0; e < kE; ++e) g[e] = gpos(map, G::rank() * G::QN + (uint32_t)G::lpos(e));
+        for (uint32_t e = 0; e < E; ++e) g[e] = gpos(map, G::rank() * G::QN + (uint32_t)G::lpos(e));
 #pragma unroll
-        for (uint32_t e = 0; e < kE; ++e) x[e] = src[g[e]];
-        residues<kE, A::kSecond>(x, S.pt()->pc[i]);
+        for (uint32_t e = 0; e < E; ++e) x[e] = src[g[e]];
+        residues<E, A::kSecond>(x, S.pt()->pc[i]);
 #pragma unroll
-        for (uint32_t e = 0; e < kE; ++e) buf[G::spos(e)] = A::store(A::of(x[e]));
+        for (uint32_t e = 0; e < E; ++e) buf[G::spos(e)] = A::store(A::of(x[e]));
     }
     __syncthreads();
     const typename A::C c = A::consts(S.pt()->pc[i]);
     const TwRow tw = tw_row<true>(*S.pt(), i, LOGN);
     const u64* const fin = S.t().fin_q + 8ull * i;
 #pragma unroll 1
-    for (uint32_t g = 0; g < kG; ++g) {
+    for (uint32_t g = 0; g < G::KG; ++g) {
         typename A::V v[8];
-        const u64* const sp = buf + adjacent<LOGQ, LOGCL>(g);
+        const u64* const sp = buf + adjacent<LOGQ, LOGCL, E>(g);
 #pragma unroll
         for (uint32_t e = 0; e < 8; ++e) v[e] = A::load(sp[e]);
-        inv_first<A, LOGQ, LOGCL>(v, g, buf, tw, c);
+        inv_first<A, LOGQ, LOGCL, E>(v, g, buf, tw, c);
     }
-    inv_rounds_call<A, LOGQ, LOGCL, 1>(buf, nullptr, S.pt(), i, fin);
+    inv_rounds_call<A, LOGQ, LOGCL, E, 1>(buf, nullptr, S.pt(), i, fin);
     G::sync_all();
     u64* const dst = S.coef(i);
-    u64 v[kE];
+    u64 v[E];
 #pragma unroll
-    for (uint32_t g = 0; g < kG; ++g) inv_gather<LOGQ, LOGCL>(v + 8 * g, g, buf);
+    for (uint32_t g = 0; g < G::KG; ++g) inv_gather<LOGQ, LOGCL, E>(v + 8 * g, g, buf);
 #pragma unroll
-    for (uint32_t g = 0; g < kG; ++g) {
-        inv_leave<A, LOGQ, LOGCL>(v + 8 * g, tw, c, fin);
+    for (uint32_t g = 0; g < G::KG; ++g) {
+        inv_leave<A, LOGQ, LOGCL, E>(v + 8 * g, tw, c, fin);
 #pragma unroll
-        for (uint32_t e = 0; e < 8; ++e) dst[leave_x<LOGQ, LOGCL>(8 * g + e)] = v[8 * g + e];
+        for (uint32_t e = 0; e < 8; ++e) dst[leave_x<LOGQ, LOGCL, E>(8 * g + e)] = v[8 * g + e];
     }
 }
 
 // The end of both sums' inverse transforms at special slot k, to the scratch.
-template <class A, int LOGQ, int LOGCL, bool SINGLE>
-__device__ AFHE_KS_FN void leave_sums(const Slot<LOGQ, LOGCL, SINGLE> S, uint32_t k, const u64* fin) {
-    using G = Geo<LOGQ, LOGCL>;
+template <class A, int LOGQ, int LOGCL, uint32_t E, bool SINGLE>
+__device__ AFHE_KS_FN void leave_sums(const Slot<LOGQ, LOGCL, E, SINGLE> S, uint32_t k, const u64* fin) {
+    using G = Geo<LOGQ, LOGCL, E>;
     const uint32_t prime = S.t().p_base + k;
     const typename A::C c = A::consts(S.pt()->pc[prime]);
     const TwRow tw = tw_row<true>(*S.pt(), prime, G::LOGN);
     // the next eight positions are on their way while these are transformed
     u64 v[8], nv[8];
-    inv_gather<LOGQ, LOGCL>(v, 0, S.buf(1));
+    inv_gather<LOGQ, LOGCL, E>(v, 0, S.buf(1));
 #pragma unroll 1
-    for (uint32_t g = 0; g < 2 * kG; ++g) {
-        if (g + 1 < 2 * kG) inv_gather<LOGQ, LOGCL>(nv, (g + 1) >> 1, S.buf(1 + ((g + 1) & 1)));
-        inv_leave<A, LOGQ, LOGCL>(v, tw, c, fin);
+    for (uint32_t g = 0; g < 2 * G::KG; ++g) {
+        if (g + 1 < 2 * G::KG) inv_gather<LOGQ, LOGCL, E>(nv, (g + 1) >> 1, S.buf(1 + ((g + 1) & 1)));
+        inv_leave<A, LOGQ, LOGCL, E>(v, tw, c, fin);
         u64* const dst = S.coef(S.l + 2 * k + (g & 1));
 #pragma unroll
         for (uint32_t e = 0; e < 8; ++e) {
-            dst[leave_x<LOGQ, LOGCL>(8 * (g >> 1) + e)] = v[e];
+            dst[leave_x<LOGQ, LOGCL, E>(8 * (g >> 1) + e)] = v[e];
             v[e] = nv[e];
         }
     }
@@ -609,23 +608,23 @@ __device__ AFHE_KS_FN void leave_sums(const Slot<LOGQ, LOGCL, SINGLE> S, uint32_
 
 // Phase 1, special slot k: both sums' coefficients times PHatInv -> scratch.
 // Enters and leaves with an arrive (see digit_slot).
-template <class A, int LOGQ, int LOGCL, bool PREP, bool SINGLE>
-__device__ __forceinline__ void special_slot(const Slot<LOGQ, LOGCL, SINGLE>& S, uint32_t k) {
-    using G = Geo<LOGQ, LOGCL>;
+template <class A, int LOGQ, int LOGCL, uint32_t E, bool PREP, bool SINGLE>
+__device__ __forceinline__ void special_slot(const Slot<LOGQ, LOGCL, E, SINGLE>& S, uint32_t k) {
+    using G = Geo<LOGQ, LOGCL, E>;
     constexpr int LOGN = G::LOGN;
     const OpTabs& t = S.t();
     const uint32_t prime = t.p_base + k;
     if (SINGLE) {
-        digit_slot<A, LOGQ, LOGCL, PREP>(S, S.l + k, 0, true, true);
+        digit_slot<A, LOGQ, LOGCL, E, PREP>(S, S.l + k, 0, true, true);
     } else {
 #pragma unroll 1
         for (uint32_t j = 0; j < t.parts; ++j)
-            digit_slot<A, LOGQ, LOGCL, PREP>(S, S.l + k, j, j == 0, j + 1 == t.parts);
+            digit_slot<A, LOGQ, LOGCL, E, PREP>(S, S.l + k, j, j == 0, j + 1 == t.parts);
     }
     const u64* const fin = t.fin_p + 8ull * k;
-    inv_rounds_call<A, LOGQ, LOGCL, 2>(S.buf(1), S.buf(2), S.pt(), prime, fin);
+    inv_rounds_call<A, LOGQ, LOGCL, E, 2>(S.buf(1), S.buf(2), S.pt(), prime, fin);
     G::sync_all();
-    leave_sums<A, LOGQ, LOGCL>(S, k, fin);
+    leave_sums<A, LOGQ, LOGCL, E>(S, k, fin);
     G::arrive();
 }
 
@@ -647,13 +646,13 @@ __device__ __forceinline__ u64 moddown_value(u64 s, u64 y, const ulonglong2& pin
 // halves, c0 joining the first as c0 P (it comes out of the product with P^-1).
 // OwnGather reads input and c0 at lpos(e0) .. lpos(e0 + 7) through the
 // automorphism, own_products makes the products of four of them.
-template <class A, int LOGQ, int LOGCL>
+template <class A, int LOGQ, int LOGCL, uint32_t E>
 struct OwnGather {
     u64 d[8], cv[8];
     template <bool SINGLE>
-    __device__ __forceinline__ void load(const Slot<LOGQ, LOGCL, SINGLE>& S, const EntryKey& ek, uint32_t i,
+    __device__ __forceinline__ void load(const Slot<LOGQ, LOGCL, E, SINGLE>& S, const EntryKey& ek, uint32_t i,
                                          uint32_t e0) {
-        using G = Geo<LOGQ, LOGCL>;
+        using G = Geo<LOGQ, LOGCL, E>;
         const KsFusedArgs& a = S.a;
         const u64* const src = S.in() + ((u64)i << G::LOGN);
         const u64* const cb = a.arena + (a.f.has_c0 ? a.f.c0.at(S.z()) : 0) + ((u64)i << G::LOGN);
@@ -671,11 +670,11 @@ struct OwnGather {
         }
     }
 };
-template <class A, int LOGQ, int LOGCL, bool PREP, bool SINGLE>
-__device__ __forceinline__ void own_products(const Slot<LOGQ, LOGCL, SINGLE>& S, const EntryKey& ek, uint32_t i,
+template <class A, int LOGQ, int LOGCL, uint32_t E, bool PREP, bool SINGLE>
+__device__ __forceinline__ void own_products(const Slot<LOGQ, LOGCL, E, SINGLE>& S, const EntryKey& ek, uint32_t i,
                                              uint32_t e0, const u64* d, const u64* cv, typename A::V* p0,
                                              typename A::V* p1, const typename A::C& c) {
-    using G = Geo<LOGQ, LOGCL>;
+    using G = Geo<LOGQ, LOGCL, E>;
     const KsFusedArgs& a = S.a;
     const OpTabs& t = S.t();
     const u64 kofs = ((((u64)(i / t.alpha) * a.key_stride + i) << G::LOGN) + G::rank() * G::QN) + threadIdx.x;
@@ -711,40 +710,40 @@ __device__ __forceinline__ void own_products(const Slot<LOGQ, LOGCL, SINGLE>& S,
 
 // BConv of the special limbs of sum h to q_i (approx_mod_down's
 // fast_bases_conv) into a forward transform.
-template <class A, int LOGQ, int LOGCL, bool SINGLE>
-__device__ __forceinline__ void moddown_enter(const Slot<LOGQ, LOGCL, SINGLE>& S, uint32_t i, uint32_t h, u64* W,
+template <class A, int LOGQ, int LOGCL, uint32_t E, bool SINGLE>
+__device__ __forceinline__ void moddown_enter(const Slot<LOGQ, LOGCL, E, SINGLE>& S, uint32_t i, uint32_t h, u64* W,
                                               bool wait) {
-    convert_enter<A, LOGQ, LOGCL>(S.coef(S.l + h), 2, S.a.K, S.t().phat_modq_sp + 4ull * i, S.l, W, S.pt(), i, wait);
+    convert_enter<A, LOGQ, LOGCL, E>(S.coef(S.l + h), 2, S.a.K, S.t().phat_modq_sp + 4ull * i, S.l, W, S.pt(), i, wait);
 }
 // the last round of a buffer, back in place
-template <class A, int LOGQ, int LOGCL>
+template <class A, int LOGQ, int LOGCL, uint32_t E>
 __device__ AFHE_KS_FN void fwd_finish(u64* W, const PrimeTables* pt, uint32_t prime) {
     const TwRow tw = tw_row<false>(*pt, prime, LOGQ + LOGCL);
     const typename A::C c = A::consts(pt->pc[prime]);
 #pragma unroll 1
-    for (uint32_t g = 0; g < kG; ++g) {
+    for (uint32_t g = 0; g < Geo<LOGQ, LOGCL, E>::KG; ++g) {
         typename A::V v[8];
-        fwd_last<A, LOGQ, LOGCL>(v, g, W, tw, c);
-        u64* const sp = W + adjacent<LOGQ, LOGCL>(g);
+        fwd_last<A, LOGQ, LOGCL, E>(v, g, W, tw, c);
+        u64* const sp = W + adjacent<LOGQ, LOGCL, E>(g);
 #pragma unroll
         for (uint32_t e = 0; e < 8; ++e) sp[e] = A::store(v[e]);
     }
 }
 
 // The own digit's products at Q limb i, to A0 / A1.
-template <class A, int LOGQ, int LOGCL, bool PREP>
-__device__ AFHE_KS_FN void own_sums(const Slot<LOGQ, LOGCL, false> S, uint32_t i) {
-    using G = Geo<LOGQ, LOGCL>;
+template <class A, int LOGQ, int LOGCL, uint32_t E, bool PREP>
+__device__ AFHE_KS_FN void own_sums(const Slot<LOGQ, LOGCL, E, false> S, uint32_t i) {
+    using G = Geo<LOGQ, LOGCL, E>;
     const typename A::C c = A::consts(S.pt()->pc[i]);
     const EntryKey ek = entry_key(S.a, S.z());
 #pragma unroll 1
-    for (uint32_t e0 = 0; e0 < kE; e0 += 8) {
-        OwnGather<A, LOGQ, LOGCL> og;
+    for (uint32_t e0 = 0; e0 < E; e0 += 8) {
+        OwnGather<A, LOGQ, LOGCL, E> og;
         og.load(S, ek, i, e0);
 #pragma unroll
         for (uint32_t f = 0; f < 8; f += 4) {
             typename A::V p0[4], p1[4];
-            own_products<A, LOGQ, LOGCL, PREP>(S, ek, i, e0 + f, og.d + f, og.cv + f, p0, p1, c);
+            own_products<A, LOGQ, LOGCL, E, PREP>(S, ek, i, e0 + f, og.d + f, og.cv + f, p0, p1, c);
 #pragma unroll
             for (uint32_t e = 0; e < 4; ++e) {
                 S.buf(1)[G::spos(e0 + f + e)] = A::store(p0[e]);
@@ -754,9 +753,9 @@ __device__ AFHE_KS_FN void own_sums(const Slot<LOGQ, LOGCL, false> S, uint32_t i
     }
 }
 // ModDown combine of half h at Q limb i, to the output.
-template <class A, int LOGQ, int LOGCL>
-__device__ AFHE_KS_FN void combine_half(const Slot<LOGQ, LOGCL, false> S, uint32_t i, uint32_t h) {
-    using G = Geo<LOGQ, LOGCL>;
+template <class A, int LOGQ, int LOGCL, uint32_t E>
+__device__ AFHE_KS_FN void combine_half(const Slot<LOGQ, LOGCL, E, false> S, uint32_t i, uint32_t h) {
+    using G = Geo<LOGQ, LOGCL, E>;
     const KsFusedArgs& a = S.a;
     const typename A::C c = A::consts(S.pt()->pc[i]);
     const u64 q = S.pt()->pc[i].q;
@@ -766,7 +765,7 @@ __device__ AFHE_KS_FN void combine_half(const Slot<LOGQ, LOGCL, false> S, uint32
     const ulonglong2* const pi = (const ulonglong2*)(S.t().p_inv_tc + 4ull * i);
     const ulonglong2 pi0 = __ldg(pi), pi1 = A::kSecond ? __ldg(pi + 1) : ulonglong2{};
 #pragma unroll 1
-    for (uint32_t e0 = 0; e0 < kE; e0 += 8) {
+    for (uint32_t e0 = 0; e0 < E; e0 += 8) {
         u64 ex[8];
 #pragma unroll
         for (uint32_t e = 0; e < 8; ++e) ex[e] = a.f.has_acc ? acc[(e0 + e) * G::T] : 0;
@@ -779,45 +778,45 @@ __device__ AFHE_KS_FN void combine_half(const Slot<LOGQ, LOGCL, false> S, uint32
 }
 
 // Phase 2, Q limb i. Enters and leaves with an arrive (see digit_slot).
-template <class A, int LOGQ, int LOGCL, bool PREP>
-__device__ __forceinline__ void output_limb(const Slot<LOGQ, LOGCL, false>& S, uint32_t i) {
-    using G = Geo<LOGQ, LOGCL>;
+template <class A, int LOGQ, int LOGCL, uint32_t E, bool PREP>
+__device__ __forceinline__ void output_limb(const Slot<LOGQ, LOGCL, E, false>& S, uint32_t i) {
+    using G = Geo<LOGQ, LOGCL, E>;
     const uint32_t own = i / S.t().alpha, parts = S.t().parts;
-    own_sums<A, LOGQ, LOGCL, PREP>(S, i);
+    own_sums<A, LOGQ, LOGCL, E, PREP>(S, i);
     // (the barriers of the next transform come before the sums are read)
 #pragma unroll 1
     for (uint32_t j = 0; j < parts; ++j)
-        if (j != own) digit_slot<A, LOGQ, LOGCL, PREP>(S, i, j, false, false);
+        if (j != own) digit_slot<A, LOGQ, LOGCL, E, PREP>(S, i, j, false, false);
 #pragma unroll 1
     for (uint32_t h = 0; h < 2; ++h) {
-        moddown_enter<A, LOGQ, LOGCL>(S, i, h, S.buf(0), true);
+        moddown_enter<A, LOGQ, LOGCL, E>(S, i, h, S.buf(0), true);
         G::sync_all();
-        fwd_rounds_call<A, LOGQ, LOGCL, 1>(S.buf(0), nullptr, S.pt(), i);
-        fwd_finish<A, LOGQ, LOGCL>(S.buf(0), S.pt(), i);
+        fwd_rounds_call<A, LOGQ, LOGCL, E, 1>(S.buf(0), nullptr, S.pt(), i);
+        fwd_finish<A, LOGQ, LOGCL, E>(S.buf(0), S.pt(), i);
         __syncthreads();
-        combine_half<A, LOGQ, LOGCL>(S, i, h);
+        combine_half<A, LOGQ, LOGCL, E>(S, i, h);
         G::arrive();
     }
 }
 
 // The combine of both halves with a single digit: the limb's own products are
 // formed here (input and c0 gathered once), the results stay in the slices.
-template <class A, int LOGQ, int LOGCL, bool PREP>
-__device__ AFHE_KS_FN void combine_both(const Slot<LOGQ, LOGCL, true> S, uint32_t i) {
-    using G = Geo<LOGQ, LOGCL>;
+template <class A, int LOGQ, int LOGCL, uint32_t E, bool PREP>
+__device__ AFHE_KS_FN void combine_both(const Slot<LOGQ, LOGCL, E, true> S, uint32_t i) {
+    using G = Geo<LOGQ, LOGCL, E>;
     const typename A::C c = A::consts(S.pt()->pc[i]);
     const u64 q = S.pt()->pc[i].q;
     const EntryKey ek = entry_key(S.a, S.z());
     const ulonglong2* const pi = (const ulonglong2*)(S.t().p_inv_tc + 4ull * i);
     const ulonglong2 pi0 = __ldg(pi), pi1 = A::kSecond ? __ldg(pi + 1) : ulonglong2{};
 #pragma unroll 1
-    for (uint32_t e0 = 0; e0 < kE; e0 += 8) {
-        OwnGather<A, LOGQ, LOGCL> og;
+    for (uint32_t e0 = 0; e0 < E; e0 += 8) {
+        OwnGather<A, LOGQ, LOGCL, E> og;
         og.load(S, ek, i, e0);
 #pragma unroll
         for (uint32_t f = 0; f < 8; f += 4) {
             typename A::V p0[4], p1[4];
-            own_products<A, LOGQ, LOGCL, PREP>(S, ek, i, e0 + f, og.d + f, og.cv + f, p0, p1, c);
+            own_products<A, LOGQ, LOGCL, E, PREP>(S, ek, i, e0 + f, og.d + f, og.cv + f, p0, p1, c);
 #pragma unroll
             for (uint32_t e = 0; e < 4; ++e) {
                 u64& r0 = S.buf(1)[G::spos(e0 + f + e)];
@@ -828,9 +827,9 @@ __device__ AFHE_KS_FN void combine_both(const Slot<LOGQ, LOGCL, true> S, uint32_
         }
     }
 }
-template <int LOGQ, int LOGCL>
-__device__ AFHE_KS_FN void store_both(const Slot<LOGQ, LOGCL, true> S, uint32_t i) {
-    using G = Geo<LOGQ, LOGCL>;
+template <int LOGQ, int LOGCL, uint32_t E>
+__device__ AFHE_KS_FN void store_both(const Slot<LOGQ, LOGCL, E, true> S, uint32_t i) {
+    using G = Geo<LOGQ, LOGCL, E>;
     const KsFusedArgs& a = S.a;
     const u64 q = S.pt()->pc[i].q;
     const u64 x0 = ((u64)i << G::LOGN) + G::rank() * G::QN + threadIdx.x;
@@ -839,7 +838,7 @@ __device__ AFHE_KS_FN void store_both(const Slot<LOGQ, LOGCL, true> S, uint32_t 
         u64* const out = a.arena + (h ? a.out1 : a.out0).at(S.z()) + x0;
         const u64* const acc = a.arena + (a.f.has_acc ? (h ? a.f.acc1 : a.f.acc0).at(S.z()) + x0 : 0);
 #pragma unroll 1
-        for (uint32_t e0 = 0; e0 < kE; e0 += 8) {
+        for (uint32_t e0 = 0; e0 < E; e0 += 8) {
             u64 ex[8];
 #pragma unroll
             for (uint32_t e = 0; e < 8; ++e) ex[e] = a.f.has_acc ? acc[(e0 + e) * G::T] : 0;
@@ -855,17 +854,17 @@ __device__ AFHE_KS_FN void store_both(const Slot<LOGQ, LOGCL, true> S, uint32_t 
 // Phase 2 with a single digit: both halves' transforms side by side in the two
 // slices. The outputs wait in the slices for a barrier over the polynomial's
 // CTAs, since they may lie where another CTA gathers from.
-template <class A, int LOGQ, int LOGCL, bool PREP>
-__device__ __forceinline__ void output_limb(const Slot<LOGQ, LOGCL, true>& S, uint32_t i) {
-    using G = Geo<LOGQ, LOGCL>;
-    moddown_enter<A, LOGQ, LOGCL>(S, i, 0, S.buf(1), true);
-    moddown_enter<A, LOGQ, LOGCL>(S, i, 1, S.buf(2), false);
+template <class A, int LOGQ, int LOGCL, uint32_t E, bool PREP>
+__device__ __forceinline__ void output_limb(const Slot<LOGQ, LOGCL, E, true>& S, uint32_t i) {
+    using G = Geo<LOGQ, LOGCL, E>;
+    moddown_enter<A, LOGQ, LOGCL, E>(S, i, 0, S.buf(1), true);
+    moddown_enter<A, LOGQ, LOGCL, E>(S, i, 1, S.buf(2), false);
     G::sync_all();
-    fwd_rounds_call<A, LOGQ, LOGCL, 2>(S.buf(1), S.buf(2), S.pt(), i);
-    fwd_finish<A, LOGQ, LOGCL>(S.buf(1), S.pt(), i);
-    fwd_finish<A, LOGQ, LOGCL>(S.buf(2), S.pt(), i);
+    fwd_rounds_call<A, LOGQ, LOGCL, E, 2>(S.buf(1), S.buf(2), S.pt(), i);
+    fwd_finish<A, LOGQ, LOGCL, E>(S.buf(1), S.pt(), i);
+    fwd_finish<A, LOGQ, LOGCL, E>(S.buf(2), S.pt(), i);
     __syncthreads();
-    combine_both<A, LOGQ, LOGCL, PREP>(S, i);
+    combine_both<A, LOGQ, LOGCL, E, PREP>(S, i);
     G::sync_all();
     store_both(S, i);
     G::arrive();
@@ -876,29 +875,29 @@ __device__ __forceinline__ void output_limb(const Slot<LOGQ, LOGCL, true>& S, ui
 // thread): three of SINGLE's would fit the shared memory, but at 80 registers
 // the split arithmetic spills and the L1 that is left no longer holds the
 // twiddles (N = 2^15, 2 + 4 limbs, 240 ciphertexts: 2.87 ms against 2.34).
-inline constexpr int ks_min_ctas(int logq) { return (int)(512u / ((1u << logq) / kE)); }
+inline constexpr int ks_min_ctas(uint32_t threads) { return (int)(512u / threads); }
 
-template <int LOGQ, int LOGCL, bool PREP, bool SINGLE>
-__global__ void __launch_bounds__((1u << LOGQ) / kE, ks_min_ctas(LOGQ))
+template <int LOGQ, int LOGCL, uint32_t E, bool PREP, bool SINGLE>
+__global__ void __launch_bounds__(Geo<LOGQ, LOGCL, E>::T, ks_min_ctas(Geo<LOGQ, LOGCL, E>::T))
     ks_fused_kernel(const __grid_constant__ KsFusedArgs a) {
-    using G = Geo<LOGQ, LOGCL>;
+    using G = Geo<LOGQ, LOGCL, E>;
     const uint32_t l = a.mixed ? (uint32_t)a.lvz.at(blockIdx.x >> LOGCL) : a.sizeQl;
-    const Slot<LOGQ, LOGCL, SINGLE> S{a, a.lvtabs + l, l};
+    const Slot<LOGQ, LOGCL, E, SINGLE> S{a, a.lvtabs + l, l};
     const OpTabs& t = S.t();
     // limbs alternate between two slices: a limb's gather from every CTA may
     // still run while the next one is loaded
 #pragma unroll 1
     for (uint32_t i = 0; i < l; ++i) {
         u64* const buf = S.buf(1 + (i & 1));
-        if (S.pt()->pc[i].fp) input_limb<ArFp, LOGQ, LOGCL>(S, i, buf);
-        else input_limb<ArSp, LOGQ, LOGCL>(S, i, buf);
+        if (S.pt()->pc[i].fp) input_limb<ArFp, LOGQ, LOGCL, E>(S, i, buf);
+        else input_limb<ArSp, LOGQ, LOGCL, E>(S, i, buf);
     }
     G::arrive();
     // a thread reads back only the coefficients it stored itself
 #pragma unroll 1
     for (uint32_t k = 0; k < a.K; ++k) {
-        if (S.pt()->pc[t.p_base + k].fp) special_slot<ArFp, LOGQ, LOGCL, PREP>(S, k);
-        else special_slot<ArSp, LOGQ, LOGCL, PREP>(S, k);
+        if (S.pt()->pc[t.p_base + k].fp) special_slot<ArFp, LOGQ, LOGCL, E, PREP>(S, k);
+        else special_slot<ArSp, LOGQ, LOGCL, E, PREP>(S, k);
     }
     if constexpr (!SINGLE) {        // A0 / A1 are written before the next wait: the last gathers from them
         G::wait();
@@ -906,8 +905,8 @@ __global__ void __launch_bounds__((1u << LOGQ) / kE, ks_min_ctas(LOGQ))
     }
 #pragma unroll 1
     for (uint32_t i = 0; i < l; ++i) {
-        if (S.pt()->pc[i].fp) output_limb<ArFp, LOGQ, LOGCL, PREP>(S, i);
-        else output_limb<ArSp, LOGQ, LOGCL, PREP>(S, i);
+        if (S.pt()->pc[i].fp) output_limb<ArFp, LOGQ, LOGCL, E, PREP>(S, i);
+        else output_limb<ArSp, LOGQ, LOGCL, E, PREP>(S, i);
     }
     G::wait();
 }
@@ -915,10 +914,10 @@ __global__ void __launch_bounds__((1u << LOGQ) / kE, ks_min_ctas(LOGQ))
 template <int LOGQ, bool SINGLE>
 constexpr size_t fused_smem() { return (SINGLE ? 2ull : 3ull) * ((1u << LOGQ) + (1u << LOGQ) / 16) * sizeof(u64); }
 
-template <int LOGQ, int LOGCL, bool PREP, bool SINGLE>
+template <int LOGQ, int LOGCL, uint32_t E, bool PREP, bool SINGLE>
 cudaError_t launch_fused_v(const KsFusedArgs& a, uint32_t nz, cudaStream_t st) {
-    constexpr uint32_t T = Geo<LOGQ, LOGCL>::T;
-    auto kern = ks_fused_kernel<LOGQ, LOGCL, PREP, SINGLE>;
+    constexpr uint32_t T = Geo<LOGQ, LOGCL, E>::T;
+    auto kern = ks_fused_kernel<LOGQ, LOGCL, E, PREP, SINGLE>;
     constexpr size_t smem = fused_smem<LOGQ, SINGLE>();
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
@@ -942,6 +941,19 @@ cudaError_t launch_fused_v(const KsFusedArgs& a, uint32_t nz, cudaStream_t st) {
     }
     count_launches(1);
     return cudaGetLastError();
+}
+
+// Values per thread: sixteen. Where one CTA carries a ciphertext, eight in launches of
+// up to half a wave: as many CTAs as fit at once then have twice the threads, and a
+// thread half the chain (rotations, us, 16 / 8: N = 2^10, three digits, 120: 120 / 65;
+// N = 2^11, two, 74: 88 / 56; N = 2^12, three, 148: 189 / 135; past half a wave, N =
+// 2^12, 260: 261 / 304, N = 2^11, two, 592: 150 / 160).
+template <int LOGQ, int LOGCL, bool PREP, bool SINGLE>
+cudaError_t launch_fused(const KsFusedArgs& a, uint32_t nz, cudaStream_t st) {
+    if constexpr (LOGCL == 0) {
+        if (2 * nz <= (uint32_t)key_switch_fused_capacity(LOGQ)) return launch_fused_v<LOGQ, LOGCL, 8, PREP, SINGLE>(a, nz, st);
+    }
+    return launch_fused_v<LOGQ, LOGCL, 16, PREP, SINGLE>(a, nz, st);
 }
 
 // Launches by ring degree, one source file each (ksfused_single.cu, _multi.cu,

@@ -5,7 +5,7 @@ namespace afhe {
 namespace ksf {
 
 cudaError_t launch_multi(int log_n, const KsFusedArgs& a, uint32_t nz, cudaStream_t st) {
-#define LAUNCH(Q, C) launch_fused_v<Q, C, true, false>(a, nz, st)
+#define LAUNCH(Q, C) launch_fused<Q, C, true, false>(a, nz, st)
     AFHE_KS_BY_DEGREE(log_n, LAUNCH, cudaErrorInvalidValue)
 #undef LAUNCH
 }
@@ -15,9 +15,9 @@ namespace {
 // (0 when it cannot place even one: the multi-kernel path is used then).
 template <int LOGQ, int LOGCL>
 int fused_capacity() {
-    auto kern = ks_fused_kernel<LOGQ, LOGCL, true, false>;
+    auto kern = ks_fused_kernel<LOGQ, LOGCL, 16, true, false>;
     constexpr size_t smem = fused_smem<LOGQ, false>();
-    constexpr uint32_t T = Geo<LOGQ, LOGCL>::T;
+    constexpr uint32_t T = Geo<LOGQ, LOGCL, 16>::T;
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
         cudaGetLastError();
         return 0;

@@ -7,7 +7,7 @@ namespace afhe {
 namespace ksf {
 
 cudaError_t launch_raw(int log_n, const KsFusedArgs& a, uint32_t nz, cudaStream_t st) {
-#define LAUNCH(Q, C) launch_fused_v<Q, C, false, false>(a, nz, st)
+#define LAUNCH(Q, C) launch_fused<Q, C, false, false>(a, nz, st)
     AFHE_KS_BY_DEGREE(log_n, LAUNCH, cudaErrorInvalidValue)
 #undef LAUNCH
 }

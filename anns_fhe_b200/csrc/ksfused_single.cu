@@ -5,7 +5,7 @@ namespace afhe {
 namespace ksf {
 
 cudaError_t launch_single(int log_n, const KsFusedArgs& a, uint32_t nz, cudaStream_t st) {
-#define LAUNCH(Q, C) launch_fused_v<Q, C, true, true>(a, nz, st)
+#define LAUNCH(Q, C) launch_fused<Q, C, true, true>(a, nz, st)
     AFHE_KS_BY_DEGREE(log_n, LAUNCH, cudaErrorInvalidValue)
 #undef LAUNCH
 }

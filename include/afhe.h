@@ -195,9 +195,8 @@ int afhe_copy_poly(afhe_ctx* ctx, uint64_t dst_offset, uint64_t src_offset, uint
  *                      what is left of a larger launch after whole waves
  *                      (AFHE_OPT_KS_CAPACITY) where a wave of its own would take
  *                      longer; 1: every launch is one kernel. The default (half
- *                      a wave of SMs, by one CTA per 2^13 coefficients) stands,
- *                      from N = 2^13 on, for a line drawn by level. Same
- *                      residues. */
+ *                      a wave of SMs, by one CTA per 2^13 coefficients) stands
+ *                      for a line drawn by level. Same residues. */
 #define AFHE_OPT_FUSED_MIN 3u
 /*   AFHE_OPT_KS_CAPACITY (read only) ciphertexts the one-kernel key switch
  *                      runs at once on this GPU (CTAs, or clusters above
