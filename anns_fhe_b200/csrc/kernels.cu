@@ -27,30 +27,31 @@ void set_ntt_plan(int log_n, int plan) { g_ntt_plan[log_n].store(plan, std::memo
 // ---------------------------------------------------------------------------
 // elementwise
 // ---------------------------------------------------------------------------
-// Four coefficients a thread, 256 apart: the loads of all are on their way
+// PER coefficients a thread, 256 apart: the loads of all are on their way
 // before the first is used. Products of primes below 2^50 in doubles (10 FP64
 // instructions in place of about 95 multiplier cycles for the 128-bit product
-// and its reduction).
-constexpr uint32_t kEwPer = 4;
-template <int OP>
+// and its reduction). Four a thread, or one in launches of few words, which four in a
+// row take longer than the launch itself (products of one limb one after another,
+// N = 2^11, us, four / one: 60 bits 4.1 / 3.4, 50 bits 4.1 / 3.3; of 2^17 words 4.1 both).
+template <int OP, uint32_t PER>
 __global__ void __launch_bounds__(256) elementwise_kernel(const PrimeConst* __restrict__ pc, uint32_t prime0,
                                                           u64* __restrict__ arena, uint32_t n, const ZBases zb) {
     const uint32_t l = blockIdx.y, z = blockIdx.z;
     const PrimeConst p = pc[prime0 + l];
-    const uint32_t i0 = blockIdx.x * (256 * kEwPer) + threadIdx.x;
+    const uint32_t i0 = blockIdx.x * (256 * PER) + threadIdx.x;
     const u64 off = (u64)l * n + i0;
     const u64* a = arena + zb.src.at(z) + off;
     const u64* b = arena + zb.aux.at(z) + off;
     u64* o = arena + zb.out.at(z) + off;
-    u64 x[kEwPer], y[kEwPer];
+    u64 x[PER], y[PER];
 #pragma unroll
-    for (uint32_t k = 0; k < kEwPer; ++k) {
+    for (uint32_t k = 0; k < PER; ++k) {
         const bool in = i0 + 256 * k < n;
         x[k] = in ? a[256 * k] : 0;
         y[k] = OP != EW_COPY && in ? b[256 * k] : 0;
     }
 #pragma unroll
-    for (uint32_t k = 0; k < kEwPer; ++k) {
+    for (uint32_t k = 0; k < PER; ++k) {
         u64 r = x[k];
         if (OP == EW_ADD) r = add_mod(x[k], y[k], p.q);
         else if (OP == EW_SUB) r = sub_mod(x[k], y[k], p.q);
@@ -59,15 +60,25 @@ __global__ void __launch_bounds__(256) elementwise_kernel(const PrimeConst* __re
     }
 }
 
+constexpr u64 kEwFew = 1u << 16;     // words
+template <int OP>
+void launch_ew(bool few, const PrimeConst* pc, uint32_t prime0, u64* arena, uint32_t n, uint32_t limbs, uint32_t nz,
+               const ZBases& zb, cudaStream_t st) {
+    const uint32_t per = few ? 256 : 256 * 4;
+    const dim3 grid((n + per - 1) / per, limbs, nz);
+    if (few) elementwise_kernel<OP, 1><<<grid, 256, 0, st>>>(pc, prime0, arena, n, zb);
+    else elementwise_kernel<OP, 4><<<grid, 256, 0, st>>>(pc, prime0, arena, n, zb);
+}
+
 cudaError_t launch_elementwise(ElemOp op, const PrimeConst* pc, uint32_t prime0, u64* arena, uint32_t n,
                                uint32_t limbs, uint32_t nz, const ZBases& zb, cudaStream_t st) {
     if (limbs == 0 || nz == 0) return cudaSuccess;
-    dim3 grid((n + 256 * kEwPer - 1) / (256 * kEwPer), limbs, nz);
+    const bool few = (u64)n * limbs * nz <= kEwFew;
     switch (op) {
-    case EW_ADD: elementwise_kernel<EW_ADD><<<grid, 256, 0, st>>>(pc, prime0, arena, n, zb); break;
-    case EW_SUB: elementwise_kernel<EW_SUB><<<grid, 256, 0, st>>>(pc, prime0, arena, n, zb); break;
-    case EW_MUL: elementwise_kernel<EW_MUL><<<grid, 256, 0, st>>>(pc, prime0, arena, n, zb); break;
-    default: elementwise_kernel<EW_COPY><<<grid, 256, 0, st>>>(pc, prime0, arena, n, zb); break;
+    case EW_ADD: launch_ew<EW_ADD>(few, pc, prime0, arena, n, limbs, nz, zb, st); break;
+    case EW_SUB: launch_ew<EW_SUB>(few, pc, prime0, arena, n, limbs, nz, zb, st); break;
+    case EW_MUL: launch_ew<EW_MUL>(few, pc, prime0, arena, n, limbs, nz, zb, st); break;
+    default: launch_ew<EW_COPY>(few, pc, prime0, arena, n, limbs, nz, zb, st); break;
     }
     count_launches(1);
     return cudaGetLastError();
