@@ -36,8 +36,6 @@ cudaError_t upload(afhe_ctx* ctx, void* dst, const void* src, size_t bytes) {
     return bytes ? cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, ctx->st) : cudaSuccess;
 }
 
-u64 host_shoup(u64 w, u64 q) { return (u64)(((unsigned __int128)w << 64) / q); }
-
 // The primitive 2N-th root behind prime i's twiddles (Q primes first, then
 // P): the one the parameters name, else the smallest.
 u64 root_of(const afhe_ctx* ctx, uint32_t i) {
@@ -83,19 +81,20 @@ int zf_from(afhe_ctx* ctx, const u64* vals, uint32_t n, ZField* out) {
 
 namespace {
 
-// transforms: with the constants in transform form (only a transform needs them)
-PrimeConst host_prime_const(u64 q, u64 ninv, u64 itw1, bool transforms) {
-    PrimeConst c{};
+void set_reductions(PrimeBase& c, u64 q) {
     c.q = q;
     ModConst m = make_modconst(q);
     c.r64 = m.r64;
     c.r64_sh = m.r64_sh;
     c.one_sh = m.one_sh;
+}
+
+PrimeConst host_prime_const(u64 q, u64 ninv, u64 itw1) {
+    PrimeConst c{};
+    set_reductions(c, q);
     c.ninv = ninv % q;
-    c.ninv_sh = host_shoup(c.ninv, q);
     c.w1ninv = (u64)((unsigned __int128)(itw1 % q) * c.ninv % q);
-    c.w1ninv_sh = host_shoup(c.w1ninv, q);
-    if (transforms) set_transform_constants(c);
+    set_transform_constants(c);
     return c;
 }
 
@@ -213,7 +212,7 @@ int build_native_tables(afhe_ctx* ctx) {
         u64 q = primes[i];
         u64* const iw = &itw[(size_t)i * n];
         gen_twiddles(ctx->log_n, q, root_of(ctx, i), &tw[(size_t)i * n], iw);
-        pc[i] = host_prime_const(q, inv_mod(n % q, q), iw[1], true);
+        pc[i] = host_prime_const(q, inv_mod(n % q, q), iw[1]);
     }
     DevPrimeSet& s = ctx->nat;
     s.count = np;
@@ -1048,15 +1047,16 @@ extern "C" int afhe_dispatch(afhe_ctx* ctx, const afhe_accel_args* a) {
         if (!range_ok(a->src_a_offset, LN, pw) || !range_ok(a->src_b_offset, LN, pw) || !range_ok(a->dst_offset, LN, pw))
             return fail(ctx, AFHE_E_RANGE, "poly operands out of range");
         // these ops need only the call's primes (fhe_accel_top.cpp:242-270)
-        std::vector<PrimeConst> pc(L);
+        // (64 bytes a prime: a larger copy than half a kilobyte takes 4 us longer)
+        std::vector<PrimeBase> pc(L);
         for (uint32_t i = 0; i < L; ++i) {
             if (a->rns_primes[i] < 3 || a->rns_primes[i] >= (1ull << 61)) return fail(ctx, AFHE_E_ARG, "modulus out of range");
-            pc[i] = host_prime_const(a->rns_primes[i], 1, 1, false);
+            set_reductions(pc[i], a->rns_primes[i]);     // (products through 128 bits)
         }
-        static_assert(sizeof(PrimeConst) % sizeof(u64) == 0, "PrimeConst is staged as words");
+        static_assert(sizeof(PrimeBase) % sizeof(u64) == 0, "PrimeBase is staged as words");
         u64* dpc_words = nullptr;
-        if ((rc = ring_put(ctx, pc.data(), L * sizeof(PrimeConst) / sizeof(u64), &dpc_words)) != AFHE_OK) return rc;
-        const PrimeConst* dpc = (const PrimeConst*)dpc_words;
+        if ((rc = ring_put(ctx, pc.data(), L * sizeof(PrimeBase) / sizeof(u64), &dpc_words)) != AFHE_OK) return rc;
+        const PrimeBase* dpc = (const PrimeBase*)dpc_words;
         // operands that partially overlap the output are staged (scratch words [0, 2LN))
         u64 sa, sb; bool ia, ib;
         if ((rc = stage(ctx, a->src_a_offset, LN, a->dst_offset, LN, 0, &sa, &ia)) != AFHE_OK) return rc;

@@ -169,7 +169,8 @@ enum ElemOp { EW_ADD = 0, EW_SUB = 1, EW_MUL = 2, EW_COPY = 3 };
 
 // out[l] = a[l] op b[l] for limbs l < limbs, primes from pc[prime0 + l]; z
 // entries with per-z offsets in zb (src = a, aux = b, out = out).
-cudaError_t launch_elementwise(ElemOp op, const PrimeConst* pc, uint32_t prime0, u64* arena, uint32_t n,
+template <class PC>                       // PrimeConst or PrimeBase
+cudaError_t launch_elementwise(ElemOp op, const PC* pc, uint32_t prime0, u64* arena, uint32_t n,
                                uint32_t limbs, uint32_t nz, const ZBases& zb, cudaStream_t st);
 
 // Ciphertext tensor product operands, per z (word offsets into one arena).

@@ -1,15 +1,10 @@
-// kernels.cu -- CUDA kernels and launchers for the CKKS evaluation core.
+// kernels.cu -- CUDA kernels and launchers for the CKKS evaluation core: pointwise
+// operations, tensor products, automorphisms, sums of plaintext products (the
+// diagonal method's among them), plain transforms and the tables' constants.
 //
 // Reference functions restated here (paths inside iheydardoost/ANNS_FHE):
 //   poly_add / poly_sub / poly_mul      hardware_fpga_model/hls/src/poly_arith.cpp:3-38
 //   automorphism                        hardware_fpga_model/hls/src/automorphism.cpp:3-12
-//   rescale                             hardware_fpga_model/hls/src/rescale.cpp:3-72
-//   fast_bases_conv / approx_mod_down   hardware_fpga_model/hls/src/key_switch.cpp:7-163
-//   key_switch                          hardware_fpga_model/hls/src/key_switch.cpp:167-439
-// Fusion: the base conversions run as the prologue of the NTT that consumes
-// them; the rescale combine (a_i * q_l^-1 + NTT(...)) and the ModDown combine
-// ((x_Q - y) * P^-1) run as the NTT epilogue; the evaluation-key inner product
-// accumulates all digits of a limb in 128-bit registers and reduces once.
 #include <atomic>
 
 #include "internal.h"
@@ -33,11 +28,11 @@ void set_ntt_plan(int log_n, int plan) { g_ntt_plan[log_n].store(plan, std::memo
 // and its reduction). Four a thread, or one in launches of few words, which four in a
 // row take longer than the launch itself (products of one limb one after another,
 // N = 2^11, us, four / one: 60 bits 4.1 / 3.4, 50 bits 4.1 / 3.3; of 2^17 words 4.1 both).
-template <int OP, uint32_t PER>
-__global__ void __launch_bounds__(256) elementwise_kernel(const PrimeConst* __restrict__ pc, uint32_t prime0,
+template <int OP, uint32_t PER, class PC>
+__global__ void __launch_bounds__(256) elementwise_kernel(const PC* __restrict__ pc, uint32_t prime0,
                                                           u64* __restrict__ arena, uint32_t n, const ZBases zb) {
     const uint32_t l = blockIdx.y, z = blockIdx.z;
-    const PrimeConst p = pc[prime0 + l];
+    const PrimeBase p = pc[prime0 + l];
     const uint32_t i0 = blockIdx.x * (256 * PER) + threadIdx.x;
     const u64 off = (u64)l * n + i0;
     const u64* a = arena + zb.src.at(z) + off;
@@ -61,16 +56,17 @@ __global__ void __launch_bounds__(256) elementwise_kernel(const PrimeConst* __re
 }
 
 constexpr u64 kEwFew = 1u << 16;     // words
-template <int OP>
-void launch_ew(bool few, const PrimeConst* pc, uint32_t prime0, u64* arena, uint32_t n, uint32_t limbs, uint32_t nz,
+template <int OP, class PC>
+void launch_ew(bool few, const PC* pc, uint32_t prime0, u64* arena, uint32_t n, uint32_t limbs, uint32_t nz,
                const ZBases& zb, cudaStream_t st) {
     const uint32_t per = few ? 256 : 256 * 4;
     const dim3 grid((n + per - 1) / per, limbs, nz);
-    if (few) elementwise_kernel<OP, 1><<<grid, 256, 0, st>>>(pc, prime0, arena, n, zb);
-    else elementwise_kernel<OP, 4><<<grid, 256, 0, st>>>(pc, prime0, arena, n, zb);
+    if (few) elementwise_kernel<OP, 1, PC><<<grid, 256, 0, st>>>(pc, prime0, arena, n, zb);
+    else elementwise_kernel<OP, 4, PC><<<grid, 256, 0, st>>>(pc, prime0, arena, n, zb);
 }
 
-cudaError_t launch_elementwise(ElemOp op, const PrimeConst* pc, uint32_t prime0, u64* arena, uint32_t n,
+template <class PC>
+cudaError_t launch_elementwise(ElemOp op, const PC* pc, uint32_t prime0, u64* arena, uint32_t n,
                                uint32_t limbs, uint32_t nz, const ZBases& zb, cudaStream_t st) {
     if (limbs == 0 || nz == 0) return cudaSuccess;
     const bool few = (u64)n * limbs * nz <= kEwFew;
@@ -83,6 +79,10 @@ cudaError_t launch_elementwise(ElemOp op, const PrimeConst* pc, uint32_t prime0,
     count_launches(1);
     return cudaGetLastError();
 }
+template cudaError_t launch_elementwise(ElemOp, const PrimeConst*, uint32_t, u64*, uint32_t, uint32_t, uint32_t,
+                                        const ZBases&, cudaStream_t);
+template cudaError_t launch_elementwise(ElemOp, const PrimeBase*, uint32_t, u64*, uint32_t, uint32_t, uint32_t,
+                                        const ZBases&, cudaStream_t);
 
 // ---------------------------------------------------------------------------
 // ciphertext tensor product (fhe_host_driver.cpp:280-286):
@@ -249,18 +249,15 @@ constexpr uint32_t kDiagTile = 256, kDiagUnits = 128;
 // halves below 2^57: room for 32 of the middle ones, used for at most 16 of
 // them twice); recombined in 128 bits.
 constexpr uint32_t kHalfBits = 25, kHalfMask = (1u << kHalfBits) - 1, kWordBits = 2 * kHalfBits;
-__device__ __forceinline__ void mad_wide(u64& acc, uint32_t a, uint32_t b) {
-    asm("mad.wide.u32 %0, %1, %2, %0;" : "+l"(acc) : "r"(a), "r"(b));
-}
 struct Halves {
     u64 s00, s01, s11;
 };
 __device__ __forceinline__ void halves_mad(Halves& h, uint32_t v0, uint32_t v1, u64 x) {
     const uint32_t x0 = (uint32_t)x & kHalfMask, x1 = (uint32_t)(x >> kHalfBits);
-    mad_wide(h.s00, v0, x0);
-    mad_wide(h.s01, v0, x1);
-    mad_wide(h.s01, v1, x0);
-    mad_wide(h.s11, v1, x1);
+    h.s00 = mad_wide_u32(v0, x0, h.s00);
+    h.s01 = mad_wide_u32(v0, x1, h.s01);
+    h.s01 = mad_wide_u32(v1, x0, h.s01);
+    h.s11 = mad_wide_u32(v1, x1, h.s11);
 }
 __device__ __forceinline__ u64 halves_reduce(const Halves& h, const ModConst& m) {
     u64 lo = h.s00, hi = 0;
@@ -698,9 +695,7 @@ __global__ void prime_consts_kernel(PrimeConst* pc, const u64* q, const u64* nin
     c.r64_sh = m.r64_sh;
     c.one_sh = m.one_sh;
     c.ninv = ninv[i] % c.q;
-    c.ninv_sh = shoup_companion(c.ninv, c.q);
     c.w1ninv = mul_mod(itw[(u64)i * n + 1] % c.q, c.ninv, m);
-    c.w1ninv_sh = shoup_companion(c.w1ninv, c.q);
     set_transform_constants(c);
     pc[i] = c;
 }

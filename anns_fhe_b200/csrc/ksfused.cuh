@@ -611,7 +611,6 @@ __device__ AFHE_KS_FN void leave_sums(const Slot<LOGQ, LOGCL, E, SINGLE> S, uint
 template <class A, int LOGQ, int LOGCL, uint32_t E, bool PREP, bool SINGLE>
 __device__ __forceinline__ void special_slot(const Slot<LOGQ, LOGCL, E, SINGLE>& S, uint32_t k) {
     using G = Geo<LOGQ, LOGCL, E>;
-    constexpr int LOGN = G::LOGN;
     const OpTabs& t = S.t();
     const uint32_t prime = t.p_base + k;
     if (SINGLE) {

@@ -14,7 +14,6 @@ inline bool range_ok(u64 off, u64 words, u64 size) { return off <= size && words
 extern thread_local std::string g_last_error;
 int fail(afhe_ctx* ctx, int code, const std::string& msg);
 int cuda_fail(afhe_ctx* ctx, cudaError_t e, const char* where);
-u64 host_shoup(u64 w, u64 q);
 // Copy host memory to the device on the context's stream, where what
 // reads it is launched: the stream is non-blocking, so nothing on it waits for a
 // copy on the legacy stream, which may return before its data has arrived.

@@ -57,8 +57,6 @@ AFHE_HD u64 mul_shoup_lazy(u64 a, u64 w, u64 wsh, u64 q) {
 
 AFHE_HD u64 csub(u64 x, u64 q) { return x >= q ? x - q : x; }
 
-AFHE_HD u64 mul_shoup(u64 a, u64 w, u64 wsh, u64 q) { return csub(mul_shoup_lazy(a, w, wsh, q), q); }
-
 AFHE_HD u64 add_mod(u64 a, u64 b, u64 q) { return csub(a + b, q); }
 AFHE_HD u64 sub_mod(u64 a, u64 b, u64 q) { return a >= b ? a - b : a + q - b; }
 

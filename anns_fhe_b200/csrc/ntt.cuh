@@ -28,8 +28,8 @@
 //     sums need no reduction for several stages: 6.8 butterflies per clock
 //     per SM;
 //   * larger q (< 2^61): the operand is split into 32-bit halves, each with
-//     its own multiple of the constant mod q, so that the quotient has 32 bits
-//     and everything but three wide products is a low product (ArSp): 4.0
+//     its own multiple of the constant mod q, so that the quotient is below 2^33
+//     and everything but three wide products is a low product (ArSp): 3.3 to 3.7
 //     butterflies per clock per SM.
 #pragma once
 #include <cstdint>
@@ -44,17 +44,19 @@ void count_launches(uint64_t k);
 // split one (ArSp).
 constexpr u64 kFpLimit = 1ull << 50;
 
-// Per-prime constants (160 bytes). The pairs at the end are in the form the
-// prime's transforms use (see transform_constant).
-struct PrimeConst {
+// A modulus' constants (64 bytes): what sums and products of words need.
+struct PrimeBase {
     u64 q;
-    u64 ninv, ninv_sh;        // N^-1 mod q and its Shoup companion
-    u64 w1ninv, w1ninv_sh;    // itw[1] * N^-1 (fused last inverse stage)
     u64 r64, r64_sh, one_sh;  // reduce128 constants
     u64 fp;                   // q < kFpLimit
     double qd, qi;            // q and 1/q as doubles (fp)
     u64 over;                 // the bits above q's own
-    u64 nv[4], w1nv[4];       // ninv and w1ninv as transform constants
+};
+// Per-prime constants of the transforms (144 bytes). The arrays are in the form the
+// prime's transforms use (see transform_constant).
+struct PrimeConst : PrimeBase {
+    u64 ninv, w1ninv;         // N^-1 mod q, itw[1] * N^-1 (fused last inverse stage)
+    u64 nv[4], w1nv[4];       // the same as transform constants
 };
 
 // A constant w mod q as a transform multiplies by it:
@@ -127,7 +129,7 @@ AFHE_HD constexpr uint32_t tw_place(int log_n, int p, uint32_t c) {
     return (((1u << log_n) >> (R + K)) * (1 + tw_slot(K, s, c & ((1u << low) - 1)))) + (c >> low);
 }
 
-AFHE_HD ModConst modconst_of(const PrimeConst& p) {
+AFHE_HD ModConst modconst_of(const PrimeBase& p) {
     ModConst m;
     m.q = p.q; m.r64 = p.r64; m.r64_sh = p.r64_sh; m.one_sh = p.one_sh;
     return m;
@@ -187,14 +189,14 @@ struct ZBases {
 };
 
 // x mod q, any x
-__device__ __forceinline__ u64 residue(u64 x, const PrimeConst& pc) {
+__device__ __forceinline__ u64 residue(u64 x, const PrimeBase& pc) {
     return x < pc.q ? x : csub(mul_shoup_lazy(x, 1, pc.one_sh, pc.q), pc.q);
 }
 // Words from outside as residues: one branch, rarely taken, behind all their
 // loads. Unless EXACT, words below the next power of two (so below 2q) stay as
 // they are.
 template <int M, bool EXACT>
-__device__ __forceinline__ void residues(u64* v, const PrimeConst& pc) {
+__device__ __forceinline__ void residues(u64* v, const PrimeBase& pc) {
     u64 bits = 0;
     bool words = false;
 #pragma unroll
@@ -231,12 +233,6 @@ struct StorePlain {
         base[zb.out.at(z) + j.out + x] = v;
     }
 };
-
-__device__ __forceinline__ u64 canon4(u64 v, u64 q) {
-    u64 q2 = q << 1;
-    v = v >= q2 ? v - q2 : v;
-    return v >= q ? v - q : v;
-}
 
 __device__ __forceinline__ double as_double(u64 v) { return __longlong_as_double((long long)v); }
 __device__ __forceinline__ u64 as_bits(double v) { return (u64)__double_as_longlong(v); }
@@ -339,7 +335,7 @@ __device__ __forceinline__ double fp_mul2(double a, double b, double q, double q
 
 // The product of any two words, canonical: in doubles where both are residues
 // of a prime below 2^50, else 128 bits and their reduction.
-__device__ __forceinline__ u64 mul_words(u64 a, u64 b, const PrimeConst& pc) {
+__device__ __forceinline__ u64 mul_words(u64 a, u64 b, const PrimeBase& pc) {
     if (pc.fp && a < pc.q && b < pc.q) return fp_canon(fp_mul2(fp_of(a), fp_of(b), pc.qd, pc.qi), pc.qd);
     return mul_mod(a, b, modconst_of(pc));
 }
