@@ -75,15 +75,12 @@ AFHE_HD u64 bits_of(double x) {
 #endif
 }
 AFHE_HD void split_constant(u64 w, u64 q, u64* o) {
-    u64 w1 = w;
-    for (int i = 0; i < 32; ++i) {
-        w1 <<= 1;
-        if (w1 >= q) w1 -= q;
-    }
+    const u64 sh = shoup_companion(w, q);
+    const u64 w1 = (w << 32) - (sh >> 32) * q;          // w 2^32 mod q
     o[0] = w;
     o[1] = w1;
     const double s = 0x1p948;                 // 2^-52 2^1000
-    o[2] = bits_of((double)(shoup_companion(w, q) >> 12) * s);
+    o[2] = bits_of((double)(sh >> 12) * s);
     o[3] = bits_of((double)(shoup_companion(w1, q) >> 12) * s);
 }
 AFHE_HD void transform_constant(u64 w, u64 q, u64* o) {
