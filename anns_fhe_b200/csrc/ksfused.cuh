@@ -31,11 +31,12 @@
 //     Two cluster barriers per slot;
 //   * the last forward round (eight adjacent values per thread), the products
 //     with the key and the first inverse round run on the same registers;
-//   * rounds exchange values within 512, 64 or 8 threads, and only those wait
+//   * rounds exchange values within the CTA, 64 or 8 threads, and only those wait
 //     for one another.
 //
 // Shared memory: three padded slices (W for transforms, A0 / A1 for the two
-// sums): 104 KB per CTA at 2^12 values, two CTAs per SM.
+// sums), or two with a single digit (W is A0): 104 or 70 KB per CTA at 2^12 values,
+// two CTAs per SM.
 //
 // The key limbs every CTA of a launch reads are the same, so they come from
 // L2. A registered key comes as a prepared copy (key_prep_kernel): pairs in

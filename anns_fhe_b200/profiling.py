@@ -166,8 +166,10 @@ def mac_roofline(outputs: int = 64, units: int = 16, limbs: int = 2, reps: int =
     plaintexts placed at multiples of 1,024 slots; the plaintexts come from
     `units` units of 128 diagonals at `limbs` limbs (1 GiB at 16 units, more
     than L2). Timed with CUDA events on the context stream after 3 warm-up
-    calls. Algorithmic bytes: every plaintext read once per output, the
-    outputs written, the 16 sources (2 polynomials) read once. The kernel
+    calls. Algorithmic bytes: every plaintext read once (eight results meet the
+    same ones under other placements; operand_bytes counts them for each output, which
+    is what the kernel reads through L2), the outputs written, the 16 sources (2
+    polynomials) read once. The kernel
     is the diagonal chain's (afhe_eval_diag_inner_batch), or with `generic`
     afhe_eval_mac_plain_batch on the same terms."""
     import numpy as np
@@ -231,11 +233,13 @@ def mac_roofline(outputs: int = 64, units: int = 16, limbs: int = 2, reps: int =
         e1.record(st)
         e1.synchronize()
         ms = e0.elapsed_time(e1) / reps
-        alg = (len(T) * w + outputs * 2 * w + n1 * 2 * w) * 8
+        rest = outputs * 2 * w + n1 * 2 * w
+        alg = (len(np.unique(Ta["pt"])) * w + rest) * 8
         peak, src = load_peaks()
         return {"profile": "mac_plain" if generic else "diag_inner", "outputs": outputs, "terms": len(T),
                 "limbs": limbs, "ms": round(ms, 4),
-                "algorithmic_bytes": alg, "achieved_gbs": round(alg / ms / 1e6, 1), "peak_gbs": peak,
+                "algorithmic_bytes": alg, "operand_bytes": (len(T) * w + rest) * 8,
+                "achieved_gbs": round(alg / ms / 1e6, 1), "peak_gbs": peak,
                 "frac": round(alg / ms / 1e6 / peak, 3), "peak_source": src}
     finally:
         ctx.close()

@@ -204,9 +204,10 @@ int afhe_copy_poly(afhe_ctx* ctx, uint64_t dst_offset, uint64_t src_offset, uint
  *                      of it fills its waves; 0 where it cannot run. */
 #define AFHE_OPT_KS_CAPACITY 4u
 /*   AFHE_OPT_KS_EPT    8 or 16, AFHE_OPT_KS_SLICE 12 or 13: launch shapes of
- *                      earlier one-kernel key switches. It has one shape now (16
- *                      values per thread, slices of 2^12 coefficients, of 2^13 at
- *                      N = 2^16); the values are kept for callers that set and
+ *                      earlier one-kernel key switches. Its shape follows N and the
+ *                      launch now (16 values per thread, or 8 up to half a wave at
+ *                      N <= 2^12; slices of 2^12 coefficients, of 2^13 at N = 2^16);
+ *                      the values are kept for callers that set and
  *                      read them and change nothing. */
 #define AFHE_OPT_KS_EPT 5u
 #define AFHE_OPT_KS_SLICE 6u
